@@ -67,7 +67,6 @@ enum class CountKind {
     RowTiles,       // ceil((row[i+1]-row[i]) / a)
     Array,          // arr[i]
     ArrayTimes,     // arr[i] * a
-    BitZero,        // (arr[i] >> a) & 1 == 0   (radix sort pass)
     PiecesMin1,     // max(1, ceil(arr[i] / a))
     WindowPopc,     // popcount of the a words arr[i*a .. i*a+a)
     NonEmpty,       // row[i+1] > row[i]
@@ -81,8 +80,8 @@ struct CountSpec {
 gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_t *total,
                          cudaStream_t s);
 
-// Stable sort of row indices 0..n-1 by descending key (keys < 2^bits): idx_out[i] is the
-// i-th row.  Ties keep ascending row order.  1-bit LSD radix passes built on the scan.
+// Stable sort of row indices 0..n-1 by descending key (keys <= max_key): idx_out[i] is the
+// i-th row.  Ties keep ascending row order.  LSD radix passes of up to 8 bits.
 gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
                            uint32_t *idx_out, cudaStream_t s);
 

@@ -68,12 +68,11 @@ struct CountDev {
         }
         case 2: return (uint64_t)arr[i];
         case 3: return (uint64_t)arr[i] * (uint64_t)a;
-        case 4: return (uint64_t)(((arr[i] >> a) & 1u) == 0u);
-        case 5: {
+        case 4: {
             uint32_t t = (arr[i] + a - 1) / a;
             return (uint64_t)(t ? t : 1u);
         }
-        case 6: {
+        case 5: {
             uint64_t c = 0;
             for (uint32_t j = 0; j < a; j++) c += __popc(arr[i * a + j]);
             return c;
@@ -193,9 +192,10 @@ __global__ void k_write_total(const uint64_t *bsum, size_t nb, uint64_t *out, si
     out[n] = bsum[nb];
 }
 
-static gs_status scan_impl(const CountDev &f, size_t n, uint64_t *out, uint64_t *total,
-                           cudaStream_t s)
+gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_t *total,
+                         cudaStream_t s)
 {
+    const CountDev f{(int)spec.kind, spec.row, spec.arr, spec.a};
     size_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) nb = 1;
     uint64_t *bsum = nullptr;
@@ -215,36 +215,171 @@ static gs_status scan_impl(const CountDev &f, size_t n, uint64_t *out, uint64_t 
     return GS_OK;
 }
 
-gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_t *total,
-                         cudaStream_t s)
-{
-    CountDev f{(int)spec.kind, spec.row, spec.arr, spec.a};
-    return scan_impl(f, n, out, total, s);
-}
-
 // ------------------------------------------------------------------ stable radix sort
-__global__ void k_sort_init(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *k,
-                            uint32_t *idx)
+// LSD radix sort of (key, index) pairs, at most 8 bits a pass.  A pass is bound by the bytes it
+// moves (8 in, 8 out per element; the first reads only the keys and makes the indices, the last
+// writes only the indices), so the wider the digit the fewer the bytes: one bit a pass took 14
+// passes for row lengths and 20 for a million columns.  A block ranks a tile of kRadixTile
+// elements: warps rank their own 512 in order (match of equal digits, one counter per digit and
+// warp), the warps' counts are summed per digit, and the tile is reordered in shared memory
+// before it is written, so that a digit's elements leave as one run (64 bytes on average with
+// 256 digits and 4096 elements).  Between blocks there is no waiting: the tiles' digit counts
+// are made by a pass of their own and scanned by one block per digit.
+// 4.2M elements, 20-bit keys: 20 passes of one bit 1310 us, 3 passes of 7 bits about 150 us.
+constexpr int kRadixThreads = 256;
+constexpr int kRadixWarps = kRadixThreads / 32;
+constexpr int kRadixItems = 16;
+constexpr uint32_t kRadixTile = kRadixThreads * kRadixItems;
+constexpr int kRadixDigits = 256;
+
+// ascending in max_key - key == descending in key
+template <bool FIRST>
+__device__ __forceinline__ uint32_t radix_key(uint32_t k, uint32_t max_key)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        k[i] = max_key - key[i];  // ascending in k == descending in key
-        idx[i] = i;
+    return FIRST ? max_key - k : k;
+}
+
+// count[d * tiles + t] = elements of tile t with digit d
+template <bool FIRST>
+__global__ void __launch_bounds__(kRadixThreads) k_radix_count(
+    const uint32_t *__restrict__ kin, uint32_t n, uint32_t max_key, uint32_t shift,
+    uint32_t mask, uint32_t tiles, uint32_t *__restrict__ count)
+{
+    __shared__ uint32_t h[kRadixDigits];
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t t0 = blockIdx.x * kRadixTile;
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) {
+        const uint32_t o = (uint32_t)i * kRadixThreads + threadIdx.x;
+        if (o < n - t0)
+            atomicAdd(&h[(radix_key<FIRST>(kin[t0 + o], max_key) >> shift) & mask], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x <= mask) count[(size_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+}
+
+// Exclusive prefix of one value per thread over the block; *total (shared) = the sum.
+__device__ __forceinline__ uint32_t radix_block_scan(uint32_t v, uint32_t *wsum, uint32_t *total)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += u;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < kRadixWarps; i++) {
+        if (i < w) before += wsum[i];
+        all += wsum[i];
+    }
+    if (threadIdx.x == 0) *total = all;
+    __syncthreads();
+    return before + inc - v;
+}
+
+// Block d: exclusive prefix of digit d's tile counts in place, total[d] = their sum.
+__global__ void __launch_bounds__(kRadixThreads) k_radix_scan(uint32_t *__restrict__ count,
+                                                              uint32_t tiles,
+                                                              uint32_t *__restrict__ total)
+{
+    __shared__ uint32_t wsum[kRadixWarps], sum;
+    uint32_t *c = count + (size_t)blockIdx.x * tiles;
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < tiles; b += kRadixThreads) {
+        const uint32_t i = b + threadIdx.x;
+        const uint32_t v = i < tiles ? c[i] : 0u;
+        const uint32_t e = radix_block_scan(v, wsum, &sum);
+        if (i < tiles) c[i] = carry + e;
+        carry += sum;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
+    const uint32_t *__restrict__ kin, const uint32_t *__restrict__ iin, uint32_t n,
+    uint32_t max_key, uint32_t shift, uint32_t mask, uint32_t tiles,
+    const uint32_t *__restrict__ before, const uint32_t *__restrict__ total,
+    uint32_t *__restrict__ kout, uint32_t *__restrict__ iout)
+{
+    __shared__ uint32_t wcount[kRadixWarps][kRadixDigits];
+    __shared__ uint32_t start[kRadixDigits];  // digit's first position in the sorted tile
+    __shared__ uint32_t dest[kRadixDigits];   // output index of that position
+    __shared__ uint32_t skey[kRadixTile], sidx[kRadixTile];
+    __shared__ uint32_t wsum[kRadixWarps], sum;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t t0 = blockIdx.x * kRadixTile;
+    const uint32_t cnt = min(kRadixTile, n - t0);
+#pragma unroll
+    for (int i = 0; i < kRadixWarps; i++) wcount[i][threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t key[kRadixItems], idx[kRadixItems], rank[kRadixItems];
+    const uint32_t o0 = (uint32_t)w * 32u * kRadixItems + (uint32_t)lane;
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) {
+        const uint32_t o = o0 + 32u * i;
+        key[i] = o < cnt ? radix_key<FIRST>(kin[t0 + o], max_key) : 0u;
+        idx[i] = FIRST ? t0 + o : (o < cnt ? iin[t0 + o] : 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) {
+        const bool in = o0 + 32u * i < cnt;
+        const unsigned live = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const uint32_t d = (key[i] >> shift) & mask;
+            const unsigned peers = __match_any_sync(live, d);
+            const uint32_t below = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+            rank[i] = wcount[w][d] + below;
+            __syncwarp(live);
+            if (below == 0) wcount[w][d] += (uint32_t)__popc(peers);
+            __syncwarp(live);
+        }
+    }
+    __syncthreads();
+    {
+        const uint32_t d = threadIdx.x;
+        uint32_t run = 0;
+#pragma unroll
+        for (int i = 0; i < kRadixWarps; i++) {
+            const uint32_t c = wcount[i][d];
+            wcount[i][d] = run;
+            run += c;
+        }
+        const uint32_t e = radix_block_scan(run, wsum, &sum);
+        start[d] = e;
+        const uint32_t g = radix_block_scan(d <= mask ? total[d] : 0u, wsum, &sum);
+        dest[d] = d <= mask ? g + before[(size_t)d * tiles + blockIdx.x] : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) {
+        if (o0 + 32u * i < cnt) {
+            const uint32_t d = (key[i] >> shift) & mask;
+            const uint32_t p = start[d] + wcount[w][d] + rank[i];
+            skey[p] = key[i];
+            sidx[p] = idx[i];
+        }
+    }
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < cnt; p += kRadixThreads) {
+        const uint32_t k = skey[p], d = (k >> shift) & mask;
+        const uint32_t g = dest[d] + (p - start[d]);
+        if (!LAST) kout[g] = k;
+        iout[g] = sidx[p];
     }
 }
 
-__global__ void k_sort_scatter(const uint32_t *kin, const uint32_t *iin, uint32_t n,
-                               uint32_t bit, const uint64_t *zpre, uint32_t *kout,
-                               uint32_t *iout)
+// idx[i] = i
+__global__ void k_iota(uint32_t n, uint32_t *idx)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        uint64_t z = zpre[i], Z = zpre[n];
-        uint32_t kv = kin[i];
-        uint64_t d = (((kv >> bit) & 1u) == 0u) ? z : Z + ((uint64_t)i - z);
-        kout[d] = kv;
-        iout[d] = iin[i];
-    }
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) idx[i] = i;
 }
 
 gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
@@ -253,27 +388,42 @@ gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
     if (n == 0) return GS_OK;
     int bits = 0;
     while (bits < 32 && (max_key >> bits) != 0) bits++;
-    DevBuf ka, kb, ib, z;
-    GS_TRY(ka.alloc((size_t)n * 4));
-    GS_TRY(kb.alloc((size_t)n * 4));
-    GS_TRY(ib.alloc((size_t)n * 4));
-    GS_TRY(z.alloc(((size_t)n + 1) * 8));
-    uint32_t *kin = ka.as<uint32_t>(), *kout = kb.as<uint32_t>();
-    uint32_t *iin = idx_out, *iout = ib.as<uint32_t>();
-    unsigned g = (n + 255) / 256;
-    k_sort_init<<<g, 256, 0, s>>>(key, n, max_key, kin, iin);
-    GS_CHECK_LAUNCH();
-    for (int b = 0; b < bits; b++) {
-        CountDev f{4, nullptr, kin, (uint32_t)b};
-        GS_TRY(scan_impl(f, n, z.as<uint64_t>(), nullptr, s));
-        k_sort_scatter<<<g, 256, 0, s>>>(kin, iin, n, (uint32_t)b, z.as<uint64_t>(), kout,
-                                         iout);
+    if (bits == 0) {  // all keys equal: the order they came in
+        k_iota<<<(n + 255) / 256, 256, 0, s>>>(n, idx_out);
         GS_CHECK_LAUNCH();
-        uint32_t *t = kin; kin = kout; kout = t;
-        t = iin; iin = iout; iout = t;
+        return GS_OK;
     }
-    if (iin != idx_out)
-        GS_CUDA(cudaMemcpyAsync(idx_out, iin, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+    const int passes = (bits + 7) / 8;
+    const uint32_t db = (uint32_t)((bits + passes - 1) / passes);  // bits per pass
+    const uint32_t mask = (1u << db) - 1u, digits = mask + 1u;
+    const uint32_t tiles = (uint32_t)(((uint64_t)n + kRadixTile - 1) / kRadixTile);
+    DevBuf ka, kb, ib, cnt;
+    GS_TRY(cnt.alloc(((size_t)digits * tiles + digits) * 4));
+    if (passes > 1) {
+        GS_TRY(ka.alloc((size_t)n * 4));
+        GS_TRY(ib.alloc((size_t)n * 4));
+    }
+    if (passes > 2) GS_TRY(kb.alloc((size_t)n * 4));
+    uint32_t *c = cnt.as<uint32_t>(), *tot = c + (size_t)digits * tiles;
+    uint32_t *kbuf[2] = {ka.as<uint32_t>(), kb.as<uint32_t>()};
+    const uint32_t *kin = key, *iin = nullptr;
+    for (int p = 0; p < passes; p++) {
+        const bool first = p == 0, last = p == passes - 1;
+        const uint32_t shift = db * (uint32_t)p;
+        uint32_t *kout = kbuf[p & 1];
+        // the last pass writes idx_out
+        uint32_t *iout = ((passes - 1 - p) & 1) ? ib.as<uint32_t>() : idx_out;
+        if (first) k_radix_count<true><<<tiles, kRadixThreads, 0, s>>>(kin, n, max_key, shift, mask, tiles, c);
+        else k_radix_count<false><<<tiles, kRadixThreads, 0, s>>>(kin, n, max_key, shift, mask, tiles, c);
+        k_radix_scan<<<digits, kRadixThreads, 0, s>>>(c, tiles, tot);
+        auto scatter = first ? (last ? k_radix_scatter<true, true> : k_radix_scatter<true, false>)
+                             : (last ? k_radix_scatter<false, true> : k_radix_scatter<false, false>);
+        scatter<<<tiles, kRadixThreads, 0, s>>>(kin, iin, n, max_key, shift, mask, tiles, c, tot,
+                                                kout, iout);
+        GS_CHECK_LAUNCH();
+        kin = kout;
+        iin = iout;
+    }
     GS_CUDA(cudaStreamSynchronize(s));  // scratch buffers are freed on return
     return GS_OK;
 }
