@@ -258,6 +258,7 @@ SIGNATURES = {
     "gs_batch_status": (_st, [_vp, C.POINTER(UIN), _vp]),
     "gs_batch_run": (_st, [_vp, _vp]),
     "gs_batch_run_graph": (_st, [_vp, _vp]),
+    "gs_release_cached": (_st, []),
     "gs_copy_to_host": (_st, [_vp, _vp, C.c_size_t]),
     "gs_matrix_device_status": (_st, [_vp, C.POINTER(UIN), C.c_int]),
     "gs_gen_laplacian2d": (_st, [UIN, C.POINTER(UINp), C.POINTER(UINp), C.POINTER(FPTp),

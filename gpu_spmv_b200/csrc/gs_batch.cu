@@ -551,7 +551,7 @@ gs_status build_band_t(gs_batch *B, size_t i, cudaStream_t s)
     const uint32_t n = A->nrows;
     const size_t vsize = sizeof(T), rowb = (size_t)B->kpad[i] * vsize;
     std::vector<uint32_t> permi(n), klen(n), lo(n), hi(n);
-    DevBuf dlo, dhi;
+    StreamBuf dlo(s), dhi(s);
     GS_TRY(dlo.alloc((size_t)n * 4));
     GS_TRY(dhi.alloc((size_t)n * 4));
     if (n) {
@@ -620,7 +620,7 @@ gs_status build_band_t(gs_batch *B, size_t i, cudaStream_t s)
         }
     }
     const size_t etot = blocks.empty() ? 0 : blocks.back().e1;
-    DevBuf ddst;
+    StreamBuf ddst(s);
     GS_TRY(ddst.alloc((size_t)n * 4));
     GS_TRY(bm.info.alloc((size_t)n * 8));
     GS_TRY(bm.col.alloc_zero(etot * 4, s));
@@ -889,7 +889,7 @@ gs_status gs_batch_create(gs_batch **out, UIN count, gs_matrix *const *mats, con
 gs_status gs_batch_destroy(gs_batch *B)
 {
     if (!B) return GS_OK;
-    cudaDeviceSynchronize();
+    gs::DeviceIdle idle;  // waits: no run may still use the buffers
     delete B;
     return GS_OK;
 }

@@ -73,12 +73,12 @@ gs_status gs_matrix_create_host(gs_matrix **out, const gs_convert_params *params
     if (val_type != GS_F64 && val_type != GS_F32)
         return gs::fail(GS_ERR_UNSUPPORTED, "input CSR values must be FP64 or FP32");
     *out = nullptr;
-    gs::DevBuf row, col, val;
+    cudaStream_t s = gs::cs(stream);
+    gs::StreamBuf row(s), col(s), val(s);
     const size_t vsz = gs::dtype_size(val_type);
     GS_TRY(row.alloc(((size_t)nrows + 1) * 4));
     GS_TRY(col.alloc((size_t)nnz * 4));
     GS_TRY(val.alloc((size_t)nnz * vsz));
-    cudaStream_t s = gs::cs(stream);
     GS_CUDA(cudaMemcpyAsync(row.p, h_row, ((size_t)nrows + 1) * 4, cudaMemcpyHostToDevice, s));
     if (nnz) {
         GS_CUDA(cudaMemcpyAsync(col.p, h_col, (size_t)nnz * 4, cudaMemcpyHostToDevice, s));
@@ -92,7 +92,7 @@ gs_status gs_matrix_create_host(gs_matrix **out, const gs_convert_params *params
 gs_status gs_matrix_destroy(gs_matrix *A)
 {
     if (A) {
-        cudaDeviceSynchronize();  // no kernel may still read the buffers
+        gs::DeviceIdle idle;  // waits: no kernel may still read the buffers
         delete A;
     }
     return GS_OK;
@@ -284,6 +284,12 @@ gs_status gs_matrix_device_status(const gs_matrix *A, UIN *word, int reset)
     GS_CUDA(cudaMemcpy(word, A->plan.status.p, 4, cudaMemcpyDeviceToHost));
     if (reset) GS_CUDA(cudaMemset(A->plan.status.p, 0, 4));
     return GS_OK;
+}
+
+gs_status gs_release_cached(void)
+{
+    gs::clear_error();
+    return gs::release_cached();
 }
 
 gs_status gs_copy_to_host(void *h_dst, const void *d_src, size_t bytes)

@@ -277,8 +277,8 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
 
     // ---- validate the CSR (structure and column range)
     {
-        DevBuf flag;
-        GS_TRY(flag.alloc_zero(4, s));
+        StreamBuf flag(s);
+        GS_TRY(flag.alloc_zero(4));
         k_validate<<<blocks_for(n + 1), 256, 0, s>>>(n, ncols, nnz, d_row, d_col,
                                                      flag.as<uint32_t>());
         GS_CHECK_LAUNCH();
@@ -296,7 +296,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
     f.col = d_col;
     f.val = d_val;
     f.xbake = d_xbake;
-    DevBuf P;  // 64-bit offsets
+    StreamBuf P(s);  // 64-bit offsets
     const gs_format fmt = p.format;
 
     if (fmt == GS_FMT_K1) {
@@ -304,7 +304,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
             return fail(GS_ERR_UNSUPPORTED, "FP64 K1 is stored with 32-bit columns");
         const uint32_t chunkNum = (n + 31) / 32;
         A->chunkNum = chunkNum;
-        DevBuf rl;
+        StreamBuf rl(s);
         GS_TRY(rl.alloc((size_t)n * 4));
         k_rowlen<<<blocks_for(n), 256, 0, s>>>(n, d_row, rl.as<uint32_t>());
         GS_CHECK_LAUNCH();
@@ -313,7 +313,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         GS_TRY(A->permi.alloc_zero(((size_t)chunkNum + 1) * 32 * 4, s));
         GS_TRY(stable_sort_desc(rl.as<uint32_t>(), n, maxlen, A->permi.as<uint32_t>(), s));
         GS_TRY(A->nmc.alloc_zero((size_t)chunkNum * 4, s));
-        GS_TRY(A->k1len.alloc((size_t)n * 4));
+        GS_TRY(A->k1len.alloc((size_t)n * 4, s));
         k_k1_meta<<<blocks_for(n), 256, 0, s>>>(n, chunkNum, rl.as<uint32_t>(),
                                                 A->permi.as<uint32_t>(), A->nmc.as<uint32_t>(),
                                                 A->k1len.as<uint32_t>());
@@ -326,7 +326,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         GS_TRY(exclusive_scan(cs, chunkNum, P.as<uint64_t>(), &lenvc, s));
         if (lenvc > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 lenVC exceeds 32 bits");
         A->lenVC = (uint32_t)lenvc;
-        GS_TRY(A->chp.alloc((size_t)chunkNum * 4));
+        GS_TRY(A->chp.alloc((size_t)chunkNum * 4, s));
         k_u64_to_u32<<<blocks_for(chunkNum), 256, 0, s>>>(chunkNum, P.as<uint64_t>(),
                                                          A->chp.as<uint32_t>());
         GS_CHECK_LAUNCH();
@@ -334,8 +334,8 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         const size_t vsz = dtype_size(p.vtype), isz = u16 ? 2 : 4;
         GS_TRY(A->val.alloc_zero((size_t)A->lenVC * vsz, s));
         GS_TRY(A->col.alloc_zero((size_t)A->lenVC * isz, s));
-        DevBuf col32;  // 32-bit columns before the 16-bit steps are taken
-        if (u16) GS_TRY(col32.alloc_zero((size_t)A->lenVC * 4, s));
+        StreamBuf col32(s);  // 32-bit columns before the 16-bit steps are taken
+        if (u16) GS_TRY(col32.alloc_zero((size_t)A->lenVC * 4));
         uint32_t *ocol = u16 ? col32.as<uint32_t>() : A->col.as<uint32_t>();
         GS_TRY(build_k1_plan(A->nmc.as<uint32_t>(), chunkNum, A->k1unit_chunk, A->k1unit_base,
                              A->k1partial, A->k1count, &A->k1units, s));
@@ -363,7 +363,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
             a.unit_chunk = A->k1unit_chunk.as<uint32_t>();
             a.unit_base = A->k1unit_base.as<uint32_t>();
             a.units = A->k1units;
-            GS_TRY(A->k1ck.alloc((size_t)A->k1units * 32 * 4));
+            GS_TRY(A->k1ck.alloc((size_t)A->k1units * 32 * 4, s));
             GS_TRY(build_k1_deltas(a, col32.as<uint32_t>(), A->col.as<uint16_t>(),
                                    A->k1ck.as<uint32_t>(), s));
         }
@@ -378,7 +378,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         if (fmt == GS_FMT_AXT && (thw == 0 || th == 0))
             return fail(GS_ERR_INVALID, "tileHW and tileH must be >= 1");
         if (fmt == GS_FMT_AXC && p.hbs == 0) return fail(GS_ERR_INVALID, "hbs must be >= 1");
-        GS_TRY(A->rpos.alloc(((size_t)n + 1) * 4));
+        GS_TRY(A->rpos.alloc(((size_t)n + 1) * 4, s));
         bool need_rlen = false;
         uint64_t nslots = 0;
         f.layout = kDirect;
@@ -402,7 +402,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
             A->lenAX = (uint32_t)(bricks * 2 * hbs);
             A->lenBRP = n + 1;
             A->lenMAPX = A->lenAX / 2 + 8;
-            if (p.keep_layout) GS_TRY(A->brp.alloc(((size_t)n + 1) * 4));
+            if (p.keep_layout) GS_TRY(A->brp.alloc(((size_t)n + 1) * 4, s));
             k_tables<<<blocks_for((uint64_t)n + 1), 256, 0, s>>>(
                 n, P.as<uint64_t>(), 2, hbs, 0, 0, p.keep_layout ? A->brp.as<uint32_t>() : nullptr,
                 A->rpos.as<uint32_t>());
@@ -505,7 +505,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         if (nslots > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "slot count exceeds 32 bits");
         A->nslots = (uint32_t)nslots;
         if (need_rlen) {
-            GS_TRY(A->rlen.alloc((size_t)n * 4));
+            GS_TRY(A->rlen.alloc((size_t)n * 4, s));
             k_rowlen<<<blocks_for(n), 256, 0, s>>>(n, d_row, A->rlen.as<uint32_t>());
             GS_CHECK_LAUNCH();
         }
@@ -513,12 +513,13 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         if (p.itype == GS_IDX_U16 && A->tiled)
             return fail(GS_ERR_UNSUPPORTED, "16-bit columns need tileH=1");
         GS_TRY(A->val.alloc_zero((size_t)A->nslots * dtype_size(p.vtype), s));
-        DevBuf col32;
-        DevBuf &c32 = (p.itype == GS_IDX_U16) ? col32 : A->col;
-        GS_TRY(c32.alloc_zero((size_t)A->nslots * 4, s));
+        StreamBuf col32(s);
+        const bool u16 = p.itype == GS_IDX_U16;
+        if (u16) GS_TRY(col32.alloc_zero((size_t)A->nslots * 4));
+        else GS_TRY(A->col.alloc_zero((size_t)A->nslots * 4, s));
         f.rpos = (f.layout == kCom) ? d_row : A->rpos.as<uint32_t>();
         f.oval = A->val.p;
-        f.ocol = c32.as<uint32_t>();
+        f.ocol = u16 ? col32.as<uint32_t>() : A->col.as<uint32_t>();
         if (ax_out) {
             GS_TRY(ax_out->alloc_zero((size_t)A->lenAX * 8, s));
             f.ax = ax_out->as<double>();
@@ -566,7 +567,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
             ((fmt == GS_FMT_AXT && p.mode == GS_AXT_UNC) || fmt == GS_FMT_AXC)) {
             const uint32_t w = fmt == GS_FMT_AXC ? p.hbs : thw;
             if (w == 4 || w == 8 || w == 16) {
-                DevBuf rt;
+                StreamBuf rt(s);
                 GS_TRY(rt.alloc(((size_t)n + 1) * 4));
                 k_tile_starts<<<blocks_for(n + 1), 256, 0, s>>>(n + 1, A->rpos.as<uint32_t>(), w,
                                                                 rt.as<uint32_t>());
@@ -575,7 +576,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
                 A->tile_w = w;
             }
         }
-        if (p.itype == GS_IDX_U16) {
+        if (u16) {
             GS_TRY(A->col.alloc_zero((size_t)A->nslots * 2, s));
             GS_TRY(build_u16_columns(col32.as<uint32_t>(), A->nslots, A->plan,
                                      A->col.as<uint16_t>(), s));

@@ -39,24 +39,72 @@ inline cudaStream_t cs(gs_stream s) { return reinterpret_cast<cudaStream_t>(s); 
 inline size_t dtype_size(gs_dtype t) { return t == GS_F64 ? 8 : (t == GS_F32 ? 4 : 2); }
 
 // ------------------------------------------------------------------ device buffers
-// Owning device allocation (cudaMalloc / cudaFree).
+// Device memory comes from one stream-ordered pool per device (gs_scan.cu): cudaMalloc and
+// cudaFree cost tens to hundreds of microseconds each and stop the device, and a conversion
+// makes two dozen of them (16.8M-element K1 conversion and product: 8.9 ms with them, 0.67 ms
+// from the pool; a 4.2M-element operator build, forward and adjoint: 28 -> 1.6 ms).  The pool
+// keeps at most kPoolIdle bytes that no buffer uses; the rest goes back to the device at the
+// next synchronisation, all of it with gs_release_cached(), and a cudaMalloc of this process
+// that finds too little free memory gets it from the driver (864 MiB idle, a request of 0.75 GiB
+// above the free memory granted).
+constexpr size_t kPoolIdle = size_t(1) << 30;
+
+// Owning allocation that may be used on any stream.  alloc(n) is usable everywhere at once;
+// alloc(n, s) is ordered on s like the work that fills it, which the caller orders (or
+// synchronises) before any other stream's use.  reset() waits for the device, as cudaFree does.
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    size_t reserved = 0;  // bytes taken from the pool
+    int dev = -1;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; o.bytes = 0; }
-    DevBuf &operator=(DevBuf &&o) noexcept {
-        if (this != &o) { reset(); p = o.p; bytes = o.bytes; o.p = nullptr; o.bytes = 0; }
+    DevBuf(DevBuf &&o) noexcept { *this = static_cast<DevBuf &&>(o); }
+    DevBuf &operator=(DevBuf &&o) noexcept
+    {
+        if (this != &o) {
+            reset();
+            p = o.p, bytes = o.bytes, reserved = o.reserved, dev = o.dev;
+            o.p = nullptr, o.bytes = 0;
+        }
         return *this;
     }
     ~DevBuf() { reset(); }
-    void reset() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
-    gs_status alloc(size_t nbytes);                       // rounds up, keeps 16 B of tail slack
-    gs_status alloc_zero(size_t nbytes, cudaStream_t s);  // alloc + async memset 0
+    void reset();
+    gs_status alloc(size_t nbytes);                  // rounds up, keeps 16 B of tail slack
+    gs_status alloc(size_t nbytes, cudaStream_t s);
+    gs_status alloc_zero(size_t nbytes, cudaStream_t s);  // alloc + async memset 0, on s
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
+
+// While one lives, buffers of its device that this thread resets do not wait for the device:
+// the caller has just synchronised it (destroying a matrix resets some 45 buffers).
+struct DeviceIdle {
+    DeviceIdle();
+    ~DeviceIdle();
+    int outer;
+};
+
+// Scratch of one function, used on stream s alone: allocated and freed in stream order, with no
+// synchronisation.
+struct StreamBuf {
+    explicit StreamBuf(cudaStream_t stream) : s(stream) {}
+    StreamBuf(const StreamBuf &) = delete;
+    StreamBuf &operator=(const StreamBuf &) = delete;
+    ~StreamBuf();
+    gs_status alloc(size_t nbytes);
+    gs_status alloc_zero(size_t nbytes);
+    template <class T> T *as() const { return static_cast<T *>(p); }
+    void *p = nullptr;
+
+private:
+    cudaStream_t s;
+    size_t reserved = 0;
+    int dev = -1;
+};
+// Gives the pool's unused memory back, on the current device.
+gs_status release_cached();
 
 // ------------------------------------------------------------------ scan primitives
 // Exclusive prefix sum of n 32-bit counts produced by `count(i)`, written as 64-bit

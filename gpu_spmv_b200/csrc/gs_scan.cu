@@ -29,25 +29,166 @@ gs_status fail(gs_status st, const char *fmt, ...)
 void clear_error() { g_err[0] = 0; }
 const char *last_error_text() { return g_err; }
 
-// ------------------------------------------------------------------ DevBuf
+// ------------------------------------------------------------------ device memory
+namespace {
+
+constexpr int kMaxDevices = 64;
+
+struct DevPool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;  // orders allocations and frees that belong to no stream
+    size_t live = 0, kept_for = 0;  // bytes in buffers; the value of `live` the pool was told
+};
+std::mutex g_pool_mutex;
+DevPool g_pools[kMaxDevices];  // live as long as the process, like the device's own pool
+
+thread_local int t_idle_device = -1;  // DeviceIdle
+
+gs_status pool_of(int dev, DevPool **out)
+{
+    if (dev < 0 || dev >= kMaxDevices) return fail(GS_ERR_UNSUPPORTED, "device %d", dev);
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    DevPool &P = g_pools[dev];
+    if (!P.pool) {
+        if (!P.stream) GS_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        GS_CUDA(cudaMemPoolCreate(&p, &props));
+        uint64_t keep = kPoolIdle;
+        GS_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        P.pool = p;
+    }
+    *out = &P;
+    return GS_OK;
+}
+
+// The pool holds on to what its buffers use and kPoolIdle more; it is told again when the use
+// has moved by an eighth of that.
+void pool_use(DevPool &P, size_t add, size_t sub)
+{
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    P.live = P.live + add - sub;
+    const size_t d = P.live > P.kept_for ? P.live - P.kept_for : P.kept_for - P.live;
+    if (d >= kPoolIdle / 8) {
+        uint64_t keep = P.live + kPoolIdle;
+        cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        P.kept_for = P.live;
+    }
+}
+
+size_t rounded(size_t nbytes)  // slack: vector loads may touch the tail
+{
+    return ((nbytes + 255) / 256) * 256 + 256;
+}
+
+// n bytes ordered on s, or on the pool's own stream (own)
+gs_status pool_alloc(size_t n, cudaStream_t s, bool own, void **p, int *dev)
+{
+    GS_CUDA(cudaGetDevice(dev));
+    DevPool *P = nullptr;
+    GS_TRY(pool_of(*dev, &P));
+    if (own) s = P->stream;
+    // a captured allocation would belong to the graph, not to the buffer
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GS_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return fail(GS_ERR_CUDA, "device memory is needed on a stream under capture");
+    cudaError_t e = cudaMallocFromPoolAsync(p, n, P->pool, s);
+    if (e == cudaSuccess && own) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+        return fail(GS_ERR_ALLOC, "allocation of %zu bytes failed: %s", n, cudaGetErrorString(e));
+    }
+    pool_use(*P, n, 0);
+    return GS_OK;
+}
+
+}  // namespace
+
 gs_status DevBuf::alloc(size_t nbytes)
 {
     reset();
-    size_t n = ((nbytes + 255) / 256) * 256 + 256;  // slack: vector loads may touch the tail
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e != cudaSuccess) {
-        p = nullptr;
-        cudaGetLastError();
-        return fail(GS_ERR_ALLOC, "cudaMalloc(%zu) failed: %s", n, cudaGetErrorString(e));
-    }
+    GS_TRY(pool_alloc(rounded(nbytes), nullptr, true, &p, &dev));
+    reserved = rounded(nbytes);
+    bytes = nbytes;
+    return GS_OK;
+}
+
+gs_status DevBuf::alloc(size_t nbytes, cudaStream_t s)
+{
+    reset();
+    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &dev));
+    reserved = rounded(nbytes);
     bytes = nbytes;
     return GS_OK;
 }
 
 gs_status DevBuf::alloc_zero(size_t nbytes, cudaStream_t s)
 {
+    GS_TRY(alloc(nbytes, s));
+    GS_CUDA(cudaMemsetAsync(p, 0, reserved, s));
+    return GS_OK;
+}
+
+void DevBuf::reset()
+{
+    if (!p) return;
+    int cur = -1;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    // kernels of any stream may still read it; memory of a device that cannot be waited for
+    // stays allocated
+    if (t_idle_device == dev || cudaDeviceSynchronize() == cudaSuccess) {
+        DevPool &P = g_pools[dev];
+        cudaFreeAsync(p, P.stream);
+        pool_use(P, 0, reserved);
+    }
+    if (cur != dev) cudaSetDevice(cur);
+    p = nullptr;
+    bytes = 0;
+}
+
+DeviceIdle::DeviceIdle() : outer(t_idle_device)
+{
+    int dev = -1;
+    if (cudaDeviceSynchronize() == cudaSuccess) cudaGetDevice(&dev);
+    t_idle_device = dev;
+}
+DeviceIdle::~DeviceIdle() { t_idle_device = outer; }
+
+gs_status StreamBuf::alloc(size_t nbytes)
+{
+    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &dev));
+    reserved = rounded(nbytes);
+    return GS_OK;
+}
+
+gs_status StreamBuf::alloc_zero(size_t nbytes)
+{
     GS_TRY(alloc(nbytes));
-    GS_CUDA(cudaMemsetAsync(p, 0, ((nbytes + 255) / 256) * 256 + 256, s));
+    GS_CUDA(cudaMemsetAsync(p, 0, reserved, s));
+    return GS_OK;
+}
+
+StreamBuf::~StreamBuf()
+{
+    if (!p) return;
+    cudaFreeAsync(p, s);
+    pool_use(g_pools[dev], 0, reserved);
+}
+
+gs_status release_cached()
+{
+    int dev = -1;
+    GS_CUDA(cudaGetDevice(&dev));
+    DevPool *P = nullptr;
+    GS_TRY(pool_of(dev, &P));
+    GS_CUDA(cudaDeviceSynchronize());
+    GS_CUDA(cudaMemPoolTrimTo(P->pool, 0));
     return GS_OK;
 }
 
@@ -198,16 +339,14 @@ gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_
     const CountDev f{(int)spec.kind, spec.row, spec.arr, spec.a};
     size_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) nb = 1;
-    uint64_t *bsum = nullptr;
-    GS_CUDA(cudaMallocAsync(&bsum, (nb + 1) * sizeof(uint64_t), s));
+    StreamBuf sums(s);
+    GS_TRY(sums.alloc((nb + 1) * sizeof(uint64_t)));
+    uint64_t *bsum = sums.as<uint64_t>();
     k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(f, n, bsum);
     k_scan_blocks<<<1, 1024, 0, s>>>(bsum, nb);
     k_scan_down<<<(unsigned)nb, kScanThreads, 0, s>>>(f, n, bsum, out);
     k_write_total<<<1, 1, 0, s>>>(bsum, nb, out, n);
-    cudaError_t le = cudaGetLastError();
-    cudaFreeAsync(bsum, s);
-    if (le != cudaSuccess)
-        return fail(GS_ERR_CUDA, "scan launch failed: %s", cudaGetErrorString(le));
+    GS_CHECK_LAUNCH();
     if (total) {
         GS_CUDA(cudaMemcpyAsync(total, out + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         GS_CUDA(cudaStreamSynchronize(s));
@@ -397,7 +536,7 @@ gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
     const uint32_t db = (uint32_t)((bits + passes - 1) / passes);  // bits per pass
     const uint32_t mask = (1u << db) - 1u, digits = mask + 1u;
     const uint32_t tiles = (uint32_t)(((uint64_t)n + kRadixTile - 1) / kRadixTile);
-    DevBuf ka, kb, ib, cnt;
+    StreamBuf ka(s), kb(s), ib(s), cnt(s);
     GS_TRY(cnt.alloc(((size_t)digits * tiles + digits) * 4));
     if (passes > 1) {
         GS_TRY(ka.alloc((size_t)n * 4));
@@ -424,7 +563,6 @@ gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
         kin = kout;
         iin = iout;
     }
-    GS_CUDA(cudaStreamSynchronize(s));  // scratch buffers are freed on return
     return GS_OK;
 }
 
@@ -442,16 +580,11 @@ __global__ void k_max_u32(const uint32_t *d, size_t n, uint32_t *out)
 
 gs_status reduce_max_u32(const uint32_t *d, size_t n, uint32_t *out, cudaStream_t s)
 {
-    uint32_t *dm = nullptr;
-    GS_CUDA(cudaMallocAsync(&dm, sizeof(uint32_t), s));
-    GS_CUDA(cudaMemsetAsync(dm, 0, sizeof(uint32_t), s));
-    if (n) k_max_u32<<<296, 256, 0, s>>>(d, n, dm);
-    cudaError_t le = cudaGetLastError();
-    cudaError_t ce = cudaMemcpyAsync(out, dm, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(dm, s);
-    if (le != cudaSuccess || ce != cudaSuccess)
-        return fail(GS_ERR_CUDA, "max reduce failed: %s",
-                    cudaGetErrorString(le != cudaSuccess ? le : ce));
+    StreamBuf m(s);
+    GS_TRY(m.alloc_zero(sizeof(uint32_t)));
+    if (n) k_max_u32<<<296, 256, 0, s>>>(d, n, m.as<uint32_t>());
+    GS_CHECK_LAUNCH();
+    GS_CUDA(cudaMemcpyAsync(out, m.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;
 }

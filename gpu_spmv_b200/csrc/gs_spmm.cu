@@ -240,8 +240,8 @@ gs_status split_extent(uint32_t units, const uint32_t *uc, const uint32_t *ub, u
 {
     *out = 0;
     if (!units) return GS_OK;
-    DevBuf d;
-    GS_TRY(d.alloc_zero(4, s));
+    StreamBuf d(s);
+    GS_TRY(d.alloc_zero(4));
     k_split_extent<<<blocks_of(units), 256, 0, s>>>(units, uc, ub, d.as<uint32_t>());
     GS_CHECK_LAUNCH();
     GS_CUDA(cudaMemcpyAsync(out, d.p, 4, cudaMemcpyDeviceToHost, s));
@@ -308,7 +308,7 @@ gs_status ensure_mm_scratch(gs_matrix *A, cudaStream_t s)
     if (A->mm_ready) return GS_OK;
     GS_TRY(split_extent(A->k1units, A->k1unit_chunk.as<uint32_t>(), A->k1unit_base.as<uint32_t>(),
                         &A->k1split_units, s));
-    GS_TRY(A->mmpartial.alloc((size_t)A->k1split_units * 32 * 32 * 8 + 8));
+    GS_TRY(A->mmpartial.alloc((size_t)A->k1split_units * 32 * 32 * 8 + 8, s));
     A->mm_ready = true;
     return GS_OK;
 }
@@ -378,7 +378,7 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     if (A->adj_ready) return GS_OK;
     const uint32_t n = A->nrows, m = A->ncols, nnz = A->nnz;
     // forward slot -> CSR index
-    GS_TRY(A->fsrc.alloc((size_t)A->lenVC * 4));
+    GS_TRY(A->fsrc.alloc((size_t)A->lenVC * 4, s));
     GS_CUDA(cudaMemsetAsync(A->fsrc.p, 0xff, (size_t)A->lenVC * 4, s));
     if (n) {
         k_k1_fsrc<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->permi.as<uint32_t>(),
@@ -386,10 +386,10 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
         GS_CHECK_LAUNCH();
     }
     // CSC order of the elements: stable sort of CSR indices by ascending column
-    DevBuf rowidx, key, ccount, csc, cptr;
+    StreamBuf rowidx(s), key(s), ccount(s), csc(s), cptr(s);
     GS_TRY(rowidx.alloc((size_t)nnz * 4));
     GS_TRY(key.alloc((size_t)nnz * 4));
-    GS_TRY(ccount.alloc_zero((size_t)m * 4, s));
+    GS_TRY(ccount.alloc_zero((size_t)m * 4));
     GS_TRY(csc.alloc((size_t)nnz * 4));
     if (n) {
         k_expand_rows<<<blocks_of(n), 256, 0, s>>>(n, d_row, rowidx.as<uint32_t>());
@@ -415,13 +415,13 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(A->tpermi.alloc_zero(((size_t)tchunks + 1) * 32 * 4, s));
     GS_TRY(stable_sort_desc(ccount.as<uint32_t>(), m, maxlen, A->tpermi.as<uint32_t>(), s));
     GS_TRY(A->tnmc.alloc_zero((size_t)tchunks * 4 + 4, s));
-    GS_TRY(A->tlen.alloc((size_t)m * 4 + 4));
+    GS_TRY(A->tlen.alloc((size_t)m * 4 + 4, s));
     if (m) {
         k_t_meta<<<blocks_of(m), 256, 0, s>>>(m, ccount.as<uint32_t>(), A->tpermi.as<uint32_t>(),
                                               A->tnmc.as<uint32_t>(), A->tlen.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
-    DevBuf P;
+    StreamBuf P(s);
     GS_TRY(P.alloc(((size_t)tchunks + 1) * 8));
     uint64_t lenvc = 0;
     {
@@ -432,14 +432,14 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     }
     if (lenvc > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "transposed K1 exceeds 32-bit slots");
     A->tlenVC = (uint32_t)lenvc;
-    GS_TRY(A->tchp.alloc((size_t)tchunks * 4 + 4));
+    GS_TRY(A->tchp.alloc((size_t)tchunks * 4 + 4, s));
     if (tchunks) {
         k_narrow<<<blocks_of(tchunks), 256, 0, s>>>(tchunks, P.as<uint64_t>(), A->tchp.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     const size_t vsz = A->p.vtype == GS_F64 ? 8 : 4;
     GS_TRY(A->trow.alloc_zero((size_t)A->tlenVC * 4, s));
-    GS_TRY(A->tsrc.alloc((size_t)A->tlenVC * 4));
+    GS_TRY(A->tsrc.alloc((size_t)A->tlenVC * 4, s));
     GS_CUDA(cudaMemsetAsync(A->tsrc.p, 0xff, (size_t)A->tlenVC * 4, s));
     GS_TRY(A->tval.alloc_zero((size_t)A->tlenVC * vsz, s));
     if (m) {
@@ -453,10 +453,10 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
                          A->tpartial1, A->tcount, &A->tunits, s));
     GS_TRY(split_extent(A->tunits, A->tunit_chunk.as<uint32_t>(), A->tunit_base.as<uint32_t>(),
                         &A->tsplit_units, s));
-    GS_TRY(A->tpartial.alloc((size_t)A->tsplit_units * 32 * 32 * 8 + 8));
+    GS_TRY(A->tpartial.alloc((size_t)A->tsplit_units * 32 * 32 * 8 + 8, s));
     // transposed values from the stored ones: forward slots -> CSR order (each CSR index
     // sits in exactly one forward slot) -> transposed slots
-    DevBuf vcsr;
+    StreamBuf vcsr(s);
     GS_TRY(vcsr.alloc((size_t)nnz * vsz + 8));
     const unsigned gb = 148u * 16u;
     if (A->p.vtype == GS_F64) {
@@ -474,18 +474,18 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     // forward slot -> adjoint-layout slot, through the CSR index; the CSR index -> slot maps
     // stay: a value gradient in CSR order is formed in slot order (coalesced writes) and then
     // gathered into CSR order, instead of scattering one 4- or 8-byte write per element
-    GS_TRY(A->csr2t.alloc((size_t)nnz * 4 + 4));
-    GS_TRY(A->csr2f.alloc((size_t)nnz * 4 + 4));
-    GS_TRY(A->ftslot.alloc((size_t)A->lenVC * 4 + 4));
+    GS_TRY(A->csr2t.alloc((size_t)nnz * 4 + 4, s));
+    GS_TRY(A->csr2f.alloc((size_t)nnz * 4 + 4, s));
+    GS_TRY(A->ftslot.alloc((size_t)A->lenVC * 4 + 4, s));
     k_invert_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), A->csr2t.as<uint32_t>());
     k_invert_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), A->csr2f.as<uint32_t>());
     k_compose_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), A->csr2t.as<uint32_t>(),
                                      A->ftslot.as<uint32_t>());
-    GS_TRY(A->t2f.alloc((size_t)A->tlenVC * 4 + 4));
+    GS_TRY(A->t2f.alloc((size_t)A->tlenVC * 4 + 4, s));
     k_compose_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), A->csr2f.as<uint32_t>(),
                                      A->t2f.as<uint32_t>());
     GS_CHECK_LAUNCH();
-    GS_TRY(A->vslots.alloc((size_t)max(A->lenVC, A->tlenVC) * vsz + 8));
+    GS_TRY(A->vslots.alloc((size_t)max(A->lenVC, A->tlenVC) * vsz + 8, s));
     A->adj_ready = true;
     GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;

@@ -269,7 +269,7 @@ gs_status build_k1_plan(const uint32_t *d_nmc, uint32_t chunkNum, DevBuf &unit_c
                         DevBuf &unit_base, DevBuf &partial, DevBuf &count, uint32_t *units,
                         cudaStream_t s)
 {
-    DevBuf pre;
+    StreamBuf pre(s);
     GS_TRY(pre.alloc(((size_t)chunkNum + 1) * 8));
     CountSpec spec{CountKind::PiecesMin1};
     spec.arr = d_nmc;
@@ -278,15 +278,14 @@ gs_status build_k1_plan(const uint32_t *d_nmc, uint32_t chunkNum, DevBuf &unit_c
     GS_TRY(exclusive_scan(spec, chunkNum, pre.as<uint64_t>(), &total, s));
     if (total >= 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 plan too large");
     *units = (uint32_t)total;
-    GS_TRY(unit_chunk.alloc((size_t)total * 4));
-    GS_TRY(unit_base.alloc(((size_t)chunkNum + 1) * 4));
-    GS_TRY(partial.alloc((size_t)total * 32 * 8));
+    GS_TRY(unit_chunk.alloc((size_t)total * 4, s));
+    GS_TRY(unit_base.alloc(((size_t)chunkNum + 1) * 4, s));
+    GS_TRY(partial.alloc((size_t)total * 32 * 8, s));
     GS_TRY(count.alloc_zero((size_t)chunkNum * 4, s));
     k_k1_units<<<(chunkNum + 256) / 256, 256, 0, s>>>(pre.as<uint64_t>(), d_nmc, chunkNum,
                                                      unit_chunk.as<uint32_t>(),
                                                      unit_base.as<uint32_t>());
     GS_CHECK_LAUNCH();
-    GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;
 }
 
@@ -338,8 +337,8 @@ gs_status build_k1_deltas(const K1Args &a, const uint32_t *d_col32, uint16_t *d_
                           uint32_t *d_ck, cudaStream_t s)
 {
     if (a.units == 0) return GS_OK;
-    DevBuf flag;
-    GS_TRY(flag.alloc_zero(4, s));
+    StreamBuf flag(s);
+    GS_TRY(flag.alloc_zero(4));
     k_k1_deltas<<<k1_blocks(a.units), 256, 0, s>>>(a, d_col32, d_col16, d_ck,
                                                      flag.as<uint32_t>());
     GS_CHECK_LAUNCH();

@@ -1714,8 +1714,8 @@ gs_status random_columns(const uint32_t *d_row, const uint32_t *d_col, uint32_t 
     if (n == 0) return GS_OK;
     const uint32_t samples = n < 65536u ? n : 65536u;
     const uint32_t stride = n / samples;
-    DevBuf cnt;
-    GS_TRY(cnt.alloc_zero(16, s));
+    StreamBuf cnt(s);
+    GS_TRY(cnt.alloc_zero(16));
     k_col_steps<<<(samples + 255) / 256, 256, 0, s>>>(d_row, d_col, stride, samples,
                                                       cnt.as<unsigned long long>());
     GS_CHECK_LAUNCH();
@@ -1774,18 +1774,18 @@ gs_status build_rows_plan(const uint32_t *d_rpos, const uint32_t *d_rlen, uint32
         k_set_real<<<g, 256, 0, s>>>(n, d_rpos, d_rlen, P.rbits.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
-    DevBuf pre;
+    StreamBuf pre(s);
     GS_TRY(pre.alloc(((size_t)P.nwin + 1) * 8));
     CountSpec cw{CountKind::WindowPopc};
     cw.arr = P.sbits.as<uint32_t>();
     cw.a = V;
     GS_TRY(exclusive_scan(cw, P.nwin, pre.as<uint64_t>(), nullptr, s));
-    GS_TRY(P.wcount.alloc(((size_t)P.nwin + 1) * 4));
+    GS_TRY(P.wcount.alloc(((size_t)P.nwin + 1) * 4, s));
     k_narrow_u32<<<(P.nwin + 256) / 256, 256, 0, s>>>(P.nwin + 1, pre.as<uint64_t>(),
                                                        P.wcount.as<uint32_t>());
     GS_CHECK_LAUNCH();
     // empty rows: rank -> row map and the list of rows to zero
-    DevBuf pe;
+    StreamBuf pe(s);
     GS_TRY(pe.alloc(((size_t)n + 1) * 8));
     CountSpec ce{CountKind::NonEmpty};
     ce.row = d_rpos;
@@ -1793,23 +1793,22 @@ gs_status build_rows_plan(const uint32_t *d_rpos, const uint32_t *d_rlen, uint32
     GS_TRY(exclusive_scan(ce, n, pe.as<uint64_t>(), &nonempty, s));
     P.n_empty = (uint32_t)(n - nonempty);
     if (P.n_empty) {
-        GS_TRY(P.ne.alloc((size_t)nonempty * 4 + 4));
-        GS_TRY(P.empty.alloc((size_t)P.n_empty * 4));
+        GS_TRY(P.ne.alloc((size_t)nonempty * 4 + 4, s));
+        GS_TRY(P.empty.alloc((size_t)P.n_empty * 4, s));
         k_split_rows<<<g, 256, 0, s>>>(n, d_rpos, pe.as<uint64_t>(), P.ne.as<uint32_t>(),
                                        P.empty.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     GS_TRY(P.status.alloc_zero(4, s));
-    GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;
 }
 
 gs_status build_u16_columns(const uint32_t *d_col32, uint32_t nslots, RowsPlan &P,
                             uint16_t *d_col16, cudaStream_t s)
 {
-    GS_TRY(P.colbase.alloc((size_t)P.nwin * 4 + 4));
-    DevBuf flag;
-    GS_TRY(flag.alloc_zero(4, s));
+    GS_TRY(P.colbase.alloc((size_t)P.nwin * 4 + 4, s));
+    StreamBuf flag(s);
+    GS_TRY(flag.alloc_zero(4));
     const uint32_t blocks = min((P.nwin + 7) / 8, 148u * 64u);
     if (blocks)
         k_u16_cols<<<blocks, 256, 0, s>>>(P.nwin, 32u * P.V, nslots,

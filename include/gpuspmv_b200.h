@@ -355,6 +355,11 @@ gs_status gs_spmv_host_stream(const gs_matrix *A, const void *h_x, size_t x_stri
                               gs_dtype xtype, void *h_y, size_t y_stride, gs_dtype ytype,
                               UIN count, UIN flags, gs_stream stream);
 
+/* Device memory of destroyed matrices and of conversions' scratch is kept for the next ones,
+ * up to 1 GiB per device; gs_release_cached gives it back to the device now (the current one;
+ * waits for it). */
+gs_status gs_release_cached(void);
+
 /* Synchronous device -> host copy of `bytes` bytes (for bindings that read a matrix's
  * device arrays back without a CUDA runtime of their own). */
 gs_status gs_copy_to_host(void *h_dst, const void *d_src, size_t bytes);
