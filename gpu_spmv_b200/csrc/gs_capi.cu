@@ -190,6 +190,18 @@ gs_status gs_spmv(const gs_matrix *A, const void *d_x, gs_dtype xtype, void *d_y
         t.rbits = A->plan.padded ? A->plan.rbits.as<uint32_t>() : nullptr;
         return gs::launch_tiles(t, A->tile_w, false, s);
     }
+    if (A->csr_local && !(flags & GS_FLAG_STRIPED)) {  // CSR, COM tileH = 1
+        gs::CsrArgs a{};
+        a.n = A->nrows;
+        a.nnz = A->nnz;
+        a.row = A->rpos.as<uint32_t>();
+        a.colbase = A->plan.colbase.as<uint32_t>();
+        a.val = A->val.p;
+        a.col = A->col.p;
+        a.x = d_x;
+        a.y = d_y;
+        return gs::launch_csr(a, A->p.vtype, A->p.itype, ytype, s);
+    }
     gs::RowsArgs a = gs::rows_args(A->plan);
     a.val = A->val.p;
     a.col = A->col.p;
@@ -311,18 +323,16 @@ gs_status gs_csr_spmv_f64(UIN nrows, UIN ncols, UIN nnz, const UIN *d_row, const
     if ((reinterpret_cast<uintptr_t>(d_val) & 15u) || (reinterpret_cast<uintptr_t>(d_col) & 15u))
         return gs::fail(GS_ERR_INVALID, "val and col must be 16-byte aligned");
     cudaStream_t s = gs::cs(stream);
-    gs::RowsPlan P;
-    uint32_t V = gs::kDirectV;
-    GS_TRY(gs::direct_lane_positions(d_row, d_col, nrows, nnz, &V, s));
-    GS_TRY(gs::build_rows_plan(d_row, nullptr, nrows, V, P, s));
-    gs::RowsArgs a = gs::rows_args(P);
+    gs::CsrArgs a{};
+    a.n = nrows;
+    a.nnz = nnz;
+    a.row = d_row;
     a.val = d_val;
     a.col = d_col;
     a.x = d_x;
     a.y = d_y;
-    a.nslots = nnz;
-    GS_TRY(gs::launch_rows(a, GS_F64, GS_IDX_U32, GS_F64, 0, false, false, false, s));
-    GS_CUDA(cudaStreamSynchronize(s));  // the plan's buffers are released on return
+    GS_TRY(gs::launch_csr(a, GS_F64, GS_IDX_U32, GS_F64, s));
+    GS_CUDA(cudaStreamSynchronize(s));  // y is complete on return
     return GS_OK;
 }
 

@@ -531,8 +531,14 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         // width V is chosen to divide that alignment so the aligned kernel applies.
         uint32_t V = kDirectV;
         bool aligned = false;
-        if (!reduced && !A->tiled && !need_rlen)  // FP64 CSR and COM tileH = 1
-            GS_TRY(direct_lane_positions(d_row, d_col, n, nnz, &V, s));
+        if (!A->tiled && !need_rlen) {  // CSR and COM tileH = 1
+            bool rnd = false, even = true;
+            GS_TRY(random_columns(d_row, d_col, n, &rnd, s, &even));
+            // rows of 1 or 2 FP64 elements stay on the row-stream kernel (3M rows of 1 / 2 / 3:
+            // 18.7 / 25.7 / 45.4 us there, 22.8 / 31.0 / 35.1 on the CSR kernel)
+            A->csr_local = !rnd && even && (reduced || (double)nnz >= 2.5 * n);
+            if (!reduced) V = direct_lane_positions(n, nnz, rnd);
+        }
         if (A->tiled) {
             V = th;
             aligned = fmt == GS_FMT_AXT && p.mode == GS_AXT_UNC &&

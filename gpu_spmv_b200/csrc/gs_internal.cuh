@@ -233,6 +233,7 @@ struct gs_matrix {
     // planned over tiles, for the tile kernel (launch_tiles); tile_w 0 otherwise
     gs::RowsPlan tplan;
     uint32_t tile_w = 0;
+    bool csr_local = false;  // CSR, COM tileH = 1: local columns, even rows (the CSR kernel)
     double conv_ms = 0, mfp = 0, beta = 0;
 };
 
@@ -258,17 +259,19 @@ struct RowsArgs {
 // Positions per lane of the direct (tileH = 1) layouts.
 constexpr uint32_t kDirectV = 8;
 // Positions per lane of an FP64 direct layout with x gathered at run time (CSR, COM
-// tileH = 1), from the CSR row pointers and columns: 4 when rows average fewer than 8
-// elements or fewer than a quarter of a sample of in-row column steps stay within 16
-// columns (the x gathers are random: 4 positions hold 40 registers, 6 blocks per SM, and a
-// lane's 4 values and 4 columns are one 32-byte and one 16-byte request), else 8 (streams
-// with local columns: more bytes in flight per warp).
-gs_status direct_lane_positions(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
-                                uint64_t nnz, uint32_t *V, cudaStream_t s);
+// tileH = 1): 4 when rows average fewer than 8 elements or the x gathers are random (4
+// positions hold 40 registers, 6 blocks per SM, and a lane's 4 values and 4 columns are one
+// 32-byte and one 16-byte request), else 8.
+inline uint32_t direct_lane_positions(uint32_t n, uint64_t nnz, bool random)
+{
+    return random || (double)nnz < 8.0 * n ? 4u : kDirectV;
+}
 // Whether the x gathers of a CSR matrix are close to random: fewer than a quarter of a
-// sample of in-row column steps (up to 32 steps of 65,536 rows) stay within 16 columns.
+// sample of in-row column steps (up to 32 steps of 65,536 rows) stay within 16 columns.  With
+// `even`, also whether rows are even enough to be walked side by side: over a sample of groups
+// of 32 rows, 32 times the longest is at most 2.5 times the elements.
 gs_status random_columns(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
-                         bool *random, cudaStream_t s);
+                         bool *random, cudaStream_t s, bool *even = nullptr);
 // Positions per lane for a layout whose rows start on multiples of `align` positions
 // (0: no alignment): returns the V that makes the aligned kernel apply, or kDirectV.
 uint32_t aligned_lane_positions(uint32_t align, bool *aligned);
@@ -288,6 +291,19 @@ RowsArgs rows_args(const RowsPlan &P);
 gs_status launch_tiles(const RowsArgs &a, uint32_t thw, bool baked, cudaStream_t s);
 gs_status launch_rows(const RowsArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype ytype,
                       uint32_t flags, bool tiled, bool baked, bool padded, cudaStream_t s);
+
+// The CSR product (see gs_spmv_csr.cu): CSR and COM tileH = 1 streams, positions == slots;
+// val and col 16-byte aligned.
+struct CsrArgs {
+    uint32_t n, nnz;
+    const uint32_t *row;       // row pointers
+    const uint32_t *colbase;   // 16-bit columns: base of each 256 positions
+    const void *val, *col, *x;
+    void *y;
+    bool y64;                  // set by launch_csr
+};
+gs_status launch_csr(const CsrArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype ytype,
+                     cudaStream_t s);
 
 // Slot of step j of lane `lane` in the K1 chunk that starts at slot cbase and has nmc
 // steps.  The reference's order is cbase + 32 j + lane (a warp's loads of one step are

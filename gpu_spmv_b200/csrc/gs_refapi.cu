@@ -512,11 +512,26 @@ str_res test_gcsr(const UIN cudaBlockSize, const str_matCSR m, const FPT *vec, c
 {
     (void)cudaBlockSize;
     DevBuf row, col, val, x, y;
-    gs::RowsPlan P;
-    uint32_t V = gs::kDirectV;
+    bool rnd = false, even = true;
     if (upload_csr(m, row, col, val) || h2d(x, vec, m.nrows) || y.alloc((size_t)m.nrows * 8) ||
-        gs::direct_lane_positions(row.as<UIN>(), col.as<UIN>(), m.nrows, m.nnz, &V, 0) ||
-        gs::build_rows_plan(row.as<UIN>(), nullptr, m.nrows, V, P, 0))
+        gs::random_columns(row.as<UIN>(), col.as<UIN>(), m.nrows, &rnd, 0, &even))
+        return error_res("gcsr", gs_last_error());
+    if (!rnd && even && (double)m.nnz >= 2.5 * m.nrows) {
+        gs::CsrArgs c{};
+        c.n = m.nrows;
+        c.nnz = m.nnz;
+        c.row = row.as<UIN>();
+        c.val = val.p;
+        c.col = col.p;
+        c.x = x.p;
+        c.y = y.p;
+        return timed("gcsr", m.nrows, m.nnz, [&]() {
+            return gs::launch_csr(c, GS_F64, GS_IDX_U32, GS_F64, 0);
+        }, y, ref);
+    }
+    gs::RowsPlan P;
+    if (gs::build_rows_plan(row.as<UIN>(), nullptr, m.nrows,
+                            gs::direct_lane_positions(m.nrows, m.nnz, rnd), P, 0))
         return error_res("gcsr", gs_last_error());
     gs::RowsArgs a = gs::rows_args(P);
     a.val = val.p;

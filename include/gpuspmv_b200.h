@@ -364,10 +364,9 @@ gs_status gs_release_cached(void);
  * device arrays back without a CUDA runtime of their own). */
 gs_status gs_copy_to_host(void *h_dst, const void *d_src, size_t bytes);
 
-/* CSR SpMV straight from device CSR arrays: y = A x, FP64.  Builds the kernel's row-start
- * plan on every call and returns when y is complete; for repeated products convert once
- * with gs_matrix_create(GS_FMT_CSR) and call gs_spmv.  val and col must be 16-byte
- * aligned. */
+/* CSR SpMV straight from device CSR arrays: y = A x, FP64, in one kernel on the row pointers;
+ * returns when y is complete.  For repeated products convert once with
+ * gs_matrix_create(GS_FMT_CSR) and call gs_spmv.  val and col must be 16-byte aligned. */
 gs_status gs_csr_spmv_f64(UIN nrows, UIN ncols, UIN nnz, const UIN *d_row, const UIN *d_col,
                           const double *d_val, const double *d_x, double *d_y,
                           gs_stream stream);
