@@ -878,6 +878,7 @@ gs_status gs_batch_create(gs_batch **out, UIN count, gs_matrix *const *mats, con
         a.unit_base = A->k1unit_base.as<uint32_t>();
         a.units = A->k1units;
         a.split_units = A->k1split_units;
+        a.split_extra = A->k1units - A->chunkNum;
         a.partial = A->mmpartial.p;
         a.count = B->d_counts.as<uint32_t>() + B->count_off[i];
     }

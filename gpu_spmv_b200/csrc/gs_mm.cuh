@@ -126,6 +126,7 @@ struct MMArgs {
                                                // layout's slot order, padding slots zero
     const uint32_t *unit_chunk, *unit_base;
     uint32_t units, split_units;               // units < split_units may be pieces
+    uint32_t split_extra;                      // units - chunks
     void *partial;                             // split_units * ld * 32 values
     uint32_t *count;                           // chunks * nrb arrival counters
     uint32_t ld;                               // row stride of X, Y (= K for one block)
@@ -149,9 +150,16 @@ __device__ __forceinline__ void mm_unit(const MMArgs &a, uint32_t u, uint32_t rb
     const int lane = threadIdx.x & 31;
     const uint32_t ld = a.ld;
     {
-        const uint32_t c = __ldg(a.unit_chunk + u);
-        const uint32_t ub = __ldg(a.unit_base + c);
-        const uint32_t np = __ldg(a.unit_base + c + 1) - ub;
+        // split chunks come first (chunks are sorted by decreasing length): from split_units on a
+        // unit is a whole chunk, found without the plan's two dependent loads
+        uint32_t c, ub = u, np = 1;
+        if (u >= a.split_units) {
+            c = u - a.split_extra;
+        } else {
+            c = __ldg(a.unit_chunk + u);
+            ub = __ldg(a.unit_base + c);
+            np = __ldg(a.unit_base + c + 1) - ub;
+        }
         const uint32_t piece = u - ub;
         const uint32_t g = 32u * c + (uint32_t)lane;
         const bool valid = g < a.nrows;
@@ -167,16 +175,24 @@ __device__ __forceinline__ void mm_unit(const MMArgs &a, uint32_t u, uint32_t rb
         T acc[K];
 #pragma unroll
         for (int k = 0; k < K; k++) acc[k] = T(0);
-        for (uint32_t j = j0; j < j1; j += B) {
-            T v[B], gv[B][K];
-            uint32_t cc[B];
+        // the values and columns of the next B steps load while this B's rows are gathered: their
+        // HBM latency came between every two batches of gathers (FP32 k = 8 on a 524,288-row
+        // power-law 58.4 -> 48.0 us together with the launch shape in gs_spmm.cu)
+        T v[B];
+        uint32_t cc[B];
+        auto streams = [&](uint32_t j, T(&sv)[B], uint32_t(&sc)[B]) {
 #pragma unroll
             for (int b = 0; b < B; b++) {
                 const bool in = j + b < j1;
                 const uint32_t pos = base + 32u * (j + b);
-                v[b] = in ? __ldcs(val + pos) : T(0);
-                cc[b] = in ? __ldcs(a.col + pos) : 0u;
+                sv[b] = in ? __ldcs(val + pos) : T(0);
+                sc[b] = in ? __ldcs(a.col + pos) : 0u;
             }
+        };
+        streams(j0, v, cc);
+        for (uint32_t j = j0; j < j1; j += B) {
+            T gv[B][K], vn[B];
+            uint32_t cn[B];
 #pragma unroll
             for (int b = 0; b < B; b++) {
                 if (j + b < j1) load_row<T, K>(xin, cc[b], ld, gv[b]);
@@ -185,6 +201,7 @@ __device__ __forceinline__ void mm_unit(const MMArgs &a, uint32_t u, uint32_t rb
                     for (int k = 0; k < K; k++) gv[b][k] = T(0);
                 }
             }
+            streams(j + B, vn, cn);
 #pragma unroll
             for (int b = 0; b < B; b++) {
                 if (j + b < j1) {
@@ -204,6 +221,11 @@ __device__ __forceinline__ void mm_unit(const MMArgs &a, uint32_t u, uint32_t rb
                         }
                     }
                 }
+            }
+#pragma unroll
+            for (int b = 0; b < B; b++) {
+                v[b] = vn[b];
+                cc[b] = cn[b];
             }
         }
         if constexpr (ADJ) {

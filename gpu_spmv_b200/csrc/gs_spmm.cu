@@ -28,8 +28,20 @@ namespace {
 
 using namespace mm;
 
+// Blocks of 2 warps (a place on the SM is free when two units end: FP32 k = 8 on a 524,288-row
+// power-law 53.9 us in blocks of 8, 52.0 in blocks of 2), and registers for the rows in flight
+// before warps: the gathers are bound by the L1's line requests, which 16 warps of 4 to 8 rows in
+// flight per lane keep busy (32 warps capped at 64 registers 52.0 us, 24 49.6, 16 48.0, the start
+// 58.4; k = 4 101 -> 46, FP64 k = 2 118 -> 44).  Rows of 64 bytes and more hold to 24 warps (FP64
+// k = 8 on a band 62.5 -> 60.4 us; with 16 64.6).
+constexpr int kMMThreads = 64;
+// One right-hand side streams: 32 warps (FP64 on a 27-point stencil 80^3 33.6 -> 31.1 us; with 16
+// 40.3).
+template <class T, int K>
+constexpr int kMMBlocks = (K == 1 ? 32 : (K * (int)sizeof(T) >= 64 ? 24 : 16)) / 2;
+
 template <class T, int K, bool ADJ>
-__global__ void __launch_bounds__(256) k_k1_mm(const MMArgs a)
+__global__ void __launch_bounds__(kMMThreads, kMMBlocks<T, K>) k_k1_mm(const MMArgs a)
 {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < a.units;
@@ -253,14 +265,14 @@ template <class T, bool ADJ>
 gs_status launch_mm(const MMArgs &a, uint32_t k, cudaStream_t s)
 {
     if (!a.units) return GS_OK;
-    const uint32_t blocks = min((a.units + 7) / 8, 148u * 64u);
+    const uint32_t blocks = (a.units + kMMThreads / 32 - 1) / (kMMThreads / 32);
     switch (k) {
-    case 1: k_k1_mm<T, 1, ADJ><<<blocks, 256, 0, s>>>(a); break;
-    case 2: k_k1_mm<T, 2, ADJ><<<blocks, 256, 0, s>>>(a); break;
-    case 4: k_k1_mm<T, 4, ADJ><<<blocks, 256, 0, s>>>(a); break;
-    case 8: k_k1_mm<T, 8, ADJ><<<blocks, 256, 0, s>>>(a); break;
-    case 16: k_k1_mm<T, 16, ADJ><<<blocks, 256, 0, s>>>(a); break;
-    case 32: k_k1_mm<T, 32, ADJ><<<blocks, 256, 0, s>>>(a); break;
+    case 1: k_k1_mm<T, 1, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 2: k_k1_mm<T, 2, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 4: k_k1_mm<T, 4, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 8: k_k1_mm<T, 8, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 16: k_k1_mm<T, 16, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 32: k_k1_mm<T, 32, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
     default: return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1, 2, 4, 8, 16, 32)", k);
     }
     GS_CHECK_LAUNCH();
@@ -360,6 +372,7 @@ gs_status gs_spmm(gs_matrix *A, const void *d_X, void *d_Y, gs_dtype dtype, UIN 
     a.unit_base = A->k1unit_base.as<uint32_t>();
     a.units = A->k1units;
     a.split_units = A->k1split_units;
+    a.split_extra = A->k1units - A->chunkNum;
     a.partial = A->mmpartial.p;
     a.count = A->k1count.as<uint32_t>();
     a.ld = k;
@@ -619,6 +632,7 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     a.unit_base = A->tunit_base.as<uint32_t>();
     a.units = A->tunits;
     a.split_units = A->tsplit_units;
+    a.split_extra = A->tunits - A->tchunkNum;
     a.partial = A->tpartial.p;
     a.count = A->tcount.as<uint32_t>();
     a.ld = k;
