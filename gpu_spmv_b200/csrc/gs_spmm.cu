@@ -13,9 +13,10 @@
 // Deterministic mode: the transpose is stored as its own K1 layout, built once by
 // gs_matrix_prepare_adjoint (columns of A sorted by decreasing length, each transposed slot
 // remembering the CSR index of its element and its row), and Xbar is the forward kernel run
-// on it; the same pass gathers Ybar[row_e] for Xbar and forms vbar_e against X[col] held in
-// registers, so vbar costs no extra gather.  Atomic mode: the forward layout, with Xbar
-// accumulated by atomic adds (its rounding order varies between runs).
+// on it.  vbar in CSR order is a pass of its own over the elements (k_vbar); in the transposed
+// layout's slot order the pass that gathers Ybar[row_e] for Xbar also forms vbar_e against
+// X[col] held in registers.  Atomic mode: the forward layout, with Xbar accumulated by atomic
+// adds (its rounding order varies between runs).
 //
 // The reference has no multi-RHS product and no adjoint; these extend its K1 format.
 #include <mutex>
@@ -134,6 +135,111 @@ __global__ void __launch_bounds__(256) k_k1_adj_atomic(const AtomicArgs a)
     }
 }
 
+// ------------------------------------------------------------------ value gradient
+// vbar_e = Ybar[row_e] . X[col_e] in CSR order, from the elements' rows and columns: L lanes of
+// VEC columns (32 bytes at most) per element.  A row's elements are neighbours, so Ybar's rows come
+// from L1 and the X gathers set the pace, one line request an element (FP32 k = 8, 16.8M elements:
+// 60 us at the rate of bare gathers, 93 us here; the indices of the next step load while this
+// one's rows are gathered, without which it took 145).  Before, the transposed pass formed vbar
+// beside Xbar in its own slot order and another kernel permuted it: 122 + 83 us, where Xbar alone
+// is 84 us.
+struct VbarArgs {
+    uint32_t nnz;
+    const uint32_t *row, *col;
+    const void *x, *ybar;
+    void *vbar;
+};
+
+template <class T, int VEC>
+__device__ __forceinline__ void load_slice(const T *p, T (&v)[VEC])
+{
+    if constexpr (VEC * sizeof(T) == 32) {
+        ld32(p, v);
+    } else if constexpr (VEC * sizeof(T) == 16) {
+        load_row<T, VEC>(p, 0, 0, v);
+    } else {
+#pragma unroll
+        for (int i = 0; i < VEC; i++) v[i] = __ldg(p + i);
+    }
+}
+
+constexpr int kVbarThreads = 64;
+constexpr int kVbarSteps = 8;  // steps of a warp, over consecutive elements (32: 2 % slower)
+constexpr int kVbarUnroll = 2;  // elements per lane and step (1 / 4: 4 / 2 % slower in all)
+template <class T, int K>
+__global__ void __launch_bounds__(kVbarThreads, 12) k_vbar(const VbarArgs a)
+{
+    using A = Arith<T>;
+    constexpr int L = K * (int)sizeof(T) > 32 ? K * (int)sizeof(T) / 32 : 1;
+    constexpr int VEC = K / L;
+    constexpr int U = kVbarUnroll, E = 32 / L * U;  // elements per step
+    const int lane = threadIdx.x & 31, li = lane % L;
+    const uint64_t warp = blockIdx.x * (uint64_t)(kVbarThreads / 32) + (threadIdx.x >> 5);
+    const T *__restrict__ x = static_cast<const T *>(a.x) + li * VEC;
+    const T *__restrict__ yb = static_cast<const T *>(a.ybar) + li * VEC;
+    T *__restrict__ vbar = static_cast<T *>(a.vbar);
+    uint64_t e0 = warp * (uint64_t)(E * kVbarSteps) + (uint64_t)(lane / L);
+    uint32_t r[U], c[U];
+    auto indices = [&](uint64_t e, uint32_t(&ri)[U], uint32_t(&ci)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool in = e + (uint64_t)(u * (32 / L)) < a.nnz;
+            ri[u] = in ? __ldcs(a.row + e + u * (32 / L)) : 0u;
+            ci[u] = in ? __ldcs(a.col + e + u * (32 / L)) : 0u;
+        }
+    };
+    indices(e0, r, c);
+    for (int t = 0; t < kVbarSteps; t++, e0 += E) {
+        if (e0 - (uint64_t)(lane / L) >= a.nnz) break;  // the whole warp
+        T xs[U][VEC], ys[U][VEC];
+        uint32_t rn[U], cn[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (e0 + (uint64_t)(u * (32 / L)) < a.nnz) {
+                load_slice<T, VEC>(x + (size_t)c[u] * K, xs[u]);
+                load_slice<T, VEC>(yb + (size_t)r[u] * K, ys[u]);
+            }
+        }
+        // the next step's indices load while this one's rows are gathered
+        if (t + 1 < kVbarSteps) indices(e0 + E, rn, cn);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint64_t e = e0 + (uint64_t)(u * (32 / L));
+            T d = T(0);  // the sum goes from lane to lane, in the order of the right-hand sides
+#pragma unroll
+            for (int st = 0; st < L; st++) {
+                T q = st ? __shfl_up_sync(0xffffffffu, d, 1) : T(0);
+                if (e < a.nnz) {
+#pragma unroll
+                    for (int k = 0; k < VEC; k++) q = A::add(q, A::mul(ys[u][k], xs[u][k]));
+                }
+                if (li == st) d = q;
+            }
+            if (li == L - 1 && e < a.nnz) __stcs(vbar + e, d);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) r[u] = rn[u], c[u] = cn[u];
+    }
+}
+
+template <class T> gs_status launch_vbar(const VbarArgs &a, uint32_t k, cudaStream_t s)
+{
+    if (!a.nnz) return GS_OK;
+#define GS_V(K_)                                                                            \
+    case K_: {                                                                              \
+        const uint32_t l = max(1u, K_ * (uint32_t)sizeof(T) / 32u), per = (uint32_t)(kVbarThreads / 32 * kVbarSteps * kVbarUnroll) * (32u / l); \
+        k_vbar<T, K_><<<(a.nnz - 1u) / per + 1u, kVbarThreads, 0, s>>>(a);                          \
+        break;                                                                              \
+    }
+    switch (k) {
+        GS_V(1u) GS_V(2u) GS_V(4u) GS_V(8u) GS_V(16u) GS_V(32u)
+    default: return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1, 2, 4, 8, 16, 32)", k);
+    }
+#undef GS_V
+    GS_CHECK_LAUNCH();
+    return GS_OK;
+}
+
 // ------------------------------------------------------------------ layout helpers
 // fsrc[slot] = CSR index of the element in K1 slot `slot` (kNoSrc for padding)
 __global__ void k_k1_fsrc(uint32_t n, const uint32_t *row, const uint32_t *permi,
@@ -186,11 +292,27 @@ __global__ void k_compose_map(size_t n, const uint32_t *a, const uint32_t *b, ui
     }
 }
 
-__global__ void k_expand_rows(uint32_t n, const uint32_t *row, uint32_t *rowidx)
+// rowidx[e] = row of CSR element e: a warp per 32 rows, in element order (coalesced writes; the
+// row by a search of the 32 row pointers the lanes hold).  One thread per row wrote 4.2M elements
+// in 69 us.
+__global__ void k_expand_rows(uint32_t n, const uint32_t *__restrict__ row,
+                              uint32_t *__restrict__ rowidx)
 {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    for (uint32_t e = row[r]; e < row[r + 1]; e++) rowidx[e] = r;
+    const uint32_t r0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u;
+    if (r0 >= n) return;
+    const uint32_t lane = threadIdx.x & 31u, nr = min(32u, n - r0);
+    const uint32_t b = row[r0], tot = row[r0 + nr] - b;
+    const uint32_t st = row[min(r0 + lane, n)] - b;  // start of row r0 + lane
+    for (uint32_t t = 0; t < tot; t += 32u) {
+        const uint32_t e = t + lane;
+        uint32_t r = 0;  // last of the nr rows that starts at or before e
+#pragma unroll
+        for (uint32_t d = 16; d; d >>= 1) {
+            const uint32_t s = __shfl_sync(0xffffffffu, st, (int)min(r + d, 31u));
+            if (r + d < nr && s <= e) r += d;
+        }
+        if (e < tot) rowidx[b + e] = r0 + r;
+    }
 }
 
 __global__ void k_col_keys(uint32_t nnz, uint32_t ncols, const uint32_t *col, uint32_t *key,
@@ -399,13 +521,17 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
         GS_CHECK_LAUNCH();
     }
     // CSC order of the elements: stable sort of CSR indices by ascending column
-    StreamBuf rowidx(s), key(s), ccount(s), csc(s), cptr(s);
-    GS_TRY(rowidx.alloc((size_t)nnz * 4));
+    StreamBuf key(s), ccount(s), csc(s), cptr(s);
+    // row and column of each element, for value gradients in CSR order
+    GS_TRY(A->vrow.alloc((size_t)nnz * 4, s));
+    GS_TRY(A->vcol.alloc((size_t)nnz * 4, s));
+    if (nnz)
+        GS_CUDA(cudaMemcpyAsync(A->vcol.p, d_col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
     GS_TRY(key.alloc((size_t)nnz * 4));
     GS_TRY(ccount.alloc_zero((size_t)m * 4));
     GS_TRY(csc.alloc((size_t)nnz * 4));
     if (n) {
-        k_expand_rows<<<blocks_of(n), 256, 0, s>>>(n, d_row, rowidx.as<uint32_t>());
+        k_expand_rows<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->vrow.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     if (nnz) {
@@ -457,7 +583,7 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(A->tval.alloc_zero((size_t)A->tlenVC * vsz, s));
     if (m) {
         k_t_fill<<<blocks_of(m), 256, 0, s>>>(m, A->tpermi.as<uint32_t>(), cptr.as<uint64_t>(),
-                                              csc.as<uint32_t>(), rowidx.as<uint32_t>(),
+                                              csc.as<uint32_t>(), A->vrow.as<uint32_t>(),
                                               A->tchp.as<uint32_t>(), A->trow.as<uint32_t>(),
                                               A->tsrc.as<uint32_t>());
         GS_CHECK_LAUNCH();
@@ -484,18 +610,17 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
                                                 vcsr.as<float>(), A->tval.as<float>());
     }
     GS_CHECK_LAUNCH();
-    // forward slot -> adjoint-layout slot, through the CSR index; the CSR index -> slot maps
-    // stay: a value gradient in CSR order is formed in slot order (coalesced writes) and then
-    // gathered into CSR order, instead of scattering one 4- or 8-byte write per element
-    GS_TRY(A->csr2t.alloc((size_t)nnz * 4 + 4, s));
-    GS_TRY(A->csr2f.alloc((size_t)nnz * 4 + 4, s));
+    // forward slot <-> adjoint-layout slot, through the CSR index
+    StreamBuf csr2t(s), csr2f(s);
+    GS_TRY(csr2t.alloc((size_t)nnz * 4 + 4));
+    GS_TRY(csr2f.alloc((size_t)nnz * 4 + 4));
     GS_TRY(A->ftslot.alloc((size_t)A->lenVC * 4 + 4, s));
-    k_invert_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), A->csr2t.as<uint32_t>());
-    k_invert_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), A->csr2f.as<uint32_t>());
-    k_compose_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), A->csr2t.as<uint32_t>(),
+    k_invert_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), csr2t.as<uint32_t>());
+    k_invert_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), csr2f.as<uint32_t>());
+    k_compose_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), csr2t.as<uint32_t>(),
                                      A->ftslot.as<uint32_t>());
     GS_TRY(A->t2f.alloc((size_t)A->tlenVC * 4 + 4, s));
-    k_compose_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), A->csr2f.as<uint32_t>(),
+    k_compose_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), csr2f.as<uint32_t>(),
                                      A->t2f.as<uint32_t>());
     GS_CHECK_LAUNCH();
     GS_TRY(A->vslots.alloc((size_t)max(A->lenVC, A->tlenVC) * vsz + 8, s));
@@ -580,6 +705,20 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     cudaStream_t s = cs(stream);
     const bool f64 = A->p.vtype == GS_F64;
     const unsigned gb = 148u * 16u;
+    if (mode != GS_ADJ_ATOMIC && mode != GS_ADJ_DETERMINISTIC)
+        return fail(GS_ERR_INVALID, "unknown adjoint mode %d", (int)mode);
+    // a value gradient in CSR order has its own kernel; one in slot order comes with Xbar
+    const bool csr_vbar = d_vbar && vbar_order == GS_VALUES_CSR;
+    if (csr_vbar) {
+        VbarArgs v{};
+        v.nnz = A->nnz;
+        v.row = A->vrow.as<uint32_t>();
+        v.col = A->vcol.as<uint32_t>();
+        v.x = d_X;
+        v.ybar = d_Ybar;
+        v.vbar = d_vbar;
+        GS_TRY((f64 ? launch_vbar<double>(v, k, s) : launch_vbar<float>(v, k, s)));
+    }
     if (mode == GS_ADJ_ATOMIC) {
         GS_CUDA(cudaMemsetAsync(d_Xbar, 0, (size_t)A->ncols * k * (f64 ? 8 : 4), s));
         AtomicArgs a{};
@@ -588,8 +727,8 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         a.chp = A->chp.as<uint32_t>();
         a.klen = A->k1len.as<uint32_t>();
         a.col = A->col.as<uint32_t>();
-        // vbar in forward slot order first (coalesced), then gathered into the asked order
-        const bool via_slots = d_vbar != nullptr;
+        // vbar in forward slot order first (coalesced), then gathered into the adjoint layout's
+        const bool via_slots = d_vbar && !csr_vbar;
         a.unit_chunk = A->k1unit_chunk.as<uint32_t>();
         a.unit_base = A->k1unit_base.as<uint32_t>();
         a.units = A->k1units;
@@ -597,12 +736,11 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         a.x = d_X;
         a.ybar = d_Ybar;
         a.xbar = d_Xbar;
-        a.vbar = via_slots ? A->vslots.p : d_vbar;
+        a.vbar = via_slots ? A->vslots.p : nullptr;
         GS_TRY((f64 ? launch_atomic<double>(a, k, s) : launch_atomic<float>(a, k, s)));
         if (via_slots) {
-            const bool csr = vbar_order == GS_VALUES_CSR;
-            const size_t n_out = csr ? A->nnz : A->tlenVC;
-            const uint32_t *map = csr ? A->csr2f.as<uint32_t>() : A->t2f.as<uint32_t>();
+            const size_t n_out = A->tlenVC;
+            const uint32_t *map = A->t2f.as<uint32_t>();
             if (f64)
                 k_gather_vals<double><<<gb, 256, 0, s>>>(n_out, map, A->vslots.as<double>(),
                                                          static_cast<double *>(d_vbar));
@@ -613,7 +751,6 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         }
         return GS_OK;
     }
-    if (mode != GS_ADJ_DETERMINISTIC) return fail(GS_ERR_INVALID, "unknown adjoint mode %d", (int)mode);
     MMArgs a{};
     a.nrows = A->ncols;
     a.permi = A->tpermi.as<uint32_t>();
@@ -625,9 +762,7 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     a.xin = d_Ybar;
     a.xrow = d_X;
     a.yout = d_Xbar;
-    // CSR order: vbar in the adjoint layout's slot order first, then gathered into CSR order
-    const bool via_slots = d_vbar && vbar_order == GS_VALUES_CSR;
-    a.vbar = via_slots ? A->vslots.p : d_vbar;
+    a.vbar = csr_vbar ? nullptr : d_vbar;
     a.unit_chunk = A->tunit_chunk.as<uint32_t>();
     a.unit_base = A->tunit_base.as<uint32_t>();
     a.units = A->tunits;
@@ -637,19 +772,8 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     a.count = A->tcount.as<uint32_t>();
     a.ld = k;
     a.nrb = 1;
-    GS_TRY((f64 ? launch_mm<double, true>(a, k, s) : launch_mm<float, true>(a, k, s)));
-    if (via_slots) {
-        if (f64)
-            k_gather_vals<double><<<gb, 256, 0, s>>>(A->nnz, A->csr2t.as<uint32_t>(),
-                                                     A->vslots.as<double>(),
-                                                     static_cast<double *>(d_vbar));
-        else
-            k_gather_vals<float><<<gb, 256, 0, s>>>(A->nnz, A->csr2t.as<uint32_t>(),
-                                                    A->vslots.as<float>(),
-                                                    static_cast<float *>(d_vbar));
-        GS_CHECK_LAUNCH();
-    }
-    return GS_OK;
+    if (a.vbar) return f64 ? launch_mm<double, true>(a, k, s) : launch_mm<float, true>(a, k, s);
+    return f64 ? launch_mm<double, false>(a, k, s) : launch_mm<float, false>(a, k, s);
 }
 
 }  // extern "C"

@@ -206,9 +206,10 @@ class Matrix:
             raise TypeError("vbar needs X")
         Xbar = torch.empty(self.ncols, k, dtype=dt, device=Ybar.device)
         nv = self._order_len(order)
-        vbar = torch.zeros(nv, dtype=dt, device=Ybar.device) if want_vbar else None
-        part = torch.zeros(nv, dtype=dt, device=Ybar.device) if want_vbar else None
         blocks = self._blocks(k)
+        new = torch.empty if blocks else torch.zeros
+        vbar = new(nv, dtype=dt, device=Ybar.device) if want_vbar else None
+        part = torch.empty_like(vbar) if want_vbar and len(blocks) > 1 else None
         for i, (c0, w, kp) in enumerate(blocks):
             def padded(T, rows):
                 Tb = T[:, c0:c0 + w]
@@ -219,14 +220,16 @@ class Matrix:
                 return P
             Yb = padded(Ybar, self.nrows)
             Xin = padded(X, self.ncols) if want_vbar else None
-            Xo = torch.empty(self.ncols, kp, dtype=dt, device=Ybar.device)
-            vout = (vbar if len(blocks) == 1 else part) if want_vbar else None
+            whole = kp == w and w == k
+            Xo = Xbar if whole else torch.empty(self.ncols, kp, dtype=dt, device=Ybar.device)
+            vout = vbar if i == 0 else part  # written whole, padding slots included
             L.check(L.lib().gs_spmm_adjoint(
                 self._h, Yb.data_ptr(), Xin.data_ptr() if Xin is not None else None,
                 Xo.data_ptr(), vout.data_ptr() if vout is not None else None, self.vtype, kp,
                 m, self.ORDERS[order], stream_handle(stream)), "gs_spmm_adjoint")
-            Xbar[:, c0:c0 + w] = Xo[:, :w]
-            if want_vbar and len(blocks) > 1:
+            if not whole:
+                Xbar[:, c0:c0 + w] = Xo[:, :w]
+            if want_vbar and i > 0:
                 vbar += part
         return Xbar, vbar
 

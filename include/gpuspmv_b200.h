@@ -406,8 +406,8 @@ gs_status gs_matrix_convert_values(const gs_matrix *A, const void *d_in,
 /* Xbar = A^T Ybar (Xbar [ncols][k], overwritten) and, when d_vbar is given,
  * vbar[e] = sum_r Ybar[row_e][r] * X[col_e][r] for every stored element e, in vbar_order
  * (the gradient with respect to the values; d_X is then required).  X, Ybar and Xbar are
- * 32-byte aligned.  A CSR-order vbar is formed in slot order in a buffer of the matrix and
- * gathered into CSR order (coalesced writes), so calls on one matrix must not overlap.
+ * 32-byte aligned.  The atomic mode forms a slot-order vbar in a buffer of the matrix first, so
+ * calls on one matrix must not overlap.
  * The atomic mode without d_vbar reads neither X nor a second copy of the values. */
 gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, void *d_Xbar,
                           void *d_vbar, gs_dtype dtype, UIN k, gs_adjoint_mode mode,
