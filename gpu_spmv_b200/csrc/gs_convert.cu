@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "gs_internal.cuh"
+#include "gs_k1_fill.cuh"
 
 namespace gs {
 
@@ -110,52 +111,12 @@ __global__ void __launch_bounds__(256) k_fill(const FillArgs f)
     }
 }
 
-// one warp per K1 work unit (a kK1Split-step piece of a 32-row chunk), lane = sorted row
-// g of the chunk: its elements e of the piece -> k1_slot(chp[c], nmc[c], e, g % 32); a chunk
-// of long rows is filled by as many warps as it has pieces
-template <class VIN, class VOUT>
-__global__ void k_fill_k1(uint32_t n, uint32_t units, const uint32_t *unit_chunk,
-                          const uint32_t *unit_base, const uint32_t *row, const uint32_t *col,
-                          const VIN *val, const uint32_t *permi, const uint32_t *chp,
-                          const uint32_t *nmc, bool blocked, VOUT *oval, uint32_t *ocol)
-{
-    const uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint32_t lane = threadIdx.x & 31u;
-    if (u >= units) return;
-    const uint32_t c = unit_chunk[u], j0 = (u - unit_base[c]) * kK1Split;
-    const uint32_t g = 32u * c + lane;
-    if (g >= n) return;
-    const uint32_t r = permi[g], b = row[r], len = row[r + 1] - b;
-    const uint32_t cb = chp[c], m = nmc[c], j1 = min(len, j0 + kK1Split);
-    for (uint32_t e = j0; e < j1; e++) {
-        const uint32_t pos = k1_slot(cb, m, e, lane, blocked);
-        oval[pos] = cvt<VIN, VOUT>(val[b + e]);
-        ocol[pos] = col[b + e];
-    }
-}
-
 template <class VIN>
-void launch_fill_k1(uint32_t n, uint32_t units, const uint32_t *unit_chunk,
-                    const uint32_t *unit_base, const uint32_t *row, const uint32_t *col,
-                    const VIN *val, const uint32_t *permi, const uint32_t *chp,
-                    const uint32_t *nmc, bool blocked, gs_dtype vout, void *oval, uint32_t *ocol,
-                    cudaStream_t s)
+gs_status launch_fill_k1(const k1fill::Args &a, gs_dtype vout, cudaStream_t s)
 {
-    if (!units) return;
-    const unsigned b = (units + 7) / 8;
-    if (vout == GS_F64)
-        k_fill_k1<VIN, double><<<b, 256, 0, s>>>(n, units, unit_chunk, unit_base, row, col, val,
-                                                 permi, chp, nmc, blocked,
-                                                 static_cast<double *>(oval), ocol);
-    else if (vout == GS_F32)
-        k_fill_k1<VIN, float><<<b, 256, 0, s>>>(n, units, unit_chunk, unit_base, row, col, val,
-                                                permi, chp, nmc, blocked,
-                                                static_cast<float *>(oval), ocol);
-    else
-        k_fill_k1<VIN, __nv_bfloat16><<<b, 256, 0, s>>>(n, units, unit_chunk, unit_base, row,
-                                                        col, val, permi, chp, nmc, blocked,
-                                                        static_cast<__nv_bfloat16 *>(oval),
-                                                        ocol);
+    if (vout == GS_F64) return k1fill::fill<VIN, double, true>(a, 0.0, s);
+    if (vout == GS_F32) return k1fill::fill<VIN, float, true>(a, 0.f, s);
+    return k1fill::fill<VIN, __nv_bfloat16, true>(a, __nv_bfloat16(0.f), s);
 }
 
 // first tile of each row (and the tile count at [n]): rpos / w
@@ -191,13 +152,15 @@ __global__ void k_tables(uint32_t n, const uint64_t *P, int mode, uint32_t w, ui
     }
 }
 
-__global__ void k_k1_meta(uint32_t n, uint32_t chunkNum, const uint32_t *rl,
-                          const uint32_t *permi, uint32_t *nmc, uint32_t *klen)
+// of each sorted row its length and first element; of each chunk its steps
+__global__ void k_k1_meta(uint32_t n, const uint32_t *row, const uint32_t *permi, uint32_t *nmc,
+                          uint32_t *klen, uint32_t *kstart)
 {
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < n) {
-        uint32_t l = rl[permi[g]];
+        const uint32_t r = permi[g], b = row[r], l = row[r + 1] - b;
         klen[g] = l;
+        kstart[g] = b;
         if ((g & 31) == 0) nmc[g >> 5] = l;
     }
 }
@@ -314,9 +277,11 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         GS_TRY(stable_sort_desc(rl.as<uint32_t>(), n, maxlen, A->permi.as<uint32_t>(), s));
         GS_TRY(A->nmc.alloc_zero((size_t)chunkNum * 4, s));
         GS_TRY(A->k1len.alloc((size_t)n * 4, s));
-        k_k1_meta<<<blocks_for(n), 256, 0, s>>>(n, chunkNum, rl.as<uint32_t>(),
-                                                A->permi.as<uint32_t>(), A->nmc.as<uint32_t>(),
-                                                A->k1len.as<uint32_t>());
+        StreamBuf kstart(s);
+        GS_TRY(kstart.alloc((size_t)n * 4));
+        k_k1_meta<<<blocks_for(n), 256, 0, s>>>(n, d_row, A->permi.as<uint32_t>(),
+                                                A->nmc.as<uint32_t>(), A->k1len.as<uint32_t>(),
+                                                kstart.as<uint32_t>());
         GS_CHECK_LAUNCH();
         GS_TRY(P.alloc(((size_t)chunkNum + 1) * 8));
         CountSpec cs{CountKind::ArrayTimes};
@@ -332,27 +297,31 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         GS_CHECK_LAUNCH();
         const bool u16 = p.itype == GS_IDX_U16;
         const size_t vsz = dtype_size(p.vtype), isz = u16 ? 2 : 4;
-        GS_TRY(A->val.alloc_zero((size_t)A->lenVC * vsz, s));
-        GS_TRY(A->col.alloc_zero((size_t)A->lenVC * isz, s));
+        GS_TRY(A->val.alloc((size_t)A->lenVC * vsz, s));
+        // the steps of padding slots stay 0
+        if (u16) GS_TRY(A->col.alloc_zero((size_t)A->lenVC * isz, s));
+        else GS_TRY(A->col.alloc((size_t)A->lenVC * isz, s));
         StreamBuf col32(s);  // 32-bit columns before the 16-bit steps are taken
-        if (u16) GS_TRY(col32.alloc_zero((size_t)A->lenVC * 4));
-        uint32_t *ocol = u16 ? col32.as<uint32_t>() : A->col.as<uint32_t>();
+        if (u16) GS_TRY(col32.alloc((size_t)A->lenVC * 4));
         GS_TRY(build_k1_plan(A->nmc.as<uint32_t>(), chunkNum, A->k1unit_chunk, A->k1unit_base,
                              A->k1partial, A->k1count, &A->k1units, s));
         // 16-bit steps: lane-blocked slot order (k1_slot); otherwise the reference's
-        if (val_type == GS_F64)
-            launch_fill_k1<double>(n, A->k1units, A->k1unit_chunk.as<uint32_t>(),
-                                   A->k1unit_base.as<uint32_t>(), d_row, d_col,
-                                   static_cast<const double *>(d_val), A->permi.as<uint32_t>(),
-                                   A->chp.as<uint32_t>(), A->nmc.as<uint32_t>(), u16, p.vtype,
-                                   A->val.p, ocol, s);
-        else
-            launch_fill_k1<float>(n, A->k1units, A->k1unit_chunk.as<uint32_t>(),
-                                  A->k1unit_base.as<uint32_t>(), d_row, d_col,
-                                  static_cast<const float *>(d_val), A->permi.as<uint32_t>(),
-                                  A->chp.as<uint32_t>(), A->nmc.as<uint32_t>(), u16, p.vtype,
-                                  A->val.p, ocol, s);
-        GS_CHECK_LAUNCH();
+        k1fill::Args fa{};
+        fa.n = n;
+        fa.units = A->k1units;
+        fa.unit_chunk = A->k1unit_chunk.as<uint32_t>();
+        fa.unit_base = A->k1unit_base.as<uint32_t>();
+        fa.nmc = A->nmc.as<uint32_t>();
+        fa.chp = A->chp.as<uint32_t>();
+        fa.start = kstart.as<uint32_t>();
+        fa.len = A->k1len.as<uint32_t>();
+        fa.val = d_val;
+        fa.col = d_col;
+        fa.oval = A->val.p;
+        fa.ocol = u16 ? col32.as<uint32_t>() : A->col.as<uint32_t>();
+        fa.blocked = u16;
+        if (val_type == GS_F64) GS_TRY(launch_fill_k1<double>(fa, p.vtype, s));
+        else GS_TRY(launch_fill_k1<float>(fa, p.vtype, s));
         if (u16) {
             K1Args a{};
             a.nrows = n;

@@ -132,6 +132,8 @@ gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_
 // i-th row.  Ties keep ascending row order.  LSD radix passes of up to 8 bits.
 gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
                            uint32_t *idx_out, cudaStream_t s);
+gs_status stable_sort_asc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
+                          cudaStream_t s);
 
 // Maximum of n u32 values (host result, synchronises).
 gs_status reduce_max_u32(const uint32_t *d, size_t n, uint32_t *out, cudaStream_t s);
@@ -216,7 +218,7 @@ struct gs_matrix {
     gs::DevBuf mmpartial;  // split pieces x 32 lanes x up to 32 RHS (FP64 sized)
     uint32_t k1split_units = 0;
     bool mm_ready = false, adj_ready = false;
-    gs::DevBuf fsrc;    // forward slot -> CSR index
+    gs::DevBuf kstart;  // first CSR element of each sorted row
     gs::DevBuf ftslot;  // forward slot -> adjoint-layout slot
     gs::DevBuf vrow, vcol;  // CSR index -> row, column
     gs::DevBuf t2f;     // adjoint-layout slot -> forward slot (padding: none)

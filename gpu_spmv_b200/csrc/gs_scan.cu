@@ -371,17 +371,17 @@ constexpr int kRadixItems = 16;
 constexpr uint32_t kRadixTile = kRadixThreads * kRadixItems;
 constexpr int kRadixDigits = 256;
 
-// ascending in max_key - key == descending in key
+// The first pass of a descending sort turns the keys round: ascending in flip - key
 template <bool FIRST>
-__device__ __forceinline__ uint32_t radix_key(uint32_t k, uint32_t max_key)
+__device__ __forceinline__ uint32_t radix_key(uint32_t k, uint32_t flip)
 {
-    return FIRST ? max_key - k : k;
+    return FIRST && flip ? flip - k : k;
 }
 
 // count[d * tiles + t] = elements of tile t with digit d
 template <bool FIRST>
 __global__ void __launch_bounds__(kRadixThreads) k_radix_count(
-    const uint32_t *__restrict__ kin, uint32_t n, uint32_t max_key, uint32_t shift,
+    const uint32_t *__restrict__ kin, uint32_t n, uint32_t flip, uint32_t shift,
     uint32_t mask, uint32_t tiles, uint32_t *__restrict__ count)
 {
     __shared__ uint32_t h[kRadixDigits];
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_count(
     for (int i = 0; i < kRadixItems; i++) {
         const uint32_t o = (uint32_t)i * kRadixThreads + threadIdx.x;
         if (o < n - t0)
-            atomicAdd(&h[(radix_key<FIRST>(kin[t0 + o], max_key) >> shift) & mask], 1u);
+            atomicAdd(&h[(radix_key<FIRST>(kin[t0 + o], flip) >> shift) & mask], 1u);
     }
     __syncthreads();
     if (threadIdx.x <= mask) count[(size_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scan(uint32_t *__restri
 template <bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ iin, uint32_t n,
-    uint32_t max_key, uint32_t shift, uint32_t mask, uint32_t tiles,
+    uint32_t flip, uint32_t shift, uint32_t mask, uint32_t tiles,
     const uint32_t *__restrict__ before, const uint32_t *__restrict__ total,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ iout)
 {
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
 #pragma unroll
     for (int i = 0; i < kRadixItems; i++) {
         const uint32_t o = o0 + 32u * i;
-        key[i] = o < cnt ? radix_key<FIRST>(kin[t0 + o], max_key) : 0u;
+        key[i] = o < cnt ? radix_key<FIRST>(kin[t0 + o], flip) : 0u;
         idx[i] = FIRST ? t0 + o : (o < cnt ? iin[t0 + o] : 0u);
     }
 #pragma unroll
@@ -521,8 +521,8 @@ __global__ void k_iota(uint32_t n, uint32_t *idx)
     if (i < n) idx[i] = i;
 }
 
-gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
-                           uint32_t *idx_out, cudaStream_t s)
+static gs_status stable_sort(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t flip,
+                             uint32_t *idx_out, cudaStream_t s)
 {
     if (n == 0) return GS_OK;
     int bits = 0;
@@ -552,18 +552,30 @@ gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
         uint32_t *kout = kbuf[p & 1];
         // the last pass writes idx_out
         uint32_t *iout = ((passes - 1 - p) & 1) ? ib.as<uint32_t>() : idx_out;
-        if (first) k_radix_count<true><<<tiles, kRadixThreads, 0, s>>>(kin, n, max_key, shift, mask, tiles, c);
-        else k_radix_count<false><<<tiles, kRadixThreads, 0, s>>>(kin, n, max_key, shift, mask, tiles, c);
+        if (first) k_radix_count<true><<<tiles, kRadixThreads, 0, s>>>(kin, n, flip, shift, mask, tiles, c);
+        else k_radix_count<false><<<tiles, kRadixThreads, 0, s>>>(kin, n, flip, shift, mask, tiles, c);
         k_radix_scan<<<digits, kRadixThreads, 0, s>>>(c, tiles, tot);
         auto scatter = first ? (last ? k_radix_scatter<true, true> : k_radix_scatter<true, false>)
                              : (last ? k_radix_scatter<false, true> : k_radix_scatter<false, false>);
-        scatter<<<tiles, kRadixThreads, 0, s>>>(kin, iin, n, max_key, shift, mask, tiles, c, tot,
+        scatter<<<tiles, kRadixThreads, 0, s>>>(kin, iin, n, flip, shift, mask, tiles, c, tot,
                                                 kout, iout);
         GS_CHECK_LAUNCH();
         kin = kout;
         iin = iout;
     }
     return GS_OK;
+}
+
+gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
+                           cudaStream_t s)
+{
+    return stable_sort(key, n, max_key, max_key, idx_out, s);
+}
+
+gs_status stable_sort_asc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
+                          cudaStream_t s)
+{
+    return stable_sort(key, n, max_key, 0, idx_out, s);
 }
 
 // ------------------------------------------------------------------ max reduce

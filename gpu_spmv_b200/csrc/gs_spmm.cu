@@ -21,6 +21,7 @@
 // The reference has no multi-RHS product and no adjoint; these extend its K1 format.
 #include <mutex>
 
+#include "gs_k1_fill.cuh"
 #include "gs_mm.cuh"
 
 namespace gs {
@@ -241,17 +242,6 @@ template <class T> gs_status launch_vbar(const VbarArgs &a, uint32_t k, cudaStre
 }
 
 // ------------------------------------------------------------------ layout helpers
-// fsrc[slot] = CSR index of the element in K1 slot `slot` (kNoSrc for padding)
-__global__ void k_k1_fsrc(uint32_t n, const uint32_t *row, const uint32_t *permi,
-                          const uint32_t *chp, uint32_t *fsrc)
-{
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    const uint32_t r = permi[g], b = row[r], len = row[r + 1] - b;
-    const uint32_t base = chp[g / 32] + (g % 32);
-    for (uint32_t e = 0; e < len; e++) fsrc[base + 32u * e] = b + e;
-}
-
 template <class T>
 __global__ void k_gather_vals(size_t nslots, const uint32_t *src, const T *v, T *out)
 {
@@ -272,24 +262,46 @@ __global__ void k_scatter_vals(size_t nslots, const uint32_t *src, const T *v, T
     }
 }
 
-// inv[map[i]] = i for the real entries of map
-__global__ void k_invert_map(size_t n, const uint32_t *map, uint32_t *inv)
+// Sorted row g: its first CSR element; and the way back from the row
+__global__ void k_row_places(uint32_t n, const uint32_t *row, const uint32_t *perm,
+                             uint32_t *start, uint32_t *inv)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t m = map[i];
-        if (m != kNoSrc) inv[m] = (uint32_t)i;
-    }
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    start[g] = row[perm[g]];
+    inv[perm[g]] = g;
 }
 
-// out[i] = b[a[i]] (kNoSrc stays kNoSrc)
-__global__ void k_compose_map(size_t n, const uint32_t *a, const uint32_t *b, uint32_t *out)
+// csr2f[e] = forward slot of CSR element e (its row at sorted place inv[row])
+__global__ void k_forward_slots(uint32_t nnz, const uint32_t *__restrict__ vrow,
+                                const uint32_t *__restrict__ rowptr,
+                                const uint32_t *__restrict__ inv,
+                                const uint32_t *__restrict__ chp, uint32_t *__restrict__ csr2f)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t m = a[i];
-        out[i] = m == kNoSrc ? kNoSrc : b[m];
-    }
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nnz) return;
+    const uint32_t r = vrow[e], g = __ldg(inv + r);
+    csr2f[e] = __ldg(chp + (g >> 5)) + 32u * (e - __ldg(rowptr + r)) + (g & 31u);
+}
+
+// The adjoint layout's slots, from the CSR index tsrc of each: the row and the stored value of the
+// element, its forward slot and the way back from there; padding slots 0, 0, none
+template <class T>
+__global__ void k_t_maps(uint32_t nslots, const uint32_t *__restrict__ tsrc,
+                         const uint32_t *__restrict__ vrow, const uint32_t *__restrict__ csr2f,
+                         const T *__restrict__ val, uint32_t *__restrict__ trow,
+                         T *__restrict__ tval, uint32_t *__restrict__ t2f,
+                         uint32_t *__restrict__ ftslot)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nslots) return;
+    const uint32_t e = tsrc[i];
+    const bool in = e != kNoSrc;
+    const uint32_t f = in ? __ldg(csr2f + e) : kNoSrc;
+    trow[i] = in ? __ldg(vrow + e) : 0u;
+    t2f[i] = f;
+    tval[i] = in ? __ldg(val + f) : T(0);
+    if (in) ftslot[f] = i;
 }
 
 // rowidx[e] = row of CSR element e: a warp per 32 rows, in element order (coalesced writes; the
@@ -315,22 +327,20 @@ __global__ void k_expand_rows(uint32_t n, const uint32_t *__restrict__ row,
     }
 }
 
-__global__ void k_col_keys(uint32_t nnz, uint32_t ncols, const uint32_t *col, uint32_t *key,
-                           uint32_t *count)
+__global__ void k_col_count(uint32_t nnz, const uint32_t *col, uint32_t *count)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    key[e] = ncols - 1u - col[e];  // descending key = ascending column
-    atomicAdd(count + col[e], 1u);
+    if (e < nnz) atomicAdd(count + col[e], 1u);
 }
 
-__global__ void k_t_meta(uint32_t m, const uint32_t *tl, const uint32_t *tperm, uint32_t *nmc,
-                         uint32_t *klen)
+__global__ void k_t_meta(uint32_t m, const uint64_t *cptr, const uint32_t *tperm, uint32_t *nmc,
+                         uint32_t *tlen, uint32_t *tstart)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= m) return;
-    const uint32_t l = tl[tperm[g]];
-    klen[g] = l;
+    const uint32_t j = tperm[g], b = (uint32_t)cptr[j], l = (uint32_t)cptr[j + 1] - b;
+    tlen[g] = l;
+    tstart[g] = b;
     if ((g & 31) == 0) nmc[g >> 5] = l;
 }
 
@@ -338,23 +348,6 @@ __global__ void k_narrow(uint32_t n, const uint64_t *a, uint32_t *b)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) b[i] = (uint32_t)a[i];
-}
-
-// transposed slot (chunk of sorted column g, step e) <- e-th element of column tperm[g]
-__global__ void k_t_fill(uint32_t m, const uint32_t *tperm, const uint64_t *cptr,
-                         const uint32_t *csc, const uint32_t *rowidx, const uint32_t *chp,
-                         uint32_t *trow, uint32_t *tsrc)
-{
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= m) return;
-    const uint32_t j = tperm[g];
-    const uint64_t b = cptr[j], len = cptr[j + 1] - b;
-    const uint32_t base = chp[g / 32] + (g % 32);
-    for (uint32_t e = 0; e < len; e++) {
-        const uint32_t k = csc[b + e];
-        tsrc[base + 32u * e] = k;
-        trow[base + 32u * e] = rowidx[k];
-    }
 }
 
 // largest u + 1 over units of split chunks (the prefix the partial sums need)
@@ -447,17 +440,38 @@ gs_status ensure_mm_scratch(gs_matrix *A, cudaStream_t s)
     return GS_OK;
 }
 
+// CSR order -> forward slots
+k1fill::Args forward_fill(const gs_matrix *A)
+{
+    k1fill::Args f{};
+    f.n = A->nrows;
+    f.units = A->k1units;
+    f.unit_chunk = A->k1unit_chunk.as<uint32_t>();
+    f.unit_base = A->k1unit_base.as<uint32_t>();
+    f.nmc = A->nmc.as<uint32_t>();
+    f.chp = A->chp.as<uint32_t>();
+    f.start = A->kstart.as<uint32_t>();
+    f.len = A->k1len.as<uint32_t>();
+    return f;
+}
+
 template <class T>
-void refresh_values(gs_matrix *A, const T *v, gs_value_order order, cudaStream_t s)
+gs_status refresh_values(gs_matrix *A, const T *v, gs_value_order order, cudaStream_t s)
 {
     const unsigned gb = 148u * 16u;
     if (order == GS_VALUES_CSR) {
-        k_gather_vals<T><<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), v, A->val.as<T>());
+        k1fill::Args f = forward_fill(A);
+        f.val = v;
+        f.oval = A->val.p;
+        GS_TRY((k1fill::fill<T, T, false>(f, T(0), s)));
         k_gather_vals<T><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), v, A->tval.as<T>());
     } else {
         k_gather_vals<T><<<gb, 256, 0, s>>>(A->lenVC, A->ftslot.as<uint32_t>(), v, A->val.as<T>());
-        cudaMemcpyAsync(A->tval.p, v, (size_t)A->tlenVC * sizeof(T), cudaMemcpyDeviceToDevice, s);
+        GS_CUDA(cudaMemcpyAsync(A->tval.p, v, (size_t)A->tlenVC * sizeof(T),
+                                cudaMemcpyDeviceToDevice, s));
     }
+    GS_CHECK_LAUNCH();
+    return GS_OK;
 }
 
 }  // namespace
@@ -512,33 +526,30 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(ensure_mm_scratch(A, s));
     if (A->adj_ready) return GS_OK;
     const uint32_t n = A->nrows, m = A->ncols, nnz = A->nnz;
-    // forward slot -> CSR index
-    GS_TRY(A->fsrc.alloc((size_t)A->lenVC * 4, s));
-    GS_CUDA(cudaMemsetAsync(A->fsrc.p, 0xff, (size_t)A->lenVC * 4, s));
-    if (n) {
-        k_k1_fsrc<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->permi.as<uint32_t>(),
-                                                A->chp.as<uint32_t>(), A->fsrc.as<uint32_t>());
-        GS_CHECK_LAUNCH();
-    }
-    // CSC order of the elements: stable sort of CSR indices by ascending column
-    StreamBuf key(s), ccount(s), csc(s), cptr(s);
+    GS_TRY(A->kstart.alloc((size_t)n * 4, s));
     // row and column of each element, for value gradients in CSR order
     GS_TRY(A->vrow.alloc((size_t)nnz * 4, s));
     GS_TRY(A->vcol.alloc((size_t)nnz * 4, s));
-    if (nnz)
-        GS_CUDA(cudaMemcpyAsync(A->vcol.p, d_col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
-    GS_TRY(key.alloc((size_t)nnz * 4));
+    // CSC order of the elements: stable sort of CSR indices by ascending column
+    StreamBuf ccount(s), csc(s), cptr(s), csr2f(s), inv(s);
     GS_TRY(ccount.alloc_zero((size_t)m * 4));
     GS_TRY(csc.alloc((size_t)nnz * 4));
+    GS_TRY(csr2f.alloc((size_t)nnz * 4));
+    GS_TRY(inv.alloc((size_t)n * 4));
     if (n) {
         k_expand_rows<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->vrow.as<uint32_t>());
+        k_row_places<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->permi.as<uint32_t>(),
+                                                  A->kstart.as<uint32_t>(), inv.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     if (nnz) {
-        k_col_keys<<<blocks_of(nnz), 256, 0, s>>>(nnz, m, d_col, key.as<uint32_t>(),
-                                                  ccount.as<uint32_t>());
+        GS_CUDA(cudaMemcpyAsync(A->vcol.p, d_col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
+        k_forward_slots<<<blocks_of(nnz), 256, 0, s>>>(
+            nnz, A->vrow.as<uint32_t>(), d_row, inv.as<uint32_t>(),
+            A->chp.as<uint32_t>(), csr2f.as<uint32_t>());
+        k_col_count<<<blocks_of(nnz), 256, 0, s>>>(nnz, d_col, ccount.as<uint32_t>());
         GS_CHECK_LAUNCH();
-        GS_TRY(stable_sort_desc(key.as<uint32_t>(), nnz, m ? m - 1 : 0, csc.as<uint32_t>(), s));
+        GS_TRY(stable_sort_asc(d_col, nnz, m ? m - 1 : 0, csc.as<uint32_t>(), s));
     }
     GS_TRY(cptr.alloc(((size_t)m + 1) * 8));
     {
@@ -555,9 +566,12 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(stable_sort_desc(ccount.as<uint32_t>(), m, maxlen, A->tpermi.as<uint32_t>(), s));
     GS_TRY(A->tnmc.alloc_zero((size_t)tchunks * 4 + 4, s));
     GS_TRY(A->tlen.alloc((size_t)m * 4 + 4, s));
+    StreamBuf tstart(s);
+    GS_TRY(tstart.alloc((size_t)m * 4));
     if (m) {
-        k_t_meta<<<blocks_of(m), 256, 0, s>>>(m, ccount.as<uint32_t>(), A->tpermi.as<uint32_t>(),
-                                              A->tnmc.as<uint32_t>(), A->tlen.as<uint32_t>());
+        k_t_meta<<<blocks_of(m), 256, 0, s>>>(m, cptr.as<uint64_t>(), A->tpermi.as<uint32_t>(),
+                                              A->tnmc.as<uint32_t>(), A->tlen.as<uint32_t>(),
+                                              tstart.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     StreamBuf P(s);
@@ -577,52 +591,43 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
         GS_CHECK_LAUNCH();
     }
     const size_t vsz = A->p.vtype == GS_F64 ? 8 : 4;
-    GS_TRY(A->trow.alloc_zero((size_t)A->tlenVC * 4, s));
-    GS_TRY(A->tsrc.alloc((size_t)A->tlenVC * 4, s));
-    GS_CUDA(cudaMemsetAsync(A->tsrc.p, 0xff, (size_t)A->tlenVC * 4, s));
-    GS_TRY(A->tval.alloc_zero((size_t)A->tlenVC * vsz, s));
-    if (m) {
-        k_t_fill<<<blocks_of(m), 256, 0, s>>>(m, A->tpermi.as<uint32_t>(), cptr.as<uint64_t>(),
-                                              csc.as<uint32_t>(), A->vrow.as<uint32_t>(),
-                                              A->tchp.as<uint32_t>(), A->trow.as<uint32_t>(),
-                                              A->tsrc.as<uint32_t>());
-        GS_CHECK_LAUNCH();
-    }
     GS_TRY(build_k1_plan(A->tnmc.as<uint32_t>(), tchunks, A->tunit_chunk, A->tunit_base,
                          A->tpartial1, A->tcount, &A->tunits, s));
     GS_TRY(split_extent(A->tunits, A->tunit_chunk.as<uint32_t>(), A->tunit_base.as<uint32_t>(),
                         &A->tsplit_units, s));
     GS_TRY(A->tpartial.alloc((size_t)A->tsplit_units * 32 * 32 * 8 + 8, s));
-    // transposed values from the stored ones: forward slots -> CSR order (each CSR index
-    // sits in exactly one forward slot) -> transposed slots
-    StreamBuf vcsr(s);
-    GS_TRY(vcsr.alloc((size_t)nnz * vsz + 8));
-    const unsigned gb = 148u * 16u;
-    if (A->p.vtype == GS_F64) {
-        k_scatter_vals<double><<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(),
-                                                  A->val.as<double>(), vcsr.as<double>());
-        k_gather_vals<double><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                 vcsr.as<double>(), A->tval.as<double>());
-    } else {
-        k_scatter_vals<float><<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(),
-                                                 A->val.as<float>(), vcsr.as<float>());
-        k_gather_vals<float><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                vcsr.as<float>(), A->tval.as<float>());
-    }
-    GS_CHECK_LAUNCH();
-    // forward slot <-> adjoint-layout slot, through the CSR index
-    StreamBuf csr2t(s), csr2f(s);
-    GS_TRY(csr2t.alloc((size_t)nnz * 4 + 4));
-    GS_TRY(csr2f.alloc((size_t)nnz * 4 + 4));
-    GS_TRY(A->ftslot.alloc((size_t)A->lenVC * 4 + 4, s));
-    k_invert_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), csr2t.as<uint32_t>());
-    k_invert_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), csr2f.as<uint32_t>());
-    k_compose_map<<<gb, 256, 0, s>>>(A->lenVC, A->fsrc.as<uint32_t>(), csr2t.as<uint32_t>(),
-                                     A->ftslot.as<uint32_t>());
+    GS_TRY(A->trow.alloc((size_t)A->tlenVC * 4, s));
+    GS_TRY(A->tsrc.alloc((size_t)A->tlenVC * 4, s));
+    GS_TRY(A->tval.alloc((size_t)A->tlenVC * vsz, s));
     GS_TRY(A->t2f.alloc((size_t)A->tlenVC * 4 + 4, s));
-    k_compose_map<<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), csr2f.as<uint32_t>(),
-                                     A->t2f.as<uint32_t>());
-    GS_CHECK_LAUNCH();
+    GS_TRY(A->ftslot.alloc((size_t)A->lenVC * 4 + 4, s));  // forward slot -> adjoint-layout slot
+    // adjoint-layout slot -> CSR index
+    k1fill::Args tf{};
+    tf.n = m;
+    tf.units = A->tunits;
+    tf.unit_chunk = A->tunit_chunk.as<uint32_t>();
+    tf.unit_base = A->tunit_base.as<uint32_t>();
+    tf.nmc = A->tnmc.as<uint32_t>();
+    tf.chp = A->tchp.as<uint32_t>();
+    tf.start = tstart.as<uint32_t>();
+    tf.len = A->tlen.as<uint32_t>();
+    tf.val = csc.p;
+    tf.oval = A->tsrc.p;
+    GS_TRY((k1fill::fill<uint32_t, uint32_t, false>(tf, kNoSrc, s)));
+    GS_CUDA(cudaMemsetAsync(A->ftslot.p, 0xff, (size_t)A->lenVC * 4, s));  // kNoSrc
+    if (A->tlenVC) {
+        if (A->p.vtype == GS_F64)
+            k_t_maps<double><<<blocks_of(A->tlenVC), 256, 0, s>>>(
+                A->tlenVC, A->tsrc.as<uint32_t>(), A->vrow.as<uint32_t>(), csr2f.as<uint32_t>(),
+                A->val.as<double>(), A->trow.as<uint32_t>(), A->tval.as<double>(),
+                A->t2f.as<uint32_t>(), A->ftslot.as<uint32_t>());
+        else
+            k_t_maps<float><<<blocks_of(A->tlenVC), 256, 0, s>>>(
+                A->tlenVC, A->tsrc.as<uint32_t>(), A->vrow.as<uint32_t>(), csr2f.as<uint32_t>(),
+                A->val.as<float>(), A->trow.as<uint32_t>(), A->tval.as<float>(),
+                A->t2f.as<uint32_t>(), A->ftslot.as<uint32_t>());
+        GS_CHECK_LAUNCH();
+    }
     GS_TRY(A->vslots.alloc((size_t)max(A->lenVC, A->tlenVC) * vsz + 8, s));
     A->adj_ready = true;
     GS_CUDA(cudaStreamSynchronize(s));
@@ -640,10 +645,8 @@ gs_status gs_matrix_set_values(gs_matrix *A, const void *d_val, gs_dtype dtype,
     if (order != GS_VALUES_CSR && order != GS_VALUES_SLOTS)
         return fail(GS_ERR_INVALID, "unknown value order %d", (int)order);
     cudaStream_t s = cs(stream);
-    if (dtype == GS_F64) refresh_values(A, static_cast<const double *>(d_val), order, s);
-    else refresh_values(A, static_cast<const float *>(d_val), order, s);
-    GS_CHECK_LAUNCH();
-    return GS_OK;
+    if (dtype == GS_F64) return refresh_values(A, static_cast<const double *>(d_val), order, s);
+    return refresh_values(A, static_cast<const float *>(d_val), order, s);
 }
 
 gs_status gs_matrix_value_slots(const gs_matrix *A, UIN *nslots)
