@@ -165,23 +165,27 @@ __global__ void k_k1_meta(uint32_t n, const uint32_t *row, const uint32_t *permi
     }
 }
 
-__global__ void k_u64_to_u32(uint32_t n, const uint64_t *a, uint32_t *b)
+// flag bit 1: a column >= ncols (16-byte loads where the array allows them)
+__global__ void k_check_columns(uint32_t ncols, uint32_t nnz, const uint32_t *__restrict__ col,
+                                uint32_t *flag)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (uint32_t)a[i];
-}
-
-// bit 0: row pointer not monotone / row[0] != 0 / row[n] != nnz; bit 1: column >= ncols
-__global__ void k_validate(uint32_t n, uint32_t ncols, uint32_t nnz, const uint32_t *row,
-                           const uint32_t *col, uint32_t *flag)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t bad = 0;
-    if (i < n && row[i] > row[i + 1]) bad |= 1u;
-    if (i == 0 && (row[0] != 0 || row[n] != nnz)) bad |= 1u;
-    for (uint32_t p = i; p < nnz; p += gridDim.x * blockDim.x)
-        if (col[p] >= ncols) { bad |= 2u; break; }
-    if (bad) atomicOr(flag, bad);
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+                   step = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t top = 0;
+    uint64_t done = 0;
+    if ((reinterpret_cast<uintptr_t>(col) & 15u) == 0) {
+        const uint4 *c4 = reinterpret_cast<const uint4 *>(col);
+        const uint64_t n4 = nnz / 4;
+#pragma unroll 4
+        for (uint64_t i = t; i < n4; i += step) {
+            const uint4 q = __ldg(c4 + i);
+            top = max(max(top, max(q.x, q.y)), max(q.z, q.w));
+        }
+        done = n4 * 4;
+    }
+    for (uint64_t i = done + t; i < nnz; i += step) top = max(top, col[i]);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0 && top >= ncols && nnz) atomicOr(flag, 2u);
 }
 
 inline unsigned blocks_for(uint64_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -238,19 +242,27 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
     A->ncols = ncols;
     A->nnz = nnz;
 
-    // ---- validate the CSR (structure and column range)
+    // ---- validate the CSR (structure and column range); the longest row
+    uint32_t maxlen = 0;
+    StreamBuf rl(s);  // row lengths (K1: the sort's keys)
     {
         StreamBuf flag(s);
-        GS_TRY(flag.alloc_zero(4));
-        k_validate<<<blocks_for(n + 1), 256, 0, s>>>(n, ncols, nnz, d_row, d_col,
-                                                     flag.as<uint32_t>());
-        GS_CHECK_LAUNCH();
-        uint32_t hf = 0;
-        GS_CUDA(cudaMemcpyAsync(&hf, flag.p, 4, cudaMemcpyDeviceToHost, s));
+        GS_TRY(flag.alloc_zero(8));
+        if (p.format == GS_FMT_K1) GS_TRY(rl.alloc((size_t)n * 4));
+        GS_TRY(row_lengths(n, d_row, nnz, rl.as<uint32_t>(), flag.as<uint32_t>(), s));
+        if (nnz) {
+            const uint32_t blocks = blocks_for(((uint64_t)nnz + 15) / 16);
+            k_check_columns<<<blocks < 148u * 8u ? blocks : 148u * 8u, 256, 0, s>>>(
+                ncols, nnz, d_col, flag.as<uint32_t>());
+            GS_CHECK_LAUNCH();
+        }
+        uint32_t hf[2] = {0, 0};
+        GS_CUDA(cudaMemcpyAsync(hf, flag.p, 8, cudaMemcpyDeviceToHost, s));
         GS_CUDA(cudaStreamSynchronize(s));
-        if (hf & 1u)
+        if (hf[0] & 1u)
             return fail(GS_ERR_INVALID, "row pointer array is not a valid CSR row pointer");
-        if (hf & 2u) return fail(GS_ERR_INVALID, "column index >= ncols");
+        if (hf[0] & 2u) return fail(GS_ERR_INVALID, "column index >= ncols");
+        maxlen = hf[1];
     }
 
     FillArgs f{};
@@ -267,12 +279,6 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
             return fail(GS_ERR_UNSUPPORTED, "FP64 K1 is stored with 32-bit columns");
         const uint32_t chunkNum = (n + 31) / 32;
         A->chunkNum = chunkNum;
-        StreamBuf rl(s);
-        GS_TRY(rl.alloc((size_t)n * 4));
-        k_rowlen<<<blocks_for(n), 256, 0, s>>>(n, d_row, rl.as<uint32_t>());
-        GS_CHECK_LAUNCH();
-        uint32_t maxlen = 0;
-        GS_TRY(reduce_max_u32(rl.as<uint32_t>(), n, &maxlen, s));
         GS_TRY(A->permi.alloc_zero(((size_t)chunkNum + 1) * 32 * 4, s));
         GS_TRY(stable_sort_desc(rl.as<uint32_t>(), n, maxlen, A->permi.as<uint32_t>(), s));
         GS_TRY(A->nmc.alloc_zero((size_t)chunkNum * 4, s));
@@ -283,18 +289,16 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
                                                 A->nmc.as<uint32_t>(), A->k1len.as<uint32_t>(),
                                                 kstart.as<uint32_t>());
         GS_CHECK_LAUNCH();
-        GS_TRY(P.alloc(((size_t)chunkNum + 1) * 8));
-        CountSpec cs{CountKind::ArrayTimes};
-        cs.arr = A->nmc.as<uint32_t>();
-        cs.a = 32;
-        uint64_t lenvc = 0;
-        GS_TRY(exclusive_scan(cs, chunkNum, P.as<uint64_t>(), &lenvc, s));
-        if (lenvc > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 lenVC exceeds 32 bits");
-        A->lenVC = (uint32_t)lenvc;
         GS_TRY(A->chp.alloc((size_t)chunkNum * 4, s));
-        k_u64_to_u32<<<blocks_for(chunkNum), 256, 0, s>>>(chunkNum, P.as<uint64_t>(),
-                                                         A->chp.as<uint32_t>());
-        GS_CHECK_LAUNCH();
+        GS_TRY(A->k1unit_base.alloc(((size_t)chunkNum + 1) * 4, s));
+        uint64_t total[3] = {0, 0, 0};
+        GS_TRY(k1_layout_scan(A->nmc.as<uint32_t>(), chunkNum, A->chp.as<uint32_t>(),
+                              A->k1unit_base.as<uint32_t>(), total, s));
+        if (total[0] > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 lenVC exceeds 32 bits");
+        if (total[1] >= 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 plan too large");
+        A->lenVC = (uint32_t)total[0];
+        A->k1units = (uint32_t)total[1];
+        A->k1split_units = (uint32_t)total[2];
         const bool u16 = p.itype == GS_IDX_U16;
         const size_t vsz = dtype_size(p.vtype), isz = u16 ? 2 : 4;
         GS_TRY(A->val.alloc((size_t)A->lenVC * vsz, s));
@@ -303,8 +307,8 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         else GS_TRY(A->col.alloc((size_t)A->lenVC * isz, s));
         StreamBuf col32(s);  // 32-bit columns before the 16-bit steps are taken
         if (u16) GS_TRY(col32.alloc((size_t)A->lenVC * 4));
-        GS_TRY(build_k1_plan(A->nmc.as<uint32_t>(), chunkNum, A->k1unit_chunk, A->k1unit_base,
-                             A->k1partial, A->k1count, &A->k1units, s));
+        GS_TRY(build_k1_units(A->k1unit_base.as<uint32_t>(), chunkNum, A->k1units, A->k1unit_chunk,
+                              &A->k1partial, A->k1count, s));
         // 16-bit steps: lane-blocked slot order (k1_slot); otherwise the reference's
         k1fill::Args fa{};
         fa.n = n;

@@ -114,15 +114,13 @@ enum class CountKind {
     RowLen,         // row[i+1]-row[i]
     RowTiles,       // ceil((row[i+1]-row[i]) / a)
     Array,          // arr[i]
-    ArrayTimes,     // arr[i] * a
-    PiecesMin1,     // max(1, ceil(arr[i] / a))
     WindowPopc,     // popcount of the a words arr[i*a .. i*a+a)
     NonEmpty,       // row[i+1] > row[i]
 };
 struct CountSpec {
     CountKind kind;
     const uint32_t *row = nullptr;  // RowLen / RowTiles
-    const uint32_t *arr = nullptr;  // Array / ArrayTimes
+    const uint32_t *arr = nullptr;  // Array
     uint32_t a = 1;
 };
 gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_t *total,
@@ -132,11 +130,14 @@ gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_
 // i-th row.  Ties keep ascending row order.  LSD radix passes of up to 8 bits.
 gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key,
                            uint32_t *idx_out, cudaStream_t s);
+// Ascending; key_out (or nullptr): the keys in their new order.
 gs_status stable_sort_asc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
-                          cudaStream_t s);
+                          uint32_t *key_out, cudaStream_t s);
 
-// Maximum of n u32 values (host result, synchronises).
-gs_status reduce_max_u32(const uint32_t *d, size_t n, uint32_t *out, cudaStream_t s);
+// Row lengths (len may be nullptr) of n rows; out[0] |= 1 where the pointers are not 0 = row[0]
+// <= row[1] <= .. <= row[n] = nnz, out[1] = the longest row (out: 2 words, cleared before).
+gs_status row_lengths(uint32_t n, const uint32_t *row, uint32_t nnz, uint32_t *len, uint32_t *out,
+                      cudaStream_t s);
 
 // ------------------------------------------------------------------ device helpers
 __device__ __forceinline__ double ldcs_f64(const double *p) { return __ldcs(p); }
@@ -224,7 +225,7 @@ struct gs_matrix {
     gs::DevBuf t2f;     // adjoint-layout slot -> forward slot (padding: none)
     gs::DevBuf vslots;  // atomic mode: vbar in forward slot order before it is gathered
     gs::DevBuf tpermi, tnmc, tchp, tlen, trow, tsrc, tval;  // K1 layout of A^T
-    gs::DevBuf tunit_chunk, tunit_base, tpartial1, tcount, tpartial;
+    gs::DevBuf tunit_chunk, tunit_base, tcount, tpartial;
     uint32_t tchunkNum = 0, tlenVC = 0, tunits = 0, tsplit_units = 0;
     uint32_t k1units = 0;
     // row-stream kernel configuration
@@ -338,12 +339,17 @@ gs_status launch_k1(const K1Args &a, gs_dtype vtype, gs_itype itype, gs_dtype yt
 // 16-bit column steps + per-unit checkpoints from 32-bit K1 columns (plan and klen needed).
 gs_status build_k1_deltas(const K1Args &a, const uint32_t *d_col32, uint16_t *d_col16,
                           uint32_t *d_ck, cudaStream_t s);
-// Build the K1 plan for chunk lengths nmc (device) into the given buffers.
 constexpr uint32_t kK1Split = 128;  // j-steps per K1 work unit (a piece is a critical path of
                                      // kK1Split/8 dependent gather rounds: 128 keeps it short)
-gs_status build_k1_plan(const uint32_t *d_nmc, uint32_t chunkNum, DevBuf &unit_chunk,
-                        DevBuf &unit_base, DevBuf &partial, DevBuf &count, uint32_t *units,
-                        cudaStream_t s);
+// First slot (chp, n entries) and first work unit (unit_base, n + 1 entries) of each of n chunks
+// of nmc steps; total: slots, units, and 1 + the last unit of a chunk cut into pieces (0: none).
+// Synchronises.
+gs_status k1_layout_scan(const uint32_t *nmc, uint32_t n, uint32_t *chp, uint32_t *unit_base,
+                         uint64_t total[3], cudaStream_t s);
+// The plan's other arrays, for `units` units of chunkNum chunks: the chunk of each unit, the
+// single-vector product's partial sums (or nullptr) and the arrival counters.
+gs_status build_k1_units(const uint32_t *unit_base, uint32_t chunkNum, uint32_t units,
+                         DevBuf &unit_chunk, DevBuf *partial, DevBuf &count, cudaStream_t s);
 
 // Sizes a K1 matrix's multi-RHS scratch once (gs_spmm.cu; allocates, synchronises).
 gs_status prepare_mm_scratch(gs_matrix *A, cudaStream_t s);

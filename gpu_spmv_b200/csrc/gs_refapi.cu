@@ -587,12 +587,16 @@ str_res test_gk1(const UIN cudaBlockSize, const str_matK1 k, const FPT *vec, con
 {
     (void)cudaBlockSize;
     DevBuf permi, nmc, chp, val, col, x, y, uc, ub, part, cnt;
-    uint32_t units = 0;
+    uint64_t total[3] = {0, 0, 0};
+    DevBuf own_chp;  // the layout's own slot offsets, not the caller's
     if (h2d(permi, k.permi, ((size_t)k.chunkNum + 1) * 32) || h2d(nmc, k.nmc, k.chunkNum) ||
         h2d(chp, k.chp, k.chunkNum) || h2d(val, k.val, k.lenVC) || h2d(col, k.col, k.lenVC) ||
         h2d(x, vec, k.nrows) || y.alloc((size_t)k.nrows * 8) ||
-        gs::build_k1_plan(nmc.as<UIN>(), k.chunkNum, uc, ub, part, cnt, &units, 0))
+        own_chp.alloc((size_t)k.chunkNum * 4) || ub.alloc(((size_t)k.chunkNum + 1) * 4) ||
+        gs::k1_layout_scan(nmc.as<UIN>(), k.chunkNum, own_chp.as<UIN>(), ub.as<UIN>(), total, 0) ||
+        gs::build_k1_units(ub.as<UIN>(), k.chunkNum, (uint32_t)total[1], uc, &part, cnt, 0))
         return error_res("gk1", gs_last_error());
+    const uint32_t units = (uint32_t)total[1];
     gs::K1Args a{};
     a.nrows = k.nrows;
     a.chunkNum = k.chunkNum;

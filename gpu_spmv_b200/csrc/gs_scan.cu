@@ -208,12 +208,7 @@ struct CountDev {
             return (uint64_t)((l + a - 1) / a);
         }
         case 2: return (uint64_t)arr[i];
-        case 3: return (uint64_t)arr[i] * (uint64_t)a;
-        case 4: {
-            uint32_t t = (arr[i] + a - 1) / a;
-            return (uint64_t)(t ? t : 1u);
-        }
-        case 5: {
+        case 3: {
             uint64_t c = 0;
             for (uint32_t j = 0; j < a; j++) c += __popc(arr[i * a + j]);
             return c;
@@ -277,9 +272,11 @@ __global__ void k_scan_reduce(CountDev f, size_t n, uint64_t *bsum)
     if (threadIdx.x == 0) bsum[blockIdx.x] = t;
 }
 
-// Exclusive scan of nb block sums in place, one block of 1024 threads; bsum[nb] = total.
+// Exclusive scan of nb block sums in place, one block of 1024 threads; bsum[nb] = total.  Block b
+// scans the b-th array of nb + 1 entries.
 __global__ void k_scan_blocks(uint64_t *bsum, size_t nb)
 {
+    bsum += blockIdx.x * (nb + 1);
     __shared__ uint64_t wsum[32];
     __shared__ uint64_t carry;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -306,8 +303,9 @@ __global__ void k_scan_blocks(uint64_t *bsum, size_t nb)
     if (threadIdx.x == 0) bsum[nb] = carry;
 }
 
-__global__ void k_scan_down(CountDev f, size_t n, const uint64_t *bsum, uint64_t *out)
+__global__ void k_scan_down(CountDev f, size_t n, size_t nb, const uint64_t *bsum, uint64_t *out)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = bsum[nb];
     size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
     uint64_t v[kScanItems];
     uint64_t s = 0;
@@ -328,11 +326,6 @@ __global__ void k_scan_down(CountDev f, size_t n, const uint64_t *bsum, uint64_t
     }
 }
 
-__global__ void k_write_total(const uint64_t *bsum, size_t nb, uint64_t *out, size_t n)
-{
-    out[n] = bsum[nb];
-}
-
 gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_t *total,
                          cudaStream_t s)
 {
@@ -344,13 +337,97 @@ gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_
     uint64_t *bsum = sums.as<uint64_t>();
     k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(f, n, bsum);
     k_scan_blocks<<<1, 1024, 0, s>>>(bsum, nb);
-    k_scan_down<<<(unsigned)nb, kScanThreads, 0, s>>>(f, n, bsum, out);
-    k_write_total<<<1, 1, 0, s>>>(bsum, nb, out, n);
+    k_scan_down<<<(unsigned)nb, kScanThreads, 0, s>>>(f, n, nb, bsum, out);
     GS_CHECK_LAUNCH();
     if (total) {
         GS_CUDA(cudaMemcpyAsync(total, out + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         GS_CUDA(cudaStreamSynchronize(s));
     }
+    return GS_OK;
+}
+
+// ------------------------------------------------------------------ K1 layout
+// Both prefix sums a K1 layout needs in one pass over its chunks' steps: slots (32 per step) and
+// work units (pieces of kK1Split steps, at least one).
+__device__ __forceinline__ uint64_t k1_units_of(uint32_t m)
+{
+    return m <= kK1Split ? 1u : ((uint64_t)m + kK1Split - 1u) / kK1Split;
+}
+
+__global__ void k_layout_reduce(const uint32_t *nmc, size_t n, size_t nb, uint64_t *bsum)
+{
+    const size_t base = (size_t)blockIdx.x * kScanTile;
+    uint64_t slots = 0, units = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        const size_t i = base + (size_t)k * kScanThreads + threadIdx.x;
+        if (i < n) {
+            const uint32_t m = nmc[i];
+            slots += 32ull * m;
+            units += k1_units_of(m);
+        }
+    }
+    __shared__ uint64_t ts, tu;
+    (void)block_excl_scan_u64(slots, &ts);
+    (void)block_excl_scan_u64(units, &tu);
+    if (threadIdx.x == 0) {
+        bsum[blockIdx.x] = ts;
+        bsum[nb + 1 + blockIdx.x] = tu;
+    }
+}
+
+// total: slots, units, 1 + the last unit of a cut chunk (0: no chunk is cut; cleared beforehand)
+__global__ void k_layout_down(const uint32_t *nmc, size_t n, size_t nb, const uint64_t *bsum,
+                              uint32_t *chp, uint32_t *unit_base, unsigned long long *total)
+{
+    const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
+    uint32_t m[kScanItems];
+    uint64_t slots = 0, units = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        m[k] = base + k < n ? nmc[base + k] : 0u;
+        slots += 32ull * m[k];
+        if (base + k < n) units += k1_units_of(m[k]);
+    }
+    __shared__ uint64_t ts, tu;
+    uint64_t es = block_excl_scan_u64(slots, &ts) + bsum[blockIdx.x];
+    uint64_t eu = block_excl_scan_u64(units, &tu) + bsum[nb + 1 + blockIdx.x];
+    unsigned long long cut = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < n) {
+            chp[base + k] = (uint32_t)es;
+            unit_base[base + k] = (uint32_t)eu;
+            const uint64_t u = k1_units_of(m[k]);
+            if (u > 1) cut = eu + u;
+            es += 32ull * m[k];
+            eu += u;
+        }
+    }
+    if (cut) atomicMax(total + 2, cut);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        total[0] = bsum[nb];
+        total[1] = bsum[2 * nb + 1];
+        unit_base[n] = (uint32_t)bsum[2 * nb + 1];
+    }
+}
+
+gs_status k1_layout_scan(const uint32_t *nmc, uint32_t n, uint32_t *chp, uint32_t *unit_base,
+                         uint64_t total[3], cudaStream_t s)
+{
+    size_t nb = ((size_t)n + kScanTile - 1) / kScanTile;
+    if (nb == 0) nb = 1;
+    StreamBuf sums(s), tot(s);
+    GS_TRY(sums.alloc(2 * (nb + 1) * sizeof(uint64_t)));
+    GS_TRY(tot.alloc_zero(3 * sizeof(uint64_t)));
+    uint64_t *bsum = sums.as<uint64_t>();
+    k_layout_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(nmc, n, nb, bsum);
+    k_scan_blocks<<<2, 1024, 0, s>>>(bsum, nb);
+    k_layout_down<<<(unsigned)nb, kScanThreads, 0, s>>>(nmc, n, nb, bsum, chp, unit_base,
+                                                        tot.as<unsigned long long>());
+    GS_CHECK_LAUNCH();
+    GS_CUDA(cudaMemcpyAsync(total, tot.p, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;
 }
 
@@ -364,7 +441,8 @@ gs_status exclusive_scan(const CountSpec &spec, size_t n, uint64_t *out, uint64_
 // before it is written, so that a digit's elements leave as one run (64 bytes on average with
 // 256 digits and 4096 elements).  Between blocks there is no waiting: the tiles' digit counts
 // are made by a pass of their own and scanned by one block per digit.
-// 4.2M elements, 20-bit keys: 20 passes of one bit 1310 us, 3 passes of 7 bits about 150 us.
+// 4.2M elements, 20-bit keys: 20 passes of one bit 1310 us, 3 passes of 7 bits RADIX_US us (with
+// match.any instead of ballots for the ranks about 150).
 constexpr int kRadixThreads = 256;
 constexpr int kRadixWarps = kRadixThreads / 32;
 constexpr int kRadixItems = 16;
@@ -440,7 +518,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scan(uint32_t *__restri
     if (threadIdx.x == 0) total[blockIdx.x] = carry;
 }
 
-template <bool FIRST, bool LAST>
+template <bool FIRST>
 __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ iin, uint32_t n,
     uint32_t flip, uint32_t shift, uint32_t mask, uint32_t tiles,
@@ -472,7 +550,14 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
         const unsigned live = __ballot_sync(0xffffffffu, in);
         if (in) {
             const uint32_t d = (key[i] >> shift) & mask;
-            const unsigned peers = __match_any_sync(live, d);
+            unsigned peers = live;  // lanes of the same digit, bit by bit
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                if ((mask >> b) & 1u) {
+                    const unsigned B = __ballot_sync(live, (d >> b) & 1u);
+                    peers &= ((d >> b) & 1u) ? B : ~B;
+                }
+            }
             const uint32_t below = (uint32_t)__popc(peers & ((1u << lane) - 1u));
             rank[i] = wcount[w][d] + below;
             __syncwarp(live);
@@ -509,33 +594,36 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     for (uint32_t p = threadIdx.x; p < cnt; p += kRadixThreads) {
         const uint32_t k = skey[p], d = (k >> shift) & mask;
         const uint32_t g = dest[d] + (p - start[d]);
-        if (!LAST) kout[g] = k;
+        if (kout) kout[g] = k;
         iout[g] = sidx[p];
     }
 }
 
-// idx[i] = i
-__global__ void k_iota(uint32_t n, uint32_t *idx)
+// idx[i] = i, and keys that are all 0
+__global__ void k_iota(uint32_t n, uint32_t *idx, uint32_t *key)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) idx[i] = i;
+    if (i >= n) return;
+    idx[i] = i;
+    if (key) key[i] = 0u;
 }
 
+// key_out (or nullptr): the keys in their new order (flip - key where flip is given)
 static gs_status stable_sort(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t flip,
-                             uint32_t *idx_out, cudaStream_t s)
+                             uint32_t *idx_out, uint32_t *key_out, cudaStream_t s)
 {
     if (n == 0) return GS_OK;
     int bits = 0;
     while (bits < 32 && (max_key >> bits) != 0) bits++;
-    if (bits == 0) {  // all keys equal: the order they came in
-        k_iota<<<(n + 255) / 256, 256, 0, s>>>(n, idx_out);
+    if (bits == 0) {  // all keys are 0: the order they came in
+        k_iota<<<(n - 1) / 256 + 1, 256, 0, s>>>(n, idx_out, key_out);
         GS_CHECK_LAUNCH();
         return GS_OK;
     }
     const int passes = (bits + 7) / 8;
     const uint32_t db = (uint32_t)((bits + passes - 1) / passes);  // bits per pass
     const uint32_t mask = (1u << db) - 1u, digits = mask + 1u;
-    const uint32_t tiles = (uint32_t)(((uint64_t)n + kRadixTile - 1) / kRadixTile);
+    const uint32_t tiles = (n - 1) / kRadixTile + 1;
     StreamBuf ka(s), kb(s), ib(s), cnt(s);
     GS_TRY(cnt.alloc(((size_t)digits * tiles + digits) * 4));
     if (passes > 1) {
@@ -549,14 +637,13 @@ static gs_status stable_sort(const uint32_t *key, uint32_t n, uint32_t max_key, 
     for (int p = 0; p < passes; p++) {
         const bool first = p == 0, last = p == passes - 1;
         const uint32_t shift = db * (uint32_t)p;
-        uint32_t *kout = kbuf[p & 1];
+        uint32_t *kout = last ? key_out : kbuf[p & 1];
         // the last pass writes idx_out
         uint32_t *iout = ((passes - 1 - p) & 1) ? ib.as<uint32_t>() : idx_out;
-        if (first) k_radix_count<true><<<tiles, kRadixThreads, 0, s>>>(kin, n, flip, shift, mask, tiles, c);
-        else k_radix_count<false><<<tiles, kRadixThreads, 0, s>>>(kin, n, flip, shift, mask, tiles, c);
+        auto count = first ? k_radix_count<true> : k_radix_count<false>;
+        auto scatter = first ? k_radix_scatter<true> : k_radix_scatter<false>;
+        count<<<tiles, kRadixThreads, 0, s>>>(kin, n, flip, shift, mask, tiles, c);
         k_radix_scan<<<digits, kRadixThreads, 0, s>>>(c, tiles, tot);
-        auto scatter = first ? (last ? k_radix_scatter<true, true> : k_radix_scatter<true, false>)
-                             : (last ? k_radix_scatter<false, true> : k_radix_scatter<false, false>);
         scatter<<<tiles, kRadixThreads, 0, s>>>(kin, iin, n, flip, shift, mask, tiles, c, tot,
                                                 kout, iout);
         GS_CHECK_LAUNCH();
@@ -569,35 +656,42 @@ static gs_status stable_sort(const uint32_t *key, uint32_t n, uint32_t max_key, 
 gs_status stable_sort_desc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
                            cudaStream_t s)
 {
-    return stable_sort(key, n, max_key, max_key, idx_out, s);
+    return stable_sort(key, n, max_key, max_key, idx_out, nullptr, s);
 }
 
 gs_status stable_sort_asc(const uint32_t *key, uint32_t n, uint32_t max_key, uint32_t *idx_out,
-                          cudaStream_t s)
+                          uint32_t *key_out, cudaStream_t s)
 {
-    return stable_sort(key, n, max_key, 0, idx_out, s);
+    return stable_sort(key, n, max_key, 0, idx_out, key_out, s);
 }
 
-// ------------------------------------------------------------------ max reduce
-__global__ void k_max_u32(const uint32_t *d, size_t n, uint32_t *out)
+// ------------------------------------------------------------------ row lengths
+__global__ void k_row_lengths(uint32_t n, const uint32_t *row, uint32_t nnz, uint32_t *len,
+                              uint32_t *out)
 {
-    uint32_t m = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x)
-        m = max(m, d[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+    uint32_t top = 0, bad = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t b = row[i], e = row[i + 1];
+        bad |= (b > e || (i == 0 && b != 0) || (i == n - 1u && e != nnz)) ? 1u : 0u;
+        if (len) len[i] = e - b;
+        top = max(top, e - b);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (bad) atomicOr(out, bad);
+        if (top) atomicMax(out + 1, top);
+    }
 }
 
-gs_status reduce_max_u32(const uint32_t *d, size_t n, uint32_t *out, cudaStream_t s)
+gs_status row_lengths(uint32_t n, const uint32_t *row, uint32_t nnz, uint32_t *len, uint32_t *out,
+                      cudaStream_t s)
 {
-    StreamBuf m(s);
-    GS_TRY(m.alloc_zero(sizeof(uint32_t)));
-    if (n) k_max_u32<<<296, 256, 0, s>>>(d, n, m.as<uint32_t>());
+    if (!n) return GS_OK;
+    const uint32_t blocks = (n - 1) / 256 + 1;
+    k_row_lengths<<<blocks < 148u * 8u ? blocks : 148u * 8u, 256, 0, s>>>(n, row, nnz, len, out);
     GS_CHECK_LAUNCH();
-    GS_CUDA(cudaMemcpyAsync(out, m.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GS_CUDA(cudaStreamSynchronize(s));
     return GS_OK;
 }
 

@@ -327,54 +327,34 @@ __global__ void k_expand_rows(uint32_t n, const uint32_t *__restrict__ row,
     }
 }
 
-__global__ void k_col_count(uint32_t nnz, const uint32_t *col, uint32_t *count)
+// cptr[j] = first place of a column >= j among the sorted columns, j = 0 .. m (a search per column:
+// no counting by atomics, and columns without elements cost no more than others)
+__global__ void k_col_starts(uint32_t nnz, uint32_t m, const uint32_t *__restrict__ sorted,
+                             uint32_t *__restrict__ cptr)
 {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < nnz) atomicAdd(count + col[e], 1u);
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j > m) return;
+    uint32_t lo = 0, hi = nnz;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (__ldg(sorted + mid) < j) lo = mid + 1;
+        else hi = mid;
+    }
+    cptr[j] = lo;
 }
 
-__global__ void k_t_meta(uint32_t m, const uint64_t *cptr, const uint32_t *tperm, uint32_t *nmc,
+__global__ void k_t_meta(uint32_t m, const uint32_t *cptr, const uint32_t *tperm, uint32_t *nmc,
                          uint32_t *tlen, uint32_t *tstart)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= m) return;
-    const uint32_t j = tperm[g], b = (uint32_t)cptr[j], l = (uint32_t)cptr[j + 1] - b;
+    const uint32_t j = tperm[g], b = cptr[j], l = cptr[j + 1] - b;
     tlen[g] = l;
     tstart[g] = b;
     if ((g & 31) == 0) nmc[g >> 5] = l;
 }
 
-__global__ void k_narrow(uint32_t n, const uint64_t *a, uint32_t *b)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (uint32_t)a[i];
-}
-
-// largest u + 1 over units of split chunks (the prefix the partial sums need)
-__global__ void k_split_extent(uint32_t units, const uint32_t *unit_chunk,
-                               const uint32_t *unit_base, uint32_t *out)
-{
-    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= units) return;
-    const uint32_t c = unit_chunk[u];
-    if (unit_base[c + 1] - unit_base[c] > 1) atomicMax(out, u + 1);
-}
-
 unsigned blocks_of(size_t n) { return (unsigned)((n + 255) / 256); }
-
-gs_status split_extent(uint32_t units, const uint32_t *uc, const uint32_t *ub, uint32_t *out,
-                       cudaStream_t s)
-{
-    *out = 0;
-    if (!units) return GS_OK;
-    StreamBuf d(s);
-    GS_TRY(d.alloc_zero(4));
-    k_split_extent<<<blocks_of(units), 256, 0, s>>>(units, uc, ub, d.as<uint32_t>());
-    GS_CHECK_LAUNCH();
-    GS_CUDA(cudaMemcpyAsync(out, d.p, 4, cudaMemcpyDeviceToHost, s));
-    GS_CUDA(cudaStreamSynchronize(s));
-    return GS_OK;
-}
 
 template <class T, bool ADJ>
 gs_status launch_mm(const MMArgs &a, uint32_t k, cudaStream_t s)
@@ -433,8 +413,6 @@ gs_status ensure_mm_scratch(gs_matrix *A, cudaStream_t s)
 {
     std::lock_guard<std::mutex> lock(g_mm_mutex);
     if (A->mm_ready) return GS_OK;
-    GS_TRY(split_extent(A->k1units, A->k1unit_chunk.as<uint32_t>(), A->k1unit_base.as<uint32_t>(),
-                        &A->k1split_units, s));
     GS_TRY(A->mmpartial.alloc((size_t)A->k1split_units * 32 * 32 * 8 + 8, s));
     A->mm_ready = true;
     return GS_OK;
@@ -531,9 +509,10 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(A->vrow.alloc((size_t)nnz * 4, s));
     GS_TRY(A->vcol.alloc((size_t)nnz * 4, s));
     // CSC order of the elements: stable sort of CSR indices by ascending column
-    StreamBuf ccount(s), csc(s), cptr(s), csr2f(s), inv(s);
-    GS_TRY(ccount.alloc_zero((size_t)m * 4));
+    StreamBuf ccount(s), csc(s), csorted(s), cptr(s), csr2f(s), inv(s);
+    GS_TRY(ccount.alloc((size_t)m * 4));
     GS_TRY(csc.alloc((size_t)nnz * 4));
+    GS_TRY(csorted.alloc((size_t)nnz * 4));
     GS_TRY(csr2f.alloc((size_t)nnz * 4));
     GS_TRY(inv.alloc((size_t)n * 4));
     if (n) {
@@ -547,21 +526,25 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
         k_forward_slots<<<blocks_of(nnz), 256, 0, s>>>(
             nnz, A->vrow.as<uint32_t>(), d_row, inv.as<uint32_t>(),
             A->chp.as<uint32_t>(), csr2f.as<uint32_t>());
-        k_col_count<<<blocks_of(nnz), 256, 0, s>>>(nnz, d_col, ccount.as<uint32_t>());
         GS_CHECK_LAUNCH();
-        GS_TRY(stable_sort_asc(d_col, nnz, m ? m - 1 : 0, csc.as<uint32_t>(), s));
+        GS_TRY(stable_sort_asc(d_col, nnz, m ? m - 1 : 0, csc.as<uint32_t>(),
+                               csorted.as<uint32_t>(), s));
     }
-    GS_TRY(cptr.alloc(((size_t)m + 1) * 8));
-    {
-        CountSpec cc{CountKind::Array};
-        cc.arr = ccount.as<uint32_t>();
-        GS_TRY(exclusive_scan(cc, m, cptr.as<uint64_t>(), nullptr, s));
-    }
+    GS_TRY(cptr.alloc(((size_t)m + 1) * 4));
+    k_col_starts<<<m / 256 + 1, 256, 0, s>>>(nnz, m, csorted.as<uint32_t>(), cptr.as<uint32_t>());
+    GS_CHECK_LAUNCH();
     // K1 layout of A^T: columns of A sorted by decreasing length
     const uint32_t tchunks = (m + 31) / 32;
     A->tchunkNum = tchunks;
-    uint32_t maxlen = 0;
-    GS_TRY(reduce_max_u32(ccount.as<uint32_t>(), m, &maxlen, s));
+    uint32_t top[2] = {0, 0};  // (check), longest column
+    {
+        StreamBuf out(s);
+        GS_TRY(out.alloc_zero(8));
+        GS_TRY(row_lengths(m, cptr.as<uint32_t>(), nnz, ccount.as<uint32_t>(), out.as<uint32_t>(), s));
+        GS_CUDA(cudaMemcpyAsync(top, out.p, 8, cudaMemcpyDeviceToHost, s));
+        GS_CUDA(cudaStreamSynchronize(s));
+    }
+    const uint32_t maxlen = top[1];
     GS_TRY(A->tpermi.alloc_zero(((size_t)tchunks + 1) * 32 * 4, s));
     GS_TRY(stable_sort_desc(ccount.as<uint32_t>(), m, maxlen, A->tpermi.as<uint32_t>(), s));
     GS_TRY(A->tnmc.alloc_zero((size_t)tchunks * 4 + 4, s));
@@ -569,32 +552,24 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     StreamBuf tstart(s);
     GS_TRY(tstart.alloc((size_t)m * 4));
     if (m) {
-        k_t_meta<<<blocks_of(m), 256, 0, s>>>(m, cptr.as<uint64_t>(), A->tpermi.as<uint32_t>(),
+        k_t_meta<<<blocks_of(m), 256, 0, s>>>(m, cptr.as<uint32_t>(), A->tpermi.as<uint32_t>(),
                                               A->tnmc.as<uint32_t>(), A->tlen.as<uint32_t>(),
                                               tstart.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
-    StreamBuf P(s);
-    GS_TRY(P.alloc(((size_t)tchunks + 1) * 8));
-    uint64_t lenvc = 0;
-    {
-        CountSpec cs{CountKind::ArrayTimes};
-        cs.arr = A->tnmc.as<uint32_t>();
-        cs.a = 32;
-        GS_TRY(exclusive_scan(cs, tchunks, P.as<uint64_t>(), &lenvc, s));
-    }
-    if (lenvc > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "transposed K1 exceeds 32-bit slots");
-    A->tlenVC = (uint32_t)lenvc;
     GS_TRY(A->tchp.alloc((size_t)tchunks * 4 + 4, s));
-    if (tchunks) {
-        k_narrow<<<blocks_of(tchunks), 256, 0, s>>>(tchunks, P.as<uint64_t>(), A->tchp.as<uint32_t>());
-        GS_CHECK_LAUNCH();
-    }
+    GS_TRY(A->tunit_base.alloc(((size_t)tchunks + 1) * 4, s));
+    uint64_t total[3] = {0, 0, 0};
+    GS_TRY(k1_layout_scan(A->tnmc.as<uint32_t>(), tchunks, A->tchp.as<uint32_t>(),
+                          A->tunit_base.as<uint32_t>(), total, s));
+    if (total[0] > 0xffffffffull) return fail(GS_ERR_OVERFLOW, "transposed K1 exceeds 32-bit slots");
+    if (total[1] >= 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 plan too large");
+    A->tlenVC = (uint32_t)total[0];
+    A->tunits = (uint32_t)total[1];
+    A->tsplit_units = (uint32_t)total[2];
     const size_t vsz = A->p.vtype == GS_F64 ? 8 : 4;
-    GS_TRY(build_k1_plan(A->tnmc.as<uint32_t>(), tchunks, A->tunit_chunk, A->tunit_base,
-                         A->tpartial1, A->tcount, &A->tunits, s));
-    GS_TRY(split_extent(A->tunits, A->tunit_chunk.as<uint32_t>(), A->tunit_base.as<uint32_t>(),
-                        &A->tsplit_units, s));
+    GS_TRY(build_k1_units(A->tunit_base.as<uint32_t>(), tchunks, A->tunits, A->tunit_chunk,
+                          nullptr, A->tcount, s));
     GS_TRY(A->tpartial.alloc((size_t)A->tsplit_units * 32 * 32 * 8 + 8, s));
     GS_TRY(A->trow.alloc((size_t)A->tlenVC * 4, s));
     GS_TRY(A->tsrc.alloc((size_t)A->tlenVC * 4, s));

@@ -252,39 +252,24 @@ __global__ void __launch_bounds__(256) k_k1_deltas(const K1Args a, const uint32_
     }
 }
 
-__global__ void k_k1_units(const uint64_t *ubase64, const uint32_t *nmc, uint32_t chunkNum,
-                           uint32_t *unit_chunk, uint32_t *unit_base)
+__global__ void k_k1_units(const uint32_t *unit_base, uint32_t chunkNum, uint32_t *unit_chunk)
 {
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c <= chunkNum) unit_base[c] = (uint32_t)ubase64[c];
-    if (c < chunkNum) {
-        uint32_t b = (uint32_t)ubase64[c], e = (uint32_t)ubase64[c + 1];
-        for (uint32_t u = b; u < e; u++) unit_chunk[u] = c;
-    }
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < chunkNum)
+        for (uint32_t u = unit_base[c]; u < unit_base[c + 1]; u++) unit_chunk[u] = c;
 }
 
 }  // namespace
 
-gs_status build_k1_plan(const uint32_t *d_nmc, uint32_t chunkNum, DevBuf &unit_chunk,
-                        DevBuf &unit_base, DevBuf &partial, DevBuf &count, uint32_t *units,
-                        cudaStream_t s)
+gs_status build_k1_units(const uint32_t *unit_base, uint32_t chunkNum, uint32_t units,
+                         DevBuf &unit_chunk, DevBuf *partial, DevBuf &count, cudaStream_t s)
 {
-    StreamBuf pre(s);
-    GS_TRY(pre.alloc(((size_t)chunkNum + 1) * 8));
-    CountSpec spec{CountKind::PiecesMin1};
-    spec.arr = d_nmc;
-    spec.a = kK1Split;
-    uint64_t total = 0;
-    GS_TRY(exclusive_scan(spec, chunkNum, pre.as<uint64_t>(), &total, s));
-    if (total >= 0xffffffffull) return fail(GS_ERR_OVERFLOW, "K1 plan too large");
-    *units = (uint32_t)total;
-    GS_TRY(unit_chunk.alloc((size_t)total * 4, s));
-    GS_TRY(unit_base.alloc(((size_t)chunkNum + 1) * 4, s));
-    GS_TRY(partial.alloc((size_t)total * 32 * 8, s));
+    GS_TRY(unit_chunk.alloc((size_t)units * 4, s));
+    if (partial) GS_TRY(partial->alloc((size_t)units * 32 * 8, s));
     GS_TRY(count.alloc_zero((size_t)chunkNum * 4, s));
-    k_k1_units<<<(chunkNum + 256) / 256, 256, 0, s>>>(pre.as<uint64_t>(), d_nmc, chunkNum,
-                                                     unit_chunk.as<uint32_t>(),
-                                                     unit_base.as<uint32_t>());
+    if (!chunkNum) return GS_OK;
+    k_k1_units<<<(chunkNum + 255) / 256, 256, 0, s>>>(unit_base, chunkNum,
+                                                     unit_chunk.as<uint32_t>());
     GS_CHECK_LAUNCH();
     return GS_OK;
 }
