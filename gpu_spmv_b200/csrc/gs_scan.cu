@@ -436,16 +436,16 @@ gs_status k1_layout_scan(const uint32_t *nmc, uint32_t n, uint32_t *chp, uint32_
 // moves (8 in, 8 out per element; the first reads only the keys and makes the indices, the last
 // writes only the indices), so the wider the digit the fewer the bytes: one bit a pass took 14
 // passes for row lengths and 20 for a million columns.  A block ranks a tile of kRadixTile
-// elements: warps rank their own 512 in order (match of equal digits, one counter per digit and
+// elements: warps rank their own 256 in order (ballots of equal digits, one counter per digit and
 // warp), the warps' counts are summed per digit, and the tile is reordered in shared memory
 // before it is written, so that a digit's elements leave as one run (64 bytes on average with
 // 256 digits and 4096 elements).  Between blocks there is no waiting: the tiles' digit counts
 // are made by a pass of their own and scanned by one block per digit.
-// 4.2M elements, 20-bit keys: 20 passes of one bit 1310 us, 3 passes of 7 bits RADIX_US us (with
-// match.any instead of ballots for the ranks about 150).
-constexpr int kRadixThreads = 256;
+// 4.2M elements, 20-bit keys: 20 passes of one bit 1310 us, 3 passes of 7 bits about 130 us
+// (150 in blocks of 256 threads with 16 elements each, whose registers left 3 blocks on an SM).
+constexpr int kRadixThreads = 512;
 constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kRadixItems = 16;
+constexpr int kRadixItems = 8;
 constexpr uint32_t kRadixTile = kRadixThreads * kRadixItems;
 constexpr int kRadixDigits = 256;
 
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_count(
     uint32_t mask, uint32_t tiles, uint32_t *__restrict__ count)
 {
     __shared__ uint32_t h[kRadixDigits];
-    h[threadIdx.x] = 0;
+    if (threadIdx.x < kRadixDigits) h[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t t0 = blockIdx.x * kRadixTile;
 #pragma unroll
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     const uint32_t *__restrict__ before, const uint32_t *__restrict__ total,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ iout)
 {
-    __shared__ uint32_t wcount[kRadixWarps][kRadixDigits];
+    __shared__ uint16_t wcount[kRadixWarps][kRadixDigits];
     __shared__ uint32_t start[kRadixDigits];  // digit's first position in the sorted tile
     __shared__ uint32_t dest[kRadixDigits];   // output index of that position
     __shared__ uint32_t skey[kRadixTile], sidx[kRadixTile];
@@ -533,8 +533,8 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t t0 = blockIdx.x * kRadixTile;
     const uint32_t cnt = min(kRadixTile, n - t0);
-#pragma unroll
-    for (int i = 0; i < kRadixWarps; i++) wcount[i][threadIdx.x] = 0;
+    for (int i = threadIdx.x; i < kRadixWarps * kRadixDigits / 2; i += kRadixThreads)
+        reinterpret_cast<uint32_t *>(&wcount[0][0])[i] = 0;
     __syncthreads();
     uint32_t key[kRadixItems], idx[kRadixItems], rank[kRadixItems];
     const uint32_t o0 = (uint32_t)w * 32u * kRadixItems + (uint32_t)lane;
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
             const uint32_t below = (uint32_t)__popc(peers & ((1u << lane) - 1u));
             rank[i] = wcount[w][d] + below;
             __syncwarp(live);
-            if (below == 0) wcount[w][d] += (uint32_t)__popc(peers);
+            if (below == 0) wcount[w][d] += (uint16_t)__popc(peers);
             __syncwarp(live);
         }
     }
@@ -569,16 +569,20 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(
     {
         const uint32_t d = threadIdx.x;
         uint32_t run = 0;
+        if (d < kRadixDigits) {
 #pragma unroll
-        for (int i = 0; i < kRadixWarps; i++) {
-            const uint32_t c = wcount[i][d];
-            wcount[i][d] = run;
-            run += c;
+            for (int i = 0; i < kRadixWarps; i++) {
+                const uint32_t c = wcount[i][d];
+                wcount[i][d] = (uint16_t)run;
+                run += c;
+            }
         }
         const uint32_t e = radix_block_scan(run, wsum, &sum);
-        start[d] = e;
         const uint32_t g = radix_block_scan(d <= mask ? total[d] : 0u, wsum, &sum);
-        dest[d] = d <= mask ? g + before[(size_t)d * tiles + blockIdx.x] : 0u;
+        if (d < kRadixDigits) {
+            start[d] = e;
+            dest[d] = d <= mask ? g + before[(size_t)d * tiles + blockIdx.x] : 0u;
+        }
     }
     __syncthreads();
 #pragma unroll

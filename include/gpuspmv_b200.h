@@ -356,7 +356,7 @@ gs_status gs_spmv_host_stream(const gs_matrix *A, const void *h_x, size_t x_stri
                               UIN count, UIN flags, gs_stream stream);
 
 /* Device memory of destroyed matrices and of conversions' scratch is kept for the next ones,
- * up to 1 GiB per device; gs_release_cached gives it back to the device now (the current one;
+ * up to 4 GiB per device; gs_release_cached gives it back to the device now (the current one;
  * waits for it). */
 gs_status gs_release_cached(void);
 
