@@ -241,6 +241,9 @@ SIGNATURES = {
     "gs_csr_spmv_f64": (_st, [UIN, UIN, UIN, _vp, _vp, _vp, _vp, _vp, _vp]),
     "gs_k1_spmv_f64_static": (_st, [UIN, UIN, UIN, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "gs_spmm": (_st, [_vp, _vp, _vp, C.c_int, UIN, _vp]),
+    "gs_spmm_strided": (_st, [_vp, _vp, UIN, _vp, UIN, C.c_int, UIN, UIN, _vp]),
+    "gs_spmm_adjoint_strided": (_st, [_vp, _vp, UIN, _vp, UIN, _vp, UIN, _vp, C.c_int, UIN, UIN,
+                                      _vp]),
     "gs_matrix_prepare_adjoint": (_st, [_vp, _vp, _vp, _vp]),
     "gs_matrix_set_values": (_st, [_vp, _vp, C.c_int, C.c_int, _vp]),
     "gs_matrix_value_slots": (_st, [_vp, C.POINTER(UIN)]),

@@ -131,6 +131,7 @@ struct MMArgs {
     uint32_t *count;                           // chunks * nrb arrival counters
     uint32_t ld;                               // row stride of X, Y (= K for one block)
     uint32_t nrb;                              // right-hand-side blocks per unit
+    uint32_t k, ldx, ldy;                      // mm_unit_wide: columns, row strides of X and Y
 };
 
 // Unit u of the layout, right-hand-side block rb (columns rb*K .. rb*K+K-1 of X, Y), by
@@ -265,6 +266,150 @@ __device__ __forceinline__ void mm_unit(const MMArgs &a, uint32_t u, uint32_t rb
     }
 }
 
+// VEC consecutive values: 32, 16, 8 or 4 bytes, aligned to that
+template <class T, int VEC>
+__device__ __forceinline__ void load_slice(const T *p, T (&v)[VEC])
+{
+    if constexpr (VEC * sizeof(T) == 32) {
+        ld32(p, v);
+    } else if constexpr (VEC * sizeof(T) == 16) {
+        load_row<T, VEC>(p, 0, 0, v);
+    } else if constexpr (VEC == 2 && sizeof(T) == 4) {
+        const float2 w = __ldg(reinterpret_cast<const float2 *>(p));
+        v[0] = w.x;
+        v[1] = w.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < VEC; i++) v[i] = __ldg(p + i);
+    }
+}
+
+// Unit u of the layout for any number a.k <= L * VEC of right-hand sides and any row strides, by
+// one warp (the rows of X readable up to the next multiple of VEC columns).  Lane = sorted row for the streams, as in mm_unit; the gathers go
+// by L lanes per row, VEC columns each, 32 / L rows an instruction: a row of X is one request
+// whatever its width (a lane that gathers a whole row of 64 bytes or more asks for its line twice
+// or more), and rows need neither padding nor 32-byte alignment.  Each lane sums its columns of
+// all 32 rows, one row after the other in step order: the sums and their order are mm_unit's.
+template <class T, int VEC, int L>
+__device__ __forceinline__ void mm_unit_wide(const MMArgs &a, uint32_t u)
+{
+    using A = Arith<T>;
+    constexpr int G = 32 / L;  // rows per instruction
+    // steps in flight: about 128 bytes of gathered slices per lane, 64 where the slices are below
+    // 16 bytes and the lanes many (FP64 k = 8, a band / a 524,288-row power-law with 128 and 64:
+    // 46 / 74 and 56 / 91 us; k = 5 in 8-byte slices 79 / 110 and 68 / 126)
+    constexpr int SB = L * VEC * (int)sizeof(T);  // bytes per step
+    constexpr int WB = VEC * (int)sizeof(T) >= 16 ? 128 : 64;
+    constexpr int B = SB >= WB ? 1 : (WB / SB > 4 ? 4 : WB / SB);
+    const T *__restrict__ val = static_cast<const T *>(a.val);
+    const int lane = threadIdx.x & 31, li = lane % L, gi = lane / L;
+    const bool act = (uint32_t)(li * VEC) < a.k;
+    const T *__restrict__ xin = static_cast<const T *>(a.xin) + li * VEC;
+    T *__restrict__ partial = static_cast<T *>(a.partial);
+    uint32_t c, ub = u, np = 1;
+    if (u >= a.split_units) {
+        c = u - a.split_extra;
+    } else {
+        c = __ldg(a.unit_chunk + u);
+        ub = __ldg(a.unit_base + c);
+        np = __ldg(a.unit_base + c + 1) - ub;
+    }
+    const uint32_t g = 32u * c + (uint32_t)lane;
+    const bool valid = g < a.nrows;
+    const uint32_t len = valid ? __ldg(a.klen + g) : 0u;
+    const uint32_t j0 = (u - ub) * kK1Split, j1 = min(len, j0 + kK1Split);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, j1);
+    const uint32_t base = __ldg(a.chp + c) + (uint32_t)lane;
+    const uint32_t me = valid ? __ldg(a.permi + g) : 0xffffffffu;
+    T acc[L][VEC];
+#pragma unroll
+    for (int q = 0; q < L; q++)
+#pragma unroll
+        for (int i = 0; i < VEC; i++) acc[q][i] = T(0);
+    T v[B];
+    uint32_t cc[B];
+    auto streams = [&](uint32_t j, T(&sv)[B], uint32_t(&sc)[B]) {
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            const bool in = j + b < j1;
+            const uint32_t pos = base + 32u * (j + b);
+            sv[b] = in ? __ldcs(val + pos) : T(0);
+            sc[b] = in ? __ldcs(a.col + pos) : 0u;
+        }
+    };
+    streams(j0, v, cc);
+    for (uint32_t j = j0; j < top; j += B) {
+        T gv[B][L][VEC], vn[B];
+        uint32_t cn[B];
+        unsigned live[B];
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            live[b] = __ballot_sync(0xffffffffu, j + b < j1);
+#pragma unroll
+            for (int q = 0; q < L; q++) {
+                const int src = q * G + gi;
+                const uint32_t cq = __shfl_sync(0xffffffffu, cc[b], src);
+                if (act && ((live[b] >> src) & 1u))
+                    load_slice<T, VEC>(xin + (size_t)cq * a.ldx, gv[b][q]);
+            }
+        }
+        streams(j + B, vn, cn);
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+#pragma unroll
+            for (int q = 0; q < L; q++) {
+                const int src = q * G + gi;
+                const T vq = __shfl_sync(0xffffffffu, v[b], src);
+                if (act && ((live[b] >> src) & 1u)) {
+#pragma unroll
+                    for (int i = 0; i < VEC; i++)
+                        acc[q][i] = A::add(acc[q][i], A::mul(vq, gv[b][q][i]));
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            v[b] = vn[b];
+            cc[b] = cn[b];
+        }
+    }
+    T *__restrict__ yout = static_cast<T *>(a.yout) + li * VEC;
+    if (np == 1) {
+#pragma unroll
+        for (int q = 0; q < L; q++) {
+            const uint32_t r = __shfl_sync(0xffffffffu, me, q * G + gi);
+            if (act && r != 0xffffffffu) {
+#pragma unroll
+                for (int i = 0; i < VEC; i++)
+                    if ((uint32_t)(li * VEC + i) < a.k) yout[(size_t)r * a.ldy + i] = acc[q][i];
+            }
+        }
+        return;
+    }
+    // a cut chunk: 32 x 32 partial sums per unit, column by column; the last piece adds them
+    if (act) {
+#pragma unroll
+        for (int q = 0; q < L; q++)
+#pragma unroll
+            for (int i = 0; i < VEC; i++)
+                partial[((size_t)u * 32 + li * VEC + i) * 32 + q * G + gi] = acc[q][i];
+    }
+    __threadfence();
+    __syncwarp();
+    uint32_t ticket = 0;
+    if (lane == 0) ticket = atomicAdd(a.count + c, 1u);
+    ticket = __shfl_sync(0xffffffffu, ticket, 0);
+    if (ticket == np - 1) {
+        __threadfence();
+        for (uint32_t k = 0; k < a.k; k++) {
+            T s = T(0);
+            for (uint32_t q = 0; q < np; q++)
+                s = A::add(s, __ldcg(partial + ((size_t)(ub + q) * 32 + k) * 32 + lane));
+            if (valid) static_cast<T *>(a.yout)[(size_t)me * a.ldy + k] = s;
+        }
+        if (lane == 0) a.count[c] = 0;
+    }
+}
 
 }  // namespace mm
 }  // namespace gs

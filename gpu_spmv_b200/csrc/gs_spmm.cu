@@ -19,7 +19,9 @@
 // adds (its rounding order varies between runs).
 //
 // The reference has no multi-RHS product and no adjoint; these extend its K1 format.
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "gs_k1_fill.cuh"
 #include "gs_mm.cuh"
@@ -146,39 +148,28 @@ __global__ void __launch_bounds__(256) k_k1_adj_atomic(const AtomicArgs a)
 // is 84 us.
 struct VbarArgs {
     uint32_t nnz;
+    uint32_t k, ldx, ldy;  // right-hand sides, row strides of X and Ybar
     const uint32_t *row, *col;
     const void *x, *ybar;
     void *vbar;
 };
 
-template <class T, int VEC>
-__device__ __forceinline__ void load_slice(const T *p, T (&v)[VEC])
-{
-    if constexpr (VEC * sizeof(T) == 32) {
-        ld32(p, v);
-    } else if constexpr (VEC * sizeof(T) == 16) {
-        load_row<T, VEC>(p, 0, 0, v);
-    } else {
-#pragma unroll
-        for (int i = 0; i < VEC; i++) v[i] = __ldg(p + i);
-    }
-}
-
 constexpr int kVbarThreads = 64;
 constexpr int kVbarSteps = 8;  // steps of a warp, over consecutive elements (32: 2 % slower)
 constexpr int kVbarUnroll = 2;  // elements per lane and step (1 / 4: 4 / 2 % slower in all)
-template <class T, int K>
+// CHAIN: L * VEC = k, and the sum goes from lane to lane in the order of the right-hand sides, as
+// in the transposed pass; else the lanes' sums meet in a tree.
+template <class T, int VEC, int L, bool CHAIN>
 __global__ void __launch_bounds__(kVbarThreads, 12) k_vbar(const VbarArgs a)
 {
     using A = Arith<T>;
-    constexpr int L = K * (int)sizeof(T) > 32 ? K * (int)sizeof(T) / 32 : 1;
-    constexpr int VEC = K / L;
     constexpr int U = kVbarUnroll, E = 32 / L * U;  // elements per step
     const int lane = threadIdx.x & 31, li = lane % L;
     const uint64_t warp = blockIdx.x * (uint64_t)(kVbarThreads / 32) + (threadIdx.x >> 5);
     const T *__restrict__ x = static_cast<const T *>(a.x) + li * VEC;
     const T *__restrict__ yb = static_cast<const T *>(a.ybar) + li * VEC;
     T *__restrict__ vbar = static_cast<T *>(a.vbar);
+    const bool act = CHAIN || (uint32_t)(li * VEC) < a.k;
     uint64_t e0 = warp * (uint64_t)(E * kVbarSteps) + (uint64_t)(lane / L);
     uint32_t r[U], c[U];
     auto indices = [&](uint64_t e, uint32_t(&ri)[U], uint32_t(&ci)[U]) {
@@ -196,9 +187,9 @@ __global__ void __launch_bounds__(kVbarThreads, 12) k_vbar(const VbarArgs a)
         uint32_t rn[U], cn[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (e0 + (uint64_t)(u * (32 / L)) < a.nnz) {
-                load_slice<T, VEC>(x + (size_t)c[u] * K, xs[u]);
-                load_slice<T, VEC>(yb + (size_t)r[u] * K, ys[u]);
+            if (act && e0 + (uint64_t)(u * (32 / L)) < a.nnz) {
+                load_slice<T, VEC>(x + (size_t)c[u] * a.ldx, xs[u]);
+                load_slice<T, VEC>(yb + (size_t)r[u] * a.ldy, ys[u]);
             }
         }
         // the next step's indices load while this one's rows are gathered
@@ -206,39 +197,131 @@ __global__ void __launch_bounds__(kVbarThreads, 12) k_vbar(const VbarArgs a)
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const uint64_t e = e0 + (uint64_t)(u * (32 / L));
-            T d = T(0);  // the sum goes from lane to lane, in the order of the right-hand sides
+            T d = T(0);
+            if constexpr (CHAIN) {
 #pragma unroll
-            for (int st = 0; st < L; st++) {
-                T q = st ? __shfl_up_sync(0xffffffffu, d, 1) : T(0);
-                if (e < a.nnz) {
+                for (int st = 0; st < L; st++) {
+                    T q = st ? __shfl_up_sync(0xffffffffu, d, 1) : T(0);
+                    if (e < a.nnz) {
 #pragma unroll
-                    for (int k = 0; k < VEC; k++) q = A::add(q, A::mul(ys[u][k], xs[u][k]));
+                        for (int k = 0; k < VEC; k++) q = A::add(q, A::mul(ys[u][k], xs[u][k]));
+                    }
+                    if (li == st) d = q;
                 }
-                if (li == st) d = q;
+                if (li == L - 1 && e < a.nnz) __stcs(vbar + e, d);
+            } else {
+                if (act && e < a.nnz) {
+#pragma unroll
+                    for (int k = 0; k < VEC; k++)
+                        if ((uint32_t)(li * VEC + k) < a.k)
+                            d = A::add(d, A::mul(ys[u][k], xs[u][k]));
+                }
+#pragma unroll
+                for (int o = L / 2; o; o >>= 1)
+                    d = A::add(d, __shfl_xor_sync(0xffffffffu, d, o));
+                if (li == 0 && e < a.nnz) __stcs(vbar + e, d);
             }
-            if (li == L - 1 && e < a.nnz) __stcs(vbar + e, d);
         }
 #pragma unroll
         for (int u = 0; u < U; u++) r[u] = rn[u], c[u] = cn[u];
     }
 }
 
-template <class T> gs_status launch_vbar(const VbarArgs &a, uint32_t k, cudaStream_t s)
+template <class T, int VEC, int L, bool CHAIN>
+gs_status launch_vbar_t(const VbarArgs &a, cudaStream_t s)
 {
     if (!a.nnz) return GS_OK;
-#define GS_V(K_)                                                                            \
-    case K_: {                                                                              \
-        const uint32_t l = max(1u, K_ * (uint32_t)sizeof(T) / 32u), per = (uint32_t)(kVbarThreads / 32 * kVbarSteps * kVbarUnroll) * (32u / l); \
-        k_vbar<T, K_><<<(a.nnz - 1u) / per + 1u, kVbarThreads, 0, s>>>(a);                          \
-        break;                                                                              \
+    const uint32_t per = (uint32_t)(kVbarThreads / 32 * kVbarSteps * kVbarUnroll * (32 / L));
+    k_vbar<T, VEC, L, CHAIN><<<(a.nnz - 1u) / per + 1u, kVbarThreads, 0, s>>>(a);
+    GS_CHECK_LAUNCH();
+    return GS_OK;
+}
+
+// k a power of two, rows contiguous and 32-byte aligned
+template <class T> gs_status launch_vbar(const VbarArgs &a, uint32_t k, cudaStream_t s)
+{
+#define GS_V(K_)                                                                             \
+    case K_: {                                                                               \
+        constexpr int l = K_ * (int)sizeof(T) > 32 ? K_ * (int)sizeof(T) / 32 : 1;           \
+        return launch_vbar_t<T, K_ / l, l, true>(a, s);                                      \
     }
     switch (k) {
-        GS_V(1u) GS_V(2u) GS_V(4u) GS_V(8u) GS_V(16u) GS_V(32u)
+        GS_V(1) GS_V(2) GS_V(4) GS_V(8) GS_V(16) GS_V(32)
     default: return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1, 2, 4, 8, 16, 32)", k);
     }
 #undef GS_V
-    GS_CHECK_LAUNCH();
-    return GS_OK;
+}
+
+// ------------------------------------------------------------------ any k, any row strides
+// Registers before warps, as for k_k1_mm: 12 warps per SM hold the 192 and 256 bytes of sums a lane
+// of FP64 k = 24 / 32 has (397 / 395 us with 16 and spills, 280 / 297 with 12).
+template <class T, int VEC, int L>
+constexpr int kWideBlocks = (L * VEC * (int)sizeof(T) >= 192
+                                 ? 12
+                                 : (L * VEC * (int)sizeof(T) >= 64 ? 16 : 24)) / 2;
+template <class T, int VEC, int L>
+__global__ void __launch_bounds__(kMMThreads, kWideBlocks<T, VEC, L>)
+    k_k1_mm_wide(const MMArgs a)
+{
+    const uint32_t u = blockIdx.x * (kMMThreads / 32) + (threadIdx.x >> 5);
+    if (u < a.units) mm_unit_wide<T, VEC, L>(a, u);
+}
+
+// f(VEC, L) for k right-hand sides in rows that are readable up to column `cols` and whose slices
+// may start at multiples of `align` bytes: the widest slice up to 32 bytes, lanes a power of two
+template <class T, class F> gs_status with_slices(uint32_t k, uint32_t cols, uint32_t align, F f)
+{
+    auto pick = [&](auto vec) -> gs_status {
+        constexpr int V = decltype(vec)::value;
+        const uint32_t need = (k + V - 1) / V;
+        if (need <= 1) return f(vec, std::integral_constant<int, 1>());
+        if (need <= 2) return f(vec, std::integral_constant<int, 2>());
+        if (need <= 4) return f(vec, std::integral_constant<int, 4>());
+        if constexpr (32 / V >= 8)
+            if (need <= 8) return f(vec, std::integral_constant<int, 8>());
+        if constexpr (32 / V >= 16)
+            if (need <= 16) return f(vec, std::integral_constant<int, 16>());
+        if constexpr (32 / V >= 32) return f(vec, std::integral_constant<int, 32>());
+        return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1..32)", k);
+    };
+    auto fits = [&](uint32_t v) {
+        return v <= k && align % (v * sizeof(T)) == 0 && (k + v - 1) / v * v <= cols;
+    };
+    if constexpr (sizeof(T) == 4)
+        if (fits(8) || (k > 4 && align % 32 == 0 && cols >= 8 && (k + 7) / 8 * 8 <= cols))
+            return pick(std::integral_constant<int, 8>());
+    if (fits(4) || (k == 3 && align % (4 * sizeof(T)) == 0 && cols >= 4))
+        return pick(std::integral_constant<int, 4>());
+    if (fits(2)) return pick(std::integral_constant<int, 2>());
+    return pick(std::integral_constant<int, 1>());
+}
+
+// largest power of two up to 32 that divides a pointer and a row stride in bytes
+uint32_t row_align(const void *p, size_t stride)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(p) | stride | 32u;
+    return (uint32_t)(x & (~x + 1));
+}
+
+template <class T> gs_status launch_mm_wide(const MMArgs &a, uint32_t cols, cudaStream_t s)
+{
+    if (!a.units) return GS_OK;
+    const uint32_t align = row_align(a.xin, (size_t)a.ldx * sizeof(T));
+    return with_slices<T>(a.k, cols, align, [&](auto vec, auto lanes) -> gs_status {
+        k_k1_mm_wide<T, decltype(vec)::value, decltype(lanes)::value>
+            <<<(a.units + kMMThreads / 32 - 1) / (kMMThreads / 32), kMMThreads, 0, s>>>(a);
+        GS_CHECK_LAUNCH();
+        return GS_OK;
+    });
+}
+
+template <class T> gs_status launch_vbar_wide(const VbarArgs &a, uint32_t cols, cudaStream_t s)
+{
+    const uint32_t align = std::min(row_align(a.x, (size_t)a.ldx * sizeof(T)),
+                                    row_align(a.ybar, (size_t)a.ldy * sizeof(T)));
+    return with_slices<T>(a.k, cols, align, [&](auto vec, auto lanes) -> gs_status {
+        return launch_vbar_t<T, decltype(vec)::value, decltype(lanes)::value, false>(a, s);
+    });
 }
 
 // ------------------------------------------------------------------ layout helpers
@@ -452,6 +535,80 @@ gs_status refresh_values(gs_matrix *A, const T *v, gs_value_order order, cudaStr
     return GS_OK;
 }
 
+// The forward layout and its plan; Y = A X
+MMArgs forward_args(const gs_matrix *A, const void *x, void *y)
+{
+    MMArgs a{};
+    a.nrows = A->nrows;
+    a.permi = A->permi.as<uint32_t>();
+    a.nmc = A->nmc.as<uint32_t>();
+    a.chp = A->chp.as<uint32_t>();
+    a.klen = A->k1len.as<uint32_t>();
+    a.val = A->val.p;
+    a.col = A->col.as<uint32_t>();
+    a.xin = x;
+    a.yout = y;
+    a.unit_chunk = A->k1unit_chunk.as<uint32_t>();
+    a.unit_base = A->k1unit_base.as<uint32_t>();
+    a.units = A->k1units;
+    a.split_units = A->k1split_units;
+    a.split_extra = A->k1units - A->chunkNum;
+    a.partial = A->mmpartial.p;
+    a.count = A->k1count.as<uint32_t>();
+    a.nrb = 1;
+    return a;
+}
+
+// The transposed layout and its plan; Xbar = A^T Ybar
+MMArgs adjoint_args(const gs_matrix *A, const void *ybar, void *xbar)
+{
+    MMArgs a{};
+    a.nrows = A->ncols;
+    a.permi = A->tpermi.as<uint32_t>();
+    a.nmc = A->tnmc.as<uint32_t>();
+    a.chp = A->tchp.as<uint32_t>();
+    a.klen = A->tlen.as<uint32_t>();
+    a.val = A->tval.p;
+    a.col = A->trow.as<uint32_t>();
+    a.xin = ybar;
+    a.yout = xbar;
+    a.unit_chunk = A->tunit_chunk.as<uint32_t>();
+    a.unit_base = A->tunit_base.as<uint32_t>();
+    a.units = A->tunits;
+    a.split_units = A->tsplit_units;
+    a.split_extra = A->tunits - A->tchunkNum;
+    a.partial = A->tpartial.p;
+    a.count = A->tcount.as<uint32_t>();
+    a.nrb = 1;
+    return a;
+}
+
+// Rows of 64 bytes and more go by several lanes per row (FP64 k = 8 / 16 / 32, a band 60 / 138 / 293
+// -> 46 / 87 / 141 us, a 524,288-row power-law 96 / 246 / 400 -> 75 / 194 / 300; FP32 k = 32 140 ->
+// 83 and 264 -> 200), but for FP32 k = 16, whose two lanes a row lose on a 27-point stencil 80^3 (81
+// -> 99; a band 60 -> 53, the power-law 96 -> 96).
+bool several_lanes(uint32_t k, gs_dtype dtype)
+{
+    return dtype == GS_F64 ? k >= 8 : k > 16;
+}
+
+gs_status check_strided(const gs_matrix *A, gs_dtype dtype, uint32_t k, uint32_t cols)
+{
+    GS_TRY(check_mm_matrix(A));
+    if (dtype != A->p.vtype) return fail(GS_ERR_UNSUPPORTED, "operands take the value type");
+    if (k < 1 || k > 32) return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1..32)", k);
+    if (cols < k) return fail(GS_ERR_INVALID, "%u readable columns for k = %u", cols, k);
+    return GS_OK;
+}
+// rows of k entries, `ld` apart, each entry aligned to its size
+gs_status check_rows(const char *what, const void *p, uint32_t ld, uint32_t k, gs_dtype dtype)
+{
+    if (ld < k) return fail(GS_ERR_INVALID, "%s: row stride %u below %u columns", what, ld, k);
+    if (reinterpret_cast<uintptr_t>(p) % dtype_size(dtype))
+        return fail(GS_ERR_INVALID, "%s is not aligned to its entries", what);
+    return GS_OK;
+}
+
 }  // namespace
 
 gs_status prepare_mm_scratch(gs_matrix *A, cudaStream_t s) { return ensure_mm_scratch(A, s); }
@@ -472,25 +629,10 @@ gs_status gs_spmm(gs_matrix *A, const void *d_X, void *d_Y, gs_dtype dtype, UIN 
     if (!aligned32(d_X) || !aligned32(d_Y)) return fail(GS_ERR_INVALID, "X and Y must be 32-byte aligned");
     cudaStream_t s = cs(stream);
     GS_TRY(ensure_mm_scratch(A, s));
-    MMArgs a{};
-    a.nrows = A->nrows;
-    a.permi = A->permi.as<uint32_t>();
-    a.nmc = A->nmc.as<uint32_t>();
-    a.chp = A->chp.as<uint32_t>();
-    a.klen = A->k1len.as<uint32_t>();
-    a.val = A->val.p;
-    a.col = A->col.as<uint32_t>();
-    a.xin = d_X;
-    a.yout = d_Y;
-    a.unit_chunk = A->k1unit_chunk.as<uint32_t>();
-    a.unit_base = A->k1unit_base.as<uint32_t>();
-    a.units = A->k1units;
-    a.split_units = A->k1split_units;
-    a.split_extra = A->k1units - A->chunkNum;
-    a.partial = A->mmpartial.p;
-    a.count = A->k1count.as<uint32_t>();
-    a.ld = k;
-    a.nrb = 1;
+    MMArgs a = forward_args(A, d_X, d_Y);
+    a.ld = a.k = a.ldx = a.ldy = k;
+    if (several_lanes(k, dtype))
+        return dtype == GS_F64 ? launch_mm_wide<double>(a, k, s) : launch_mm_wide<float>(a, k, s);
     if (A->p.vtype == GS_F64) return launch_mm<double, false>(a, k, s);
     return launch_mm<float, false>(a, k, s);
 }
@@ -690,6 +832,7 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     if (csr_vbar) {
         VbarArgs v{};
         v.nnz = A->nnz;
+        v.k = v.ldx = v.ldy = k;
         v.row = A->vrow.as<uint32_t>();
         v.col = A->vcol.as<uint32_t>();
         v.x = d_X;
@@ -729,29 +872,69 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         }
         return GS_OK;
     }
-    MMArgs a{};
-    a.nrows = A->ncols;
-    a.permi = A->tpermi.as<uint32_t>();
-    a.nmc = A->tnmc.as<uint32_t>();
-    a.chp = A->tchp.as<uint32_t>();
-    a.klen = A->tlen.as<uint32_t>();
-    a.val = A->tval.p;
-    a.col = A->trow.as<uint32_t>();
-    a.xin = d_Ybar;
+    MMArgs a = adjoint_args(A, d_Ybar, d_Xbar);
     a.xrow = d_X;
-    a.yout = d_Xbar;
     a.vbar = csr_vbar ? nullptr : d_vbar;
-    a.unit_chunk = A->tunit_chunk.as<uint32_t>();
-    a.unit_base = A->tunit_base.as<uint32_t>();
-    a.units = A->tunits;
-    a.split_units = A->tsplit_units;
-    a.split_extra = A->tunits - A->tchunkNum;
-    a.partial = A->tpartial.p;
-    a.count = A->tcount.as<uint32_t>();
-    a.ld = k;
-    a.nrb = 1;
+    a.ld = a.k = a.ldx = a.ldy = k;
     if (a.vbar) return f64 ? launch_mm<double, true>(a, k, s) : launch_mm<float, true>(a, k, s);
+    if (several_lanes(k, dtype))
+        return f64 ? launch_mm_wide<double>(a, k, s) : launch_mm_wide<float>(a, k, s);
     return f64 ? launch_mm<double, false>(a, k, s) : launch_mm<float, false>(a, k, s);
+}
+
+gs_status gs_spmm_strided(gs_matrix *A, const void *d_X, UIN ldx, void *d_Y, UIN ldy,
+                          gs_dtype dtype, UIN k, UIN cols, gs_stream stream)
+{
+    if (!A || !d_X || !d_Y) return fail(GS_ERR_INVALID, "NULL argument");
+    GS_TRY(check_strided(A, dtype, k, cols));
+    GS_TRY(check_rows("X", d_X, ldx, cols, dtype));
+    GS_TRY(check_rows("Y", d_Y, ldy, k, dtype));
+    if (ldx == k && ldy == k && valid_k(k) && aligned32(d_X) && aligned32(d_Y))
+        return gs_spmm(A, d_X, d_Y, dtype, k, stream);
+    cudaStream_t s = cs(stream);
+    GS_TRY(ensure_mm_scratch(A, s));
+    MMArgs a = forward_args(A, d_X, d_Y);
+    a.k = k;
+    a.ldx = ldx;
+    a.ldy = ldy;
+    return dtype == GS_F64 ? launch_mm_wide<double>(a, cols, s) : launch_mm_wide<float>(a, cols, s);
+}
+
+gs_status gs_spmm_adjoint_strided(gs_matrix *A, const void *d_Ybar, UIN ldyb, const void *d_X,
+                                  UIN ldx, void *d_Xbar, UIN ldxb, void *d_vbar, gs_dtype dtype,
+                                  UIN k, UIN cols, gs_stream stream)
+{
+    if (!A || !d_Ybar || !d_Xbar || (d_vbar && !d_X)) return fail(GS_ERR_INVALID, "NULL argument");
+    GS_TRY(check_strided(A, dtype, k, cols));
+    GS_TRY(check_rows("Ybar", d_Ybar, ldyb, cols, dtype));
+    GS_TRY(check_rows("Xbar", d_Xbar, ldxb, k, dtype));
+    if (d_vbar) GS_TRY(check_rows("X", d_X, ldx, cols, dtype));
+    if (!A->adj_ready)
+        return fail(GS_ERR_INVALID, "gs_matrix_prepare_adjoint must run first");
+    if (ldyb == k && ldxb == k && valid_k(k) && aligned32(d_Ybar) && aligned32(d_Xbar) &&
+        (!d_vbar || (ldx == k && aligned32(d_X))))
+        return gs_spmm_adjoint(A, d_Ybar, d_X, d_Xbar, d_vbar, dtype, k, GS_ADJ_DETERMINISTIC,
+                               GS_VALUES_CSR, stream);
+    cudaStream_t s = cs(stream);
+    const bool f64 = dtype == GS_F64;
+    if (d_vbar) {
+        VbarArgs v{};
+        v.nnz = A->nnz;
+        v.k = k;
+        v.ldx = ldx;
+        v.ldy = ldyb;
+        v.row = A->vrow.as<uint32_t>();
+        v.col = A->vcol.as<uint32_t>();
+        v.x = d_X;
+        v.ybar = d_Ybar;
+        v.vbar = d_vbar;
+        GS_TRY((f64 ? launch_vbar_wide<double>(v, cols, s) : launch_vbar_wide<float>(v, cols, s)));
+    }
+    MMArgs a = adjoint_args(A, d_Ybar, d_Xbar);
+    a.k = k;
+    a.ldx = ldyb;
+    a.ldy = ldxb;
+    return f64 ? launch_mm_wide<double>(a, cols, s) : launch_mm_wide<float>(a, cols, s);
 }
 
 }  // extern "C"

@@ -388,6 +388,12 @@ typedef enum { GS_VALUES_CSR = 0, GS_VALUES_SLOTS = 1 } gs_value_order;
 /* Y = A X.  The first call sizes the matrix's multi-RHS scratch (allocates, synchronises). */
 gs_status gs_spmm(gs_matrix *A, const void *d_X, void *d_Y, gs_dtype dtype, UIN k,
                   gs_stream stream);
+/* Y = A X for any k from 1 to 32 and rows of X and Y that are ldx and ldy entries apart, aligned
+ * to their entries only: columns of wider arrays and odd widths as they are.  cols (k <= cols <=
+ * ldx): the columns of each row of X that may be read; those from k on are ignored, but let an odd
+ * k take wide loads. */
+gs_status gs_spmm_strided(gs_matrix *A, const void *d_X, UIN ldx, void *d_Y, UIN ldy,
+                          gs_dtype dtype, UIN k, UIN cols, gs_stream stream);
 /* Builds what the adjoint needs from the CSR structure the matrix was created from (the
  * same d_row / d_col): the map from K1 slots to CSR indices and the K1 layout of A^T with
  * its values.  Once per matrix; allocates and synchronises. */
@@ -412,6 +418,13 @@ gs_status gs_matrix_convert_values(const gs_matrix *A, const void *d_in,
 gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, void *d_Xbar,
                           void *d_vbar, gs_dtype dtype, UIN k, gs_adjoint_mode mode,
                           gs_value_order vbar_order, gs_stream stream);
+
+/* The deterministic adjoint in the same form: Xbar = A^T Ybar for any k from 1 to 32 and any row
+ * strides and, when d_vbar is given, vbar in CSR order (d_X is then required).  cols: the columns
+ * of each row of Ybar and X that may be read. */
+gs_status gs_spmm_adjoint_strided(gs_matrix *A, const void *d_Ybar, UIN ldyb, const void *d_X,
+                                  UIN ldx, void *d_Xbar, UIN ldxb, void *d_vbar, gs_dtype dtype,
+                                  UIN k, UIN cols, gs_stream stream);
 
 /* ---- batched uneven multi-RHS products: Y_i = A_i X_i for many K1 matrices in one
  * persistent launch (no counterpart in the reference).  All matrices share one value type

@@ -1,0 +1,87 @@
+"""Multi-RHS products and the adjoint for any number of right-hand sides and any row strides: every
+column equals the single-RHS K1 product bit for bit (the same sums in the same order), for A and,
+as the adjoint, for the explicit transpose, with rows over several work pieces; the value gradient
+against its definition, |err| <= (k + 1) eps sum |Ybar||X|."""
+import numpy as np
+import pytest
+import torch
+
+from mats import csr_from_lengths
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(seed):
+    rng = np.random.default_rng(seed)
+    lens = rng.integers(0, 30, 1000)
+    lens[7], lens[500] = 700, 300  # cut chunks
+    row, col, val = csr_from_lengths(lens, 900, rng)
+    col = np.where(rng.random(len(col)) < 0.2, 5, col).astype(np.uint32)  # a long column
+    return row, col, val
+
+
+def _transpose(row, col, val, ncols):
+    order = np.argsort(col, kind="stable")
+    rows = np.repeat(np.arange(len(row) - 1), np.diff(row))
+    row_t = np.concatenate([[0], np.cumsum(np.bincount(col, minlength=ncols))]).astype(np.uint32)
+    return row_t, rows[order].astype(np.uint32), val[order]
+
+
+def _operand(rng, n, k, dt, how):
+    """[n, k]: contiguous; columns 3 .. of a wider array; every second row; transposed."""
+    full = torch.from_numpy(rng.standard_normal((2 * n, k + 7))).to(dt).cuda()
+    if how == "tight":
+        return full[:n, :k].contiguous()
+    if how == "columns":
+        return full[:n, 3:3 + k]
+    if how == "rows":
+        return full[::2, :k]
+    return full[:n, :k].t().contiguous().t()
+
+
+@pytest.mark.parametrize("vtype", ["f64", "f32"])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 15, 16, 17, 20, 24, 30, 31, 32, 40])
+@pytest.mark.parametrize("how", ["tight", "columns", "rows", "transposed"])
+def test_any_width(vtype, k, how):
+    from gpu_spmv_b200 import engine as E
+
+    rng = np.random.default_rng(k)
+    row, col, val = _matrix(3)
+    dt = torch.float64 if vtype == "f64" else torch.float32
+    A = E.Matrix(row, col, val, ncols=900, fmt="K1", vtype=vtype, adjoint=True)
+    T = E.Matrix(*_transpose(row, col, val, 900), ncols=1000, fmt="K1", vtype=vtype)
+    X, Yb = _operand(rng, 900, k, dt, how), _operand(rng, 1000, k, dt, how)
+    Y = A.spmm(X)
+    Xbar, vbar = A.adjoint(Yb, X)
+    Xonly, none = A.adjoint(Yb, want_vbar=False)
+    assert none is None and torch.equal(Xbar, Xonly)
+    for c in range(k):
+        assert torch.equal(Y[:, c], A.spmv(X[:, c].contiguous()))
+        assert torch.equal(Xbar[:, c], T.spmv(Yb[:, c].contiguous()))
+    r = np.repeat(np.arange(1000), np.diff(row))
+    y, x = Yb.double().cpu().numpy()[r], X.double().cpu().numpy()[col]
+    want, mag = np.einsum("ek,ek->e", y, x), np.einsum("ek,ek->e", np.abs(y), np.abs(x))
+    eps = 2.0 ** -53 if vtype == "f64" else 2.0 ** -24
+    err = np.abs(vbar.double().cpu().numpy() - want)
+    assert np.all(err <= ((k + 1) * eps + k * 2.0 ** -52) * mag)
+    A.close()
+    T.close()
+
+
+def test_refusals():
+    from gpu_spmv_b200 import _lib as L
+    from gpu_spmv_b200 import engine as E
+
+    row, col, val = _matrix(4)
+    A = E.Matrix(row, col, val, ncols=900, fmt="K1")
+    X, Y = torch.zeros(900, 40, device="cuda").double(), torch.zeros(1000, 40, device="cuda").double()
+    f = L.lib().gs_spmm_strided
+    assert f(A._h, X.data_ptr(), 40, Y.data_ptr(), 40, L.GS_F64, 33, 40, None) == L.GS_ERR_UNSUPPORTED
+    assert f(A._h, X.data_ptr(), 40, Y.data_ptr(), 40, L.GS_F64, 0, 40, None) == L.GS_ERR_UNSUPPORTED
+    assert f(A._h, X.data_ptr(), 4, Y.data_ptr(), 40, L.GS_F64, 5, 5, None) == L.GS_ERR_INVALID
+    assert f(A._h, X.data_ptr() + 4, 40, Y.data_ptr(), 40, L.GS_F64, 5, 5, None) == L.GS_ERR_INVALID
+    assert f(A._h, X.data_ptr(), 40, Y.data_ptr(), 40, L.GS_F32, 5, 5, None) == L.GS_ERR_UNSUPPORTED
+    assert f(A._h, X.data_ptr(), 40, Y.data_ptr(), 40, L.GS_F64, 5, 4, None) == L.GS_ERR_INVALID
+    assert f(A._h, X.data_ptr(), 6, Y.data_ptr(), 40, L.GS_F64, 5, 8, None) == L.GS_ERR_INVALID
+    assert L.lib().gs_spmm(A._h, X.data_ptr(), Y.data_ptr(), L.GS_F64, 5, None) == L.GS_ERR_UNSUPPORTED
+    A.close()
