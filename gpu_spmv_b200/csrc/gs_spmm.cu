@@ -325,6 +325,29 @@ template <class T> gs_status launch_vbar_wide(const VbarArgs &a, uint32_t cols, 
 }
 
 // ------------------------------------------------------------------ layout helpers
+// out[i] = v[src[i]], 0 where src is kNoSrc.  Four neighbours a thread, so that four gathers are in
+// flight where one was (16.8M FP32 values in random order 90 -> 82 us, 60 at the line rate);
+// n4 groups of four, for arrays whose out is 16-byte aligned.
+template <class T>
+__global__ void __launch_bounds__(256) k_gather_vals4(size_t n4, const uint4 *__restrict__ src,
+                                                      const T *__restrict__ v,
+                                                      T *__restrict__ out)
+{
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    const uint4 q = __ldcs(src + i);
+    const uint32_t s[4] = {q.x, q.y, q.z, q.w};
+    T w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = s[k] == kNoSrc ? T(0) : __ldg(v + s[k]);
+    if constexpr (sizeof(T) == 4) {
+        __stcs(reinterpret_cast<float4 *>(out) + i, make_float4(w[0], w[1], w[2], w[3]));
+    } else {
+        __stcs(reinterpret_cast<double2 *>(out) + 2 * i, make_double2(w[0], w[1]));
+        __stcs(reinterpret_cast<double2 *>(out) + 2 * i + 1, make_double2(w[2], w[3]));
+    }
+}
+
 template <class T>
 __global__ void k_gather_vals(size_t nslots, const uint32_t *src, const T *v, T *out)
 {
@@ -439,6 +462,18 @@ __global__ void k_t_meta(uint32_t m, const uint32_t *cptr, const uint32_t *tperm
 
 unsigned blocks_of(size_t n) { return (unsigned)((n + 255) / 256); }
 
+template <class T>
+gs_status gather_vals(size_t n, const DevBuf &src, const T *v, T *out, cudaStream_t s)
+{
+    if (!n) return GS_OK;
+    if (n % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0)
+        k_gather_vals4<T><<<blocks_of(n / 4), 256, 0, s>>>(n / 4, src.as<uint4>(), v, out);
+    else
+        k_gather_vals<T><<<148u * 16u, 256, 0, s>>>(n, src.as<uint32_t>(), v, out);
+    GS_CHECK_LAUNCH();
+    return GS_OK;
+}
+
 template <class T, bool ADJ>
 gs_status launch_mm(const MMArgs &a, uint32_t k, cudaStream_t s)
 {
@@ -519,15 +554,14 @@ k1fill::Args forward_fill(const gs_matrix *A)
 template <class T>
 gs_status refresh_values(gs_matrix *A, const T *v, gs_value_order order, cudaStream_t s)
 {
-    const unsigned gb = 148u * 16u;
     if (order == GS_VALUES_CSR) {
         k1fill::Args f = forward_fill(A);
         f.val = v;
         f.oval = A->val.p;
         GS_TRY((k1fill::fill<T, T, false>(f, T(0), s)));
-        k_gather_vals<T><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), v, A->tval.as<T>());
+        GS_TRY(gather_vals<T>(A->tlenVC, A->tsrc, v, A->tval.as<T>(), s));
     } else {
-        k_gather_vals<T><<<gb, 256, 0, s>>>(A->lenVC, A->ftslot.as<uint32_t>(), v, A->val.as<T>());
+        GS_TRY(gather_vals<T>(A->lenVC, A->ftslot, v, A->val.as<T>(), s));
         GS_CUDA(cudaMemcpyAsync(A->tval.p, v, (size_t)A->tlenVC * sizeof(T),
                                 cudaMemcpyDeviceToDevice, s));
     }
@@ -784,14 +818,10 @@ gs_status gs_matrix_convert_values(const gs_matrix *A, const void *d_in, gs_valu
     const unsigned gb = 148u * 16u;
     const bool f64 = dtype == GS_F64;
     if (in_order == GS_VALUES_CSR) {  // slots[t] = csr[tsrc[t]], padding 0
-        if (f64)
-            k_gather_vals<double><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                     static_cast<const double *>(d_in),
-                                                     static_cast<double *>(d_out));
-        else
-            k_gather_vals<float><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                    static_cast<const float *>(d_in),
-                                                    static_cast<float *>(d_out));
+        return f64 ? gather_vals<double>(A->tlenVC, A->tsrc, static_cast<const double *>(d_in),
+                                         static_cast<double *>(d_out), s)
+                   : gather_vals<float>(A->tlenVC, A->tsrc, static_cast<const float *>(d_in),
+                                        static_cast<float *>(d_out), s);
     } else if (in_order == GS_VALUES_SLOTS) {  // csr[tsrc[t]] = slots[t]
         if (f64)
             k_scatter_vals<double><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
@@ -824,7 +854,6 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         return fail(GS_ERR_INVALID, "Ybar, X and Xbar must be 32-byte aligned");
     cudaStream_t s = cs(stream);
     const bool f64 = A->p.vtype == GS_F64;
-    const unsigned gb = 148u * 16u;
     if (mode != GS_ADJ_ATOMIC && mode != GS_ADJ_DETERMINISTIC)
         return fail(GS_ERR_INVALID, "unknown adjoint mode %d", (int)mode);
     // a value gradient in CSR order has its own kernel; one in slot order comes with Xbar
@@ -860,15 +889,10 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         a.vbar = via_slots ? A->vslots.p : nullptr;
         GS_TRY((f64 ? launch_atomic<double>(a, k, s) : launch_atomic<float>(a, k, s)));
         if (via_slots) {
-            const size_t n_out = A->tlenVC;
-            const uint32_t *map = A->t2f.as<uint32_t>();
-            if (f64)
-                k_gather_vals<double><<<gb, 256, 0, s>>>(n_out, map, A->vslots.as<double>(),
-                                                         static_cast<double *>(d_vbar));
-            else
-                k_gather_vals<float><<<gb, 256, 0, s>>>(n_out, map, A->vslots.as<float>(),
-                                                        static_cast<float *>(d_vbar));
-            GS_CHECK_LAUNCH();
+            GS_TRY((f64 ? gather_vals<double>(A->tlenVC, A->t2f, A->vslots.as<double>(),
+                                              static_cast<double *>(d_vbar), s)
+                        : gather_vals<float>(A->tlenVC, A->t2f, A->vslots.as<float>(),
+                                             static_cast<float *>(d_vbar), s)));
         }
         return GS_OK;
     }
