@@ -378,36 +378,35 @@ __global__ void k_row_places(uint32_t n, const uint32_t *row, const uint32_t *pe
     inv[perm[g]] = g;
 }
 
-// csr2f[e] = forward slot of CSR element e (its row at sorted place inv[row])
+// place[e] = row and forward slot of CSR element e (its row at sorted place inv[row])
 __global__ void k_forward_slots(uint32_t nnz, const uint32_t *__restrict__ vrow,
                                 const uint32_t *__restrict__ rowptr,
                                 const uint32_t *__restrict__ inv,
-                                const uint32_t *__restrict__ chp, uint32_t *__restrict__ csr2f)
+                                const uint32_t *__restrict__ chp, uint2 *__restrict__ place)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nnz) return;
     const uint32_t r = vrow[e], g = __ldg(inv + r);
-    csr2f[e] = __ldg(chp + (g >> 5)) + 32u * (e - __ldg(rowptr + r)) + (g & 31u);
+    place[e] = make_uint2(r, __ldg(chp + (g >> 5)) + 32u * (e - __ldg(rowptr + r)) + (g & 31u));
 }
 
 // The adjoint layout's slots, from the CSR index tsrc of each: the row and the stored value of the
 // element, its forward slot and the way back from there; padding slots 0, 0, none
 template <class T>
 __global__ void k_t_maps(uint32_t nslots, const uint32_t *__restrict__ tsrc,
-                         const uint32_t *__restrict__ vrow, const uint32_t *__restrict__ csr2f,
-                         const T *__restrict__ val, uint32_t *__restrict__ trow,
-                         T *__restrict__ tval, uint32_t *__restrict__ t2f,
-                         uint32_t *__restrict__ ftslot)
+                         const uint2 *__restrict__ place, const T *__restrict__ val,
+                         uint32_t *__restrict__ trow, T *__restrict__ tval,
+                         uint32_t *__restrict__ t2f, uint32_t *__restrict__ ftslot)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nslots) return;
     const uint32_t e = tsrc[i];
     const bool in = e != kNoSrc;
-    const uint32_t f = in ? __ldg(csr2f + e) : kNoSrc;
-    trow[i] = in ? __ldg(vrow + e) : 0u;
-    t2f[i] = f;
-    tval[i] = in ? __ldg(val + f) : T(0);
-    if (in) ftslot[f] = i;
+    const uint2 at = in ? __ldg(place + e) : make_uint2(0u, kNoSrc);
+    trow[i] = at.x;
+    t2f[i] = at.y;
+    tval[i] = in ? __ldg(val + at.y) : T(0);
+    if (in) ftslot[at.y] = i;
 }
 
 // rowidx[e] = row of CSR element e: a warp per 32 rows, in element order (coalesced writes; the
@@ -685,11 +684,11 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     GS_TRY(A->vrow.alloc((size_t)nnz * 4, s));
     GS_TRY(A->vcol.alloc((size_t)nnz * 4, s));
     // CSC order of the elements: stable sort of CSR indices by ascending column
-    StreamBuf ccount(s), csc(s), csorted(s), cptr(s), csr2f(s), inv(s);
+    StreamBuf ccount(s), csc(s), csorted(s), cptr(s), place(s), inv(s);
     GS_TRY(ccount.alloc((size_t)m * 4));
     GS_TRY(csc.alloc((size_t)nnz * 4));
     GS_TRY(csorted.alloc((size_t)nnz * 4));
-    GS_TRY(csr2f.alloc((size_t)nnz * 4));
+    GS_TRY(place.alloc((size_t)nnz * 8));
     GS_TRY(inv.alloc((size_t)n * 4));
     if (n) {
         k_expand_rows<<<blocks_of(n), 256, 0, s>>>(n, d_row, A->vrow.as<uint32_t>());
@@ -701,7 +700,7 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
         GS_CUDA(cudaMemcpyAsync(A->vcol.p, d_col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
         k_forward_slots<<<blocks_of(nnz), 256, 0, s>>>(
             nnz, A->vrow.as<uint32_t>(), d_row, inv.as<uint32_t>(),
-            A->chp.as<uint32_t>(), csr2f.as<uint32_t>());
+            A->chp.as<uint32_t>(), place.as<uint2>());
         GS_CHECK_LAUNCH();
         GS_TRY(stable_sort_asc(d_col, nnz, m ? m - 1 : 0, csc.as<uint32_t>(),
                                csorted.as<uint32_t>(), s));
@@ -769,14 +768,14 @@ gs_status gs_matrix_prepare_adjoint(gs_matrix *A, const UIN *d_row, const UIN *d
     if (A->tlenVC) {
         if (A->p.vtype == GS_F64)
             k_t_maps<double><<<blocks_of(A->tlenVC), 256, 0, s>>>(
-                A->tlenVC, A->tsrc.as<uint32_t>(), A->vrow.as<uint32_t>(), csr2f.as<uint32_t>(),
-                A->val.as<double>(), A->trow.as<uint32_t>(), A->tval.as<double>(),
-                A->t2f.as<uint32_t>(), A->ftslot.as<uint32_t>());
+                A->tlenVC, A->tsrc.as<uint32_t>(), place.as<uint2>(), A->val.as<double>(),
+                A->trow.as<uint32_t>(), A->tval.as<double>(), A->t2f.as<uint32_t>(),
+                A->ftslot.as<uint32_t>());
         else
             k_t_maps<float><<<blocks_of(A->tlenVC), 256, 0, s>>>(
-                A->tlenVC, A->tsrc.as<uint32_t>(), A->vrow.as<uint32_t>(), csr2f.as<uint32_t>(),
-                A->val.as<float>(), A->trow.as<uint32_t>(), A->tval.as<float>(),
-                A->t2f.as<uint32_t>(), A->ftslot.as<uint32_t>());
+                A->tlenVC, A->tsrc.as<uint32_t>(), place.as<uint2>(), A->val.as<float>(),
+                A->trow.as<uint32_t>(), A->tval.as<float>(), A->t2f.as<uint32_t>(),
+                A->ftslot.as<uint32_t>());
         GS_CHECK_LAUNCH();
     }
     GS_TRY(A->vslots.alloc((size_t)max(A->lenVC, A->tlenVC) * vsz + 8, s));
