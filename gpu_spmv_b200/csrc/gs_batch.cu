@@ -23,6 +23,7 @@
 //
 // No counterpart in the reference, which runs one matrix and one right-hand side per call.
 #include <algorithm>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -81,7 +82,6 @@ struct gs_batch {
     int blocks = 0;
     double flops = 0;
     bool operands = false;
-    cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 
@@ -95,7 +95,6 @@ struct gs_batch {
     ~gs_batch()
     {
         drop_graph();
-        if (cap) cudaStreamDestroy(cap);
     }
 };
 
@@ -792,6 +791,46 @@ gs_status launch(gs_batch *B, cudaStream_t s)
 }  // namespace
 }  // namespace gs
 
+namespace {
+// A stream to capture on, held for one capture and kept for the next (making one takes 100 to
+// 400 us; there are as many as captures have ever run at once on the device).
+struct CaptureStream {
+    CaptureStream()
+    {
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) dev = -1;
+        std::lock_guard<std::mutex> lock(mutex);
+        if (dev >= 0 && !idle[dev].empty()) {
+            s = idle[dev].back();
+            idle[dev].pop_back();
+        }
+    }
+    ~CaptureStream()
+    {
+        if (!s) return;
+        if (dev < 0) {
+            cudaStreamDestroy(s);
+            return;
+        }
+        std::lock_guard<std::mutex> lock(mutex);
+        idle[dev].push_back(s);
+    }
+    gs_status ready()
+    {
+        if (!s) GS_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        return GS_OK;
+    }
+    cudaStream_t s = nullptr;
+
+private:
+    static constexpr int kDevices = 64;
+    static std::mutex mutex;
+    static std::vector<cudaStream_t> idle[kDevices];
+    int dev = -1;
+};
+std::mutex CaptureStream::mutex;
+std::vector<cudaStream_t> CaptureStream::idle[CaptureStream::kDevices];
+}  // namespace
+
 using namespace gs;
 
 extern "C" {
@@ -1035,11 +1074,12 @@ gs_status gs_batch_run_graph(gs_batch *B, gs_stream stream)
     if (!B) return fail(GS_ERR_INVALID, "NULL argument");
     if (!B->operands) return fail(GS_ERR_INVALID, "gs_batch_set_operands must run first");
     if (!B->exec) {
-        if (!B->cap) GS_CUDA(cudaStreamCreateWithFlags(&B->cap, cudaStreamNonBlocking));
-        GS_CUDA(cudaStreamBeginCapture(B->cap, cudaStreamCaptureModeThreadLocal));
-        const gs_status st = launch(B, B->cap);
+        CaptureStream cap;
+        GS_TRY(cap.ready());
+        GS_CUDA(cudaStreamBeginCapture(cap.s, cudaStreamCaptureModeThreadLocal));
+        const gs_status st = launch(B, cap.s);
         cudaGraph_t g = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(B->cap, &g);
+        const cudaError_t e = cudaStreamEndCapture(cap.s, &g);
         if (st) {
             if (g) cudaGraphDestroy(g);
             return st;
