@@ -129,22 +129,30 @@ class Matrix:
             c0 += w
         return out
 
+    @classmethod
+    def _whole(cls, T: torch.Tensor, rows: int, k: int, dt, device) -> bool:
+        """Whether the kernels of the widths 1, 2, 4, ..., 32 read T as it lies: then no view or
+        copy of it is prepared, which costs the host more than a launch (64 x 64 grid, FP32,
+        k = 8: 10.6 us a call, 17.4 through views and the strided entry point)."""
+        return (k in cls.MM_K and T.dtype == dt and T.device == device and T.shape[1] == k
+                and T.shape[0] >= rows and T.is_contiguous() and T.data_ptr() % 32 == 0)
+
     @staticmethod
-    def _rows(T: torch.Tensor, dt, w: int):
+    def _rows(T: torch.Tensor, rows: int, w: int, dt, device):
         """(T, distance of its rows, readable columns from its block's first on) for a block of w
-        columns of T [n, k]: T itself where its columns lie side by side; a copy in rows of a
+        columns of T [rows, k]: T itself where its columns lie side by side; a copy in rows of a
         multiple of 4 columns for odd and other widths that the kernels could read only in slices
-        below 16 bytes (k = 5, FP64, 200,000 rows: 7 us for the copy, 68 -> 46 for the product)."""
-        T = T.to(dt)
-        n, k = T.shape
-        if k > 1 and T.stride(1) != 1 or n > 1 and T.stride(0) < k or T.stride(0) >= 2 ** 32:
+        below 16 bytes (k = 5, FP64, 200,000 rows: 7 us for the copy, 68 -> 46 for the product).
+        The kernels know no row count of T: expand() refuses every other one."""
+        T = T.to(device=device, dtype=dt).expand(rows, w)
+        if w > 1 and T.stride(1) != 1 or rows > 1 and T.stride(0) < w or T.stride(0) >= 2 ** 32:
             T = T.contiguous()
         if w > 2 and (w * T.element_size() % 16 or T.stride(0) * T.element_size() % 16):
             kp = (w + 3) // 4 * 4
-            P = torch.empty(n, kp, dtype=dt, device=T.device)
+            P = torch.empty(rows, kp, dtype=dt, device=device)
             P[:, :w] = T
             return P, kp, kp
-        return T, max(k, T.stride(0)), w
+        return T, max(w, T.stride(0)), w
 
     def spmm(self, X: torch.Tensor, stream=None) -> torch.Tensor:
         """Y = A X for X of shape [ncols, k] (any k; run in blocks of up to 32 columns)."""
@@ -155,8 +163,12 @@ class Matrix:
             raise TypeError(f"X must be a CUDA {dt} tensor with {self.ncols} rows")
         k = X.shape[1]
         Y = torch.empty(self.nrows, k, dtype=dt, device=X.device)
+        if self._whole(X, self.ncols, k, dt, X.device):
+            L.check(L.lib().gs_spmm(self._h, X.data_ptr(), Y.data_ptr(), self.vtype, k,
+                                    stream_handle(stream)), "gs_spmm")
+            return Y
         for c0, w, _ in self._blocks(k):
-            Xb, ldx, cols = self._rows(X[:, c0:c0 + w], dt, w)
+            Xb, ldx, cols = self._rows(X[:, c0:c0 + w], self.ncols, w, dt, X.device)
             L.check(L.lib().gs_spmm_strided(self._h, Xb.data_ptr(), ldx, Y[:, c0:].data_ptr(), k,
                                             self.vtype, w, cols, stream_handle(stream)),
                     "gs_spmm_strided")
@@ -220,10 +232,14 @@ class Matrix:
         new = torch.empty if blocks else torch.zeros
         vbar = new(nv, dtype=dt, device=Ybar.device) if want_vbar else None
         part = torch.empty_like(vbar) if want_vbar and len(blocks) > 1 else None
-        if m == L.GS_ADJ_DETERMINISTIC and (order == "csr" or not want_vbar):
+        dev = Ybar.device
+        whole = (self._whole(Ybar, self.nrows, k, dt, dev)
+                 and (not want_vbar or self._whole(X, self.ncols, k, dt, dev)))
+        if not whole and m == L.GS_ADJ_DETERMINISTIC and (order == "csr" or not want_vbar):
             for i, (c0, w, _) in enumerate(blocks):
-                Yb, ldy, cols = self._rows(Ybar[:, c0:c0 + w], dt, w)
-                Xin, ldx, xcols = self._rows(X[:, c0:c0 + w], dt, w) if want_vbar else (None, k, w)
+                Yb, ldy, cols = self._rows(Ybar[:, c0:c0 + w], self.nrows, w, dt, dev)
+                Xin, ldx, xcols = (self._rows(X[:, c0:c0 + w], self.ncols, w, dt, dev)
+                                   if want_vbar else (None, k, w))
                 v = None if not want_vbar else vbar if i == 0 else part
                 L.check(L.lib().gs_spmm_adjoint_strided(
                     self._h, Yb.data_ptr(), ldy, Xin.data_ptr() if want_vbar else None, ldx,

@@ -85,3 +85,30 @@ def test_refusals():
     assert f(A._h, X.data_ptr(), 6, Y.data_ptr(), 40, L.GS_F64, 5, 8, None) == L.GS_ERR_INVALID
     assert L.lib().gs_spmm(A._h, X.data_ptr(), Y.data_ptr(), L.GS_F64, 5, None) == L.GS_ERR_UNSUPPORTED
     A.close()
+
+
+@pytest.mark.parametrize("k", [3, 4, 5, 8, 40])
+def test_adjoint_operand_forms(k):
+    """Row counts that fit neither the matrix nor a broadcast are refused on the host; a single
+    column or row is broadcast and a host tensor moved where the product copies its operands."""
+    from gpu_spmv_b200 import engine as E
+
+    rng = np.random.default_rng(k)
+    row, col, val = _matrix(5)
+    A = E.Matrix(row, col, val, ncols=900, fmt="K1", adjoint=True)
+    X = _operand(rng, 900, k, torch.float64, "columns")
+    Yb = _operand(rng, 1000, k, torch.float64, "columns")
+    Xbar, vbar = A.adjoint(Yb, X)
+    for bad_y, bad_x in [(Yb[:-1], X), (Yb, X[:-1]), (torch.cat([Yb, Yb[:1]]), X[:-1])]:
+        with pytest.raises(RuntimeError):
+            A.adjoint(bad_y, bad_x)
+        with pytest.raises(RuntimeError):
+            A.adjoint(bad_y.contiguous(), bad_x.contiguous())
+    same = A.adjoint(Yb, X.cpu())
+    assert torch.equal(same[0], Xbar) and torch.equal(same[1], vbar)
+    assert torch.equal(A.adjoint(Yb.contiguous(), X.float())[1],
+                       A.adjoint(Yb, X.float().double())[1])
+    assert torch.equal(A.adjoint(Yb, X[:1])[1], A.adjoint(Yb, X[:1].expand(900, k).contiguous())[1])
+    with pytest.raises(TypeError):
+        A.spmm(X[:-1])
+    A.close()
