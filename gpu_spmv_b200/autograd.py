@@ -10,8 +10,8 @@ right-hand sides X are differentiable inputs:
 
 Values may also live in the operator's "slots" order (op.slot_values(); the adjoint
 layout's slot order, padding slots included and kept at zero gradient): there the
-deterministic adjoint writes vbar in place instead of scattering it to CSR order, which is
-the fast layout for training the values.
+deterministic adjoint forms vbar beside X's gradient, which is the fast layout for training
+the values; in CSR order vbar is a pass of its own over the elements.
 
 No kernel here is PyTorch's: the forward runs the K1 multi-RHS kernel and the backward the
 transposed-K1 kernel (or the atomic one), both in libgpuspmv_b200.so.
@@ -33,11 +33,14 @@ class SparseOperator:
         self.dtype = E.TORCH_DTYPES[self.mat.vtype]
 
     def ensure_values(self, values: torch.Tensor, order: str = "csr"):
-        """Store `values` unless they are already the stored ones (same tensor, same version)."""
-        key = (values.data_ptr(), values._version, order)
-        if self.mat._values_key != key:
+        """Store `values` unless they are already the stored ones: the same entries of the same
+        storage, at the same version, in the same order.  The operator keeps that storage alive,
+        so that no later tensor can take its place at the same address."""
+        key = (values.untyped_storage()._cdata, values.data_ptr(), values.stride(), values.dtype,
+               values._version, order)
+        if self.mat._stored is None or self.mat._stored[0] != key:
             self.mat.set_values(values, order)
-            self.mat._values_key = key
+            self.mat._stored = (key, values.detach())
 
     def slot_values(self, values_csr: torch.Tensor) -> torch.Tensor:
         """CSR-order values -> a new tensor in the operator's slot order."""

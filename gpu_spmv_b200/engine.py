@@ -76,7 +76,7 @@ class Matrix:
         self._h = h
         self.device = dev
         self.info = self._info()
-        self._values_key = None
+        self._stored = None  # SparseOperator: what the stored values were taken from
         if adjoint:
             with torch.cuda.device(dev):
                 L.check(L.lib().gs_matrix_prepare_adjoint(h, row_t.data_ptr(), col_t.data_ptr(),
@@ -193,10 +193,10 @@ class Matrix:
         if values.dtype != dt or not values.is_cuda or values.numel() != self._order_len(order):
             raise TypeError(f"values must be {self._order_len(order)} CUDA {dt} entries")
         v = values.contiguous()
+        self._stored = None
         L.check(L.lib().gs_matrix_set_values(self._h, v.data_ptr(), self.vtype,
                                              self.ORDERS[order], stream_handle(stream)),
                 "gs_matrix_set_values")
-        self._values_key = (v.data_ptr(), getattr(values, "_version", None), order)
 
     def convert_values(self, values: torch.Tensor, to: str, stream=None) -> torch.Tensor:
         """The same values in the other order ("csr" <-> "slots")."""
@@ -312,6 +312,7 @@ class Matrix:
         return out
 
     def close(self):
+        self._stored = None
         if self._h:
             L.lib().gs_matrix_destroy(self._h)
             self._h = None
