@@ -323,6 +323,9 @@ gs_status gs_csr_spmv_f64(UIN nrows, UIN ncols, UIN nnz, const UIN *d_row, const
     if ((reinterpret_cast<uintptr_t>(d_val) & 15u) || (reinterpret_cast<uintptr_t>(d_col) & 15u))
         return gs::fail(GS_ERR_INVALID, "val and col must be 16-byte aligned");
     cudaStream_t s = gs::cs(stream);
+    // few long rows: 100 rows of 100,000 elements 0.8 ms with their plan, 2.9 ms without
+    if (!gs::csr_enough_rows(nrows, nnz, GS_F64))
+        return gs::csr_rows_product(nrows, nnz, d_row, d_col, d_val, d_x, d_y, s);
     gs::CsrArgs a{};
     a.n = nrows;
     a.nnz = nnz;

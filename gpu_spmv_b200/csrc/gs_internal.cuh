@@ -308,6 +308,12 @@ struct CsrArgs {
 };
 gs_status launch_csr(const CsrArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype ytype,
                      cudaStream_t s);
+// Whether n rows (> 0) of nnz elements are enough to keep that kernel's warps busy.
+bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype);
+// y = A x from CSR arrays, FP64, by the row-stream kernel on a plan made for the call
+// (synchronises).
+gs_status csr_rows_product(uint32_t n, uint32_t nnz, const uint32_t *d_row, const uint32_t *d_col,
+                           const double *d_val, const double *d_x, double *d_y, cudaStream_t s);
 
 // Slot of step j of lane `lane` in the K1 chunk that starts at slot cbase and has nmc
 // steps.  The reference's order is cbase + 32 j + lane (a warp's loads of one step are

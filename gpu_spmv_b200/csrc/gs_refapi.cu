@@ -516,7 +516,8 @@ str_res test_gcsr(const UIN cudaBlockSize, const str_matCSR m, const FPT *vec, c
     if (upload_csr(m, row, col, val) || h2d(x, vec, m.nrows) || y.alloc((size_t)m.nrows * 8) ||
         gs::random_columns(row.as<UIN>(), col.as<UIN>(), m.nrows, &rnd, 0, &even))
         return error_res("gcsr", gs_last_error());
-    if (!rnd && even && (double)m.nnz >= 2.5 * m.nrows) {
+    if (!rnd && even && (double)m.nnz >= 2.5 * m.nrows &&
+        gs::csr_enough_rows(m.nrows, m.nnz, GS_F64)) {
         gs::CsrArgs c{};
         c.n = m.nrows;
         c.nnz = m.nnz;

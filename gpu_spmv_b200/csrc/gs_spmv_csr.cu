@@ -24,9 +24,10 @@
 // Random columns stay on the row-stream kernel (power-law 4.2M rows: 326 us against 410 for
 // products staged in position order), and so do rows of very uneven length, which leave lanes
 // idle here (lognormal lengths of sigma 1.2, local columns, 24.5M elements: FP64 107 against 120
-// us, BF16 60 against 133): gs_matrix_create samples both (random_columns).  A product straight
-// from CSR arrays always runs here, without the sample, whose read-back costs more than it could
-// save: 27-point 101^3 180 us with the row-stream kernel and its plan's kernels, 79 us here.
+// us, BF16 60 against 133): gs_matrix_create samples both (random_columns).  Few long rows stay
+// there too (csr_enough_rows).  A product straight from CSR arrays runs here without the sample,
+// whose read-back costs more than it could save: 27-point 101^3 180 us with the row-stream kernel
+// and its plan's kernels, 79 us here.
 #include <cmath>
 
 #include "gs_internal.cuh"
@@ -218,29 +219,43 @@ gs_status launch_csr_g(const CsrArgs &a, cudaStream_t s)
     return GS_OK;
 }
 
-// The window CAP and the rows G per warp, from the average row length with 5 % to spare: two or
+// The window `cap` and the rows G per warp, from the average row length with 5 % to spare: two or
 // four rows per lane when they fit and leave an SM 32 warps (Laplacian 2048^2 67 -> 58.5 us, FP32
-// 59.5 -> 46), else 32 rows in the smallest window that holds them (256 positions instead of 480
+// 59.5 -> 46), else 32 rows in the smallest window that holds them (288 positions instead of 480
 // for the Laplacian 2048^2: 72 -> 67 us, more warps per SM; BF16 27-point with 1024 instead of
-// 512: 80 -> 68 us), else fewer rows in the largest, which is 5.8 KB of FP64 values and columns
+// 480: 80 -> 68 us), else fewer rows in the largest, which is 5.8 KB of FP64 values and columns
 // (27-point 160^3 with 256, 480, 640, 920 positions: 260, 229, 253, 224 us; 101^3 with its
 // launch and synchronisation 85, 79, 86, 79).
+struct CsrShape {
+    int cap, rows;
+};
+
+CsrShape csr_shape(uint32_t n, uint32_t nnz, bool f64)
+{
+    const int big = f64 ? 480 : 1024;
+    const double avg = (double)nnz / n;
+    auto fits = [&](int rows, int cap) { return avg * rows <= (cap - 8) / 1.05; };
+    if (fits(64, 480) && n / 64 >= 148u * 32u)
+        return {480, fits(128, 480) && n / 128 >= 148u * 32u ? 128 : 64};
+    if (fits(32, 288)) return {288, 32};
+    if (fits(32, 480)) return {480, 32};
+    for (int rows = 32; rows > 4; rows /= 2)
+        if (fits(rows, big)) return {big, rows};
+    return {big, 4};
+}
+
 template <class VT, class IT, bool PAD>
 gs_status launch_csr_t(const CsrArgs &a, cudaStream_t s)
 {
     constexpr int BIG = sizeof(VT) == 8 ? 480 : 1024;
-    const double avg = (double)a.nnz / a.n;
-    auto fits = [&](int rows, int cap) { return avg * rows <= (cap - 8) / 1.05; };
-    if (fits(64, 480) && a.n / 64 >= 148u * 32u) {
-        if (fits(128, 480) && a.n / 128 >= 148u * 32u)
-            return launch_csr_g<VT, IT, 480, 128, PAD>(a, s);
-        return launch_csr_g<VT, IT, 480, 64, PAD>(a, s);
-    }
-    if (fits(32, 288)) return launch_csr_g<VT, IT, 288, 32, PAD>(a, s);
-    if (fits(32, 480)) return launch_csr_g<VT, IT, 480, 32, PAD>(a, s);
-    if (fits(32, BIG)) return launch_csr_g<VT, IT, BIG, 32, PAD>(a, s);
-    if (fits(16, BIG)) return launch_csr_g<VT, IT, BIG, 16, PAD>(a, s);
-    if (fits(8, BIG)) return launch_csr_g<VT, IT, BIG, 8, PAD>(a, s);
+    const CsrShape c = csr_shape(a.n, a.nnz, sizeof(VT) == 8);
+    if (c.cap == 288) return launch_csr_g<VT, IT, 288, 32, PAD>(a, s);
+    if (c.rows == 128) return launch_csr_g<VT, IT, 480, 128, PAD>(a, s);
+    if (c.rows == 64) return launch_csr_g<VT, IT, 480, 64, PAD>(a, s);
+    if (c.rows == 32 && c.cap == 480) return launch_csr_g<VT, IT, 480, 32, PAD>(a, s);
+    if (c.rows == 32) return launch_csr_g<VT, IT, BIG, 32, PAD>(a, s);
+    if (c.rows == 16) return launch_csr_g<VT, IT, BIG, 16, PAD>(a, s);
+    if (c.rows == 8) return launch_csr_g<VT, IT, BIG, 8, PAD>(a, s);
     return launch_csr_g<VT, IT, BIG, 4, PAD>(a, s);
 }
 
@@ -254,6 +269,22 @@ template <class VT, class IT> gs_status launch_csr_v(const CsrArgs &a, cudaStrea
 }
 
 }  // namespace
+
+// A warp walks its four rows one after the other where they do not fit a window together (112
+// elements on average for FP64, 241 for the reduced types), and the row-stream kernel cuts the
+// stream into equal ranges whatever the rows: few rows of that length leave most of the chip idle
+// here.  us per product, row-stream -> this kernel, FP64: rows of 200 elements, 1,000 / 3,000 /
+// 6,000 / 10,000 of them 4.6 -> 7.8, 5.7 -> 7.9, 8.0 -> 8.5, 12.1 -> 9.5; of 300 6.0 -> 8.2, 7.9 ->
+// 8.4, 12.8 -> 8.9, 17.5 -> 11.2; of 1,000 9.7 -> 19, 18 -> 25, 29 -> 34, 44 -> 48 (20,000: 81 -> 78);
+// 30 rows of 100,000 534 -> 2519.  FP32: 300 5.4 -> 6.9, 6.2 -> 6.9, 8.9 -> 7.2, 13 -> 8.1.  So rows up
+// to a window long from 6,000 of them on, longer ones from 20,000.
+bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype)
+{
+    const CsrShape c = csr_shape(n, nnz, vtype == GS_F64);
+    const double avg = (double)nnz / n;
+    if (avg * c.rows <= (c.cap - 8) / 1.05) return true;
+    return n >= (avg <= c.cap ? 6000u : 20000u);
+}
 
 gs_status launch_csr(const CsrArgs &a0, gs_dtype vtype, gs_itype itype, gs_dtype ytype,
                      cudaStream_t s)

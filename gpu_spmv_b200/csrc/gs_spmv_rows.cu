@@ -1916,6 +1916,24 @@ gs_status launch_rows(const RowsArgs &a0, gs_dtype vtype, gs_itype itype, gs_dty
                 (int)itype);
 }
 
+gs_status csr_rows_product(uint32_t n, uint32_t nnz, const uint32_t *d_row, const uint32_t *d_col,
+                           const double *d_val, const double *d_x, double *d_y, cudaStream_t s)
+{
+    bool random = false;
+    if ((double)nnz >= 8.0 * n) GS_TRY(random_columns(d_row, d_col, n, &random, s));
+    RowsPlan P;
+    GS_TRY(build_rows_plan(d_row, nullptr, n, direct_lane_positions(n, nnz, random), P, s));
+    RowsArgs a = rows_args(P);
+    a.val = d_val;
+    a.col = d_col;
+    a.x = d_x;
+    a.y = d_y;
+    a.nslots = nnz;
+    GS_TRY(launch_rows(a, GS_F64, GS_IDX_U32, GS_F64, 0, false, false, false, s));
+    GS_CUDA(cudaStreamSynchronize(s));  // the plan's buffers are released on return
+    return GS_OK;
+}
+
 gs_status launch_tiles(const RowsArgs &a, uint32_t thw, bool baked, cudaStream_t s)
 {
     switch (thw) {

@@ -1,0 +1,111 @@
+"""Which kernel the CSR products run on, seen from their sums.
+
+FP64: every row is made of pairs (a, -fl(a x_j)) in neighbouring columns with x = (x_j, 1): the
+row-stream kernel rounds each product and adds a pair within a lane, so y is 0 to the last bit; the
+CSR kernel fuses multiply and add, so some rows keep a rounding error.  FP32 / BF16 with FP32 sums
+(rows of (2^30, 1, -2^30, 0) with x = 1): the row-stream kernel loses the 1, the CSR kernel sums in
+FP64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROWS, CSR = "row-stream", "csr"
+
+
+def _structure(lens, ncols=None):
+    """Rows of consecutive columns from an even one on (lens: multiples of 4), along the diagonal."""
+    l = torch.as_tensor(lens, dtype=torch.int64).cuda()
+    n = l.numel()
+    m = ncols or max(n, int(l.max()) + 2)
+    row = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    row[1:] = torch.cumsum(l, 0)
+    r = torch.repeat_interleave(torch.arange(n, device="cuda"), l)
+    e = torch.arange(int(row[-1]), device="cuda") - row[r]
+    first = torch.arange(n, device="cuda") * m // n
+    first = torch.minimum(first, m - l) // 2 * 2
+    return row.int(), (first[r] + e), e, m
+
+
+def _pairs(lens, ncols=None):
+    row, col, e, m = _structure(lens, ncols)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.rand(m, dtype=torch.float64, device="cuda", generator=g)
+    x[1::2] = 1.0
+    val = torch.randn(col.numel(), dtype=torch.float64, device="cuda", generator=g)
+    odd = e % 2 == 1
+    val[odd] = -(val[~odd] * x[col[~odd]])
+    return row, col.int(), val, x
+
+
+def kernel_f64(y):
+    return ROWS if not y.any() else CSR
+
+
+def product(lens, fmt=dict(fmt="CSR")):
+    from gpu_spmv_b200 import engine as E
+
+    row, col, val, x = _pairs(lens)
+    A = E.Matrix(row, col, val, ncols=x.numel(), **fmt)
+    y = A.spmv(x)
+    A.close()
+    return kernel_f64(y)
+
+
+def arrays(lens):
+    from gpu_spmv_b200 import engine as E
+
+    return kernel_f64(E.csr_spmv_f64(*_pairs(lens)))
+
+
+def dropin(lens):
+    from gpu_spmv_b200 import _lib as L
+    from gpu_spmv_b200 import refapi as R
+
+    row, col, val, x = (t.cpu().numpy() for t in _pairs(lens, len(lens)))
+    h = R.csr_struct(row.view(np.uint32), col.view(np.uint32), val)
+    zero = np.zeros(len(lens))
+    old = L.lib().gs_get_num_ite()
+    L.lib().gs_set_num_ite(2)
+    res = L.lib().test_gcsr(256, h.s, R.f64p(x), R.f64p(zero))
+    L.lib().gs_set_num_ite(old)
+    assert res.name == b"gcsr"
+    return kernel_f64(R.last_y(len(lens)))
+
+
+def reduced(lens, vtype, itype):
+    from gpu_spmv_b200 import engine as E
+
+    row, col, e, m = _structure(lens)
+    val = torch.tensor([2.0 ** 30, 1.0, -2.0 ** 30, 0.0], device="cuda")[e % 4]
+    A = E.Matrix(row, col.int(), val, ncols=m, fmt="CSR", vtype=vtype, itype=itype)
+    y = A.spmv(torch.ones(m, device="cuda"))
+    A.close()
+    n = torch.as_tensor(lens).cuda() / 4
+    assert not y.any() or torch.equal(y, n.float())
+    return ROWS if not y.any() else CSR
+
+
+# rows that do not fit a window of 480 positions (FP64) or 1024 together with three others: from
+# 6,000 of them on; longer than it: from 20,000
+FEW = [(1000, 100, CSR), (300, 300, ROWS), (1000, 200, ROWS), (5999, 200, ROWS), (6000, 200, CSR),
+       (30, 10000, ROWS), (19999, 600, ROWS), (20000, 600, CSR)]
+
+
+@pytest.mark.parametrize("n, length, want", FEW)
+def test_few_long_rows(n, length, want):
+    lens = [length] * n
+    assert product(lens) == want
+    assert product(lens, dict(fmt="AXT", mode="COM", tileH=1)) == want
+    assert arrays(lens) == want
+    if length <= n:
+        assert dropin(lens) == want
+
+
+@pytest.mark.parametrize("vtype, itype", [("f32", "u32"), ("f32", "u16"), ("bf16", "u32"),
+                                          ("bf16", "u16")])
+@pytest.mark.parametrize("n, length, want", [(1000, 200, CSR), (300, 400, ROWS), (5999, 400, ROWS),
+                                             (6000, 400, CSR), (30, 10000, ROWS)])
+def test_few_long_rows_reduced(vtype, itype, n, length, want):
+    assert reduced([length] * n, vtype, itype) == want
