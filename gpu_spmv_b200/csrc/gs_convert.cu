@@ -505,13 +505,10 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         uint32_t V = kDirectV;
         bool aligned = false;
         if (!A->tiled && !need_rlen) {  // CSR and COM tileH = 1
-            bool rnd = false, even = true;
-            GS_TRY(random_columns(d_row, d_col, n, &rnd, s, &even));
-            // rows of 1 or 2 FP64 elements stay on the row-stream kernel (3M rows of 1 / 2 / 3:
-            // 18.7 / 25.7 / 45.4 us there, 22.8 / 31.0 / 35.1 on the CSR kernel)
-            A->csr_local = !rnd && even && (reduced || (double)nnz >= 2.5 * n) &&
-                           csr_enough_rows(n, nnz, p.vtype);
-            if (!reduced) V = direct_lane_positions(n, nnz, rnd);
+            CsrChoice c;
+            GS_TRY(csr_choice(d_row, d_col, n, nnz, p.vtype, &c, s));
+            A->csr_local = c.local;
+            if (!reduced) V = direct_lane_positions(n, nnz, c.random);
         }
         if (A->tiled) {
             V = th;

@@ -237,7 +237,7 @@ struct gs_matrix {
     // planned over tiles, for the tile kernel (launch_tiles); tile_w 0 otherwise
     gs::RowsPlan tplan;
     uint32_t tile_w = 0;
-    bool csr_local = false;  // CSR, COM tileH = 1: local columns, even rows (the CSR kernel)
+    bool csr_local = false;  // CSR, COM tileH = 1: products on the CSR kernel (csr_choice)
     double conv_ms = 0, mfp = 0, beta = 0;
 };
 
@@ -271,11 +271,12 @@ inline uint32_t direct_lane_positions(uint32_t n, uint64_t nnz, bool random)
     return random || (double)nnz < 8.0 * n ? 4u : kDirectV;
 }
 // Whether the x gathers of a CSR matrix are close to random: fewer than a quarter of a
-// sample of in-row column steps (up to 32 steps of 65,536 rows) stay within 16 columns.  With
-// `even`, also whether rows are even enough to be walked side by side: over a sample of groups
-// of 32 rows, 32 times the longest is at most 2.5 times the elements.
+// sample of in-row column steps (up to 32 steps of 65,536 rows) stay within 16 columns.
 gs_status random_columns(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
-                         bool *random, cudaStream_t s, bool *even = nullptr);
+                         bool *random, cudaStream_t s);
+// That sample of n > 0 rows, on s: cnt[0] += steps, cnt[1] += those within 16 columns.
+gs_status sample_col_steps(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
+                           unsigned long long *cnt, cudaStream_t s);
 // Positions per lane for a layout whose rows start on multiples of `align` positions
 // (0: no alignment): returns the V that makes the aligned kernel apply, or kDirectV.
 uint32_t aligned_lane_positions(uint32_t align, bool *aligned);
@@ -310,6 +311,13 @@ gs_status launch_csr(const CsrArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype 
                      cudaStream_t s);
 // Whether n rows (> 0) of nnz elements are enough to keep that kernel's warps busy.
 bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype);
+// What a look at a CSR matrix says: whether its x gathers are close to random, and whether its
+// products suit that kernel (see csr_suits in gs_spmv_csr.cu).  Synchronises.
+struct CsrChoice {
+    bool random = false, local = false;
+};
+gs_status csr_choice(const uint32_t *d_row, const uint32_t *d_col, uint32_t n, uint32_t nnz,
+                     gs_dtype vtype, CsrChoice *out, cudaStream_t s);
 // y = A x from CSR arrays, FP64, by the row-stream kernel on a plan made for the call
 // (synchronises).
 gs_status csr_rows_product(uint32_t n, uint32_t nnz, const uint32_t *d_row, const uint32_t *d_col,

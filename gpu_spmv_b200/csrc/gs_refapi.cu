@@ -512,12 +512,11 @@ str_res test_gcsr(const UIN cudaBlockSize, const str_matCSR m, const FPT *vec, c
 {
     (void)cudaBlockSize;
     DevBuf row, col, val, x, y;
-    bool rnd = false, even = true;
+    gs::CsrChoice choice;
     if (upload_csr(m, row, col, val) || h2d(x, vec, m.nrows) || y.alloc((size_t)m.nrows * 8) ||
-        gs::random_columns(row.as<UIN>(), col.as<UIN>(), m.nrows, &rnd, 0, &even))
+        gs::csr_choice(row.as<UIN>(), col.as<UIN>(), m.nrows, m.nnz, GS_F64, &choice, 0))
         return error_res("gcsr", gs_last_error());
-    if (!rnd && even && (double)m.nnz >= 2.5 * m.nrows &&
-        gs::csr_enough_rows(m.nrows, m.nnz, GS_F64)) {
+    if (choice.local) {
         gs::CsrArgs c{};
         c.n = m.nrows;
         c.nnz = m.nnz;
@@ -532,7 +531,8 @@ str_res test_gcsr(const UIN cudaBlockSize, const str_matCSR m, const FPT *vec, c
     }
     gs::RowsPlan P;
     if (gs::build_rows_plan(row.as<UIN>(), nullptr, m.nrows,
-                            gs::direct_lane_positions(m.nrows, m.nnz, rnd), P, 0))
+                            gs::direct_lane_positions(m.nrows, m.nnz, choice.random), P,
+                            0))
         return error_res("gcsr", gs_last_error());
     gs::RowsArgs a = gs::rows_args(P);
     a.val = val.p;

@@ -24,8 +24,8 @@
 // Random columns stay on the row-stream kernel (power-law 4.2M rows: 326 us against 410 for
 // products staged in position order), and so do rows of very uneven length, which leave lanes
 // idle here (lognormal lengths of sigma 1.2, local columns, 24.5M elements: FP64 107 against 120
-// us, BF16 60 against 133): gs_matrix_create samples both (random_columns).  Few long rows stay
-// there too (csr_enough_rows).  A product straight from CSR arrays runs here without the sample,
+// us, BF16 60 against 133), few long rows (csr_enough_rows) and long rows side by side:
+// gs_matrix_create looks at the matrix (csr_suits).  A product straight from CSR arrays runs here without the sample,
 // whose read-back costs more than it could save: 27-point 101^3 180 us with the row-stream kernel
 // and its plan's kernels, 79 us here.
 #include <cmath>
@@ -284,6 +284,84 @@ bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype)
     const double avg = (double)nnz / n;
     if (avg * c.rows <= (c.cap - 8) / 1.05) return true;
     return n >= (avg <= c.cap ? 6000u : 20000u);
+}
+
+// Row lengths, for csr_suits: over `take` groups of 32 rows, `stride` groups apart, out[0] += 32
+// times the longest row, out[1] += elements; over all n rows out[2] = the longest, and over all
+// groups of G rows out[3] = the most elements (out cleared before).
+__global__ void __launch_bounds__(256) k_row_shape(const uint32_t *__restrict__ row, uint32_t n,
+                                                   uint32_t stride, uint32_t take, uint32_t G,
+                                                   unsigned long long *out)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t t = blockIdx.x * 256ull + threadIdx.x, all = gridDim.x * 256ull;
+    for (uint64_t w = t >> 5; w < take; w += all >> 5) {
+        const uint32_t r = (uint32_t)w * stride * 32u + lane;
+        const uint32_t len = row[r + 1] - row[r];
+        const uint32_t top = __reduce_max_sync(kFull, len), sum = __reduce_add_sync(kFull, len);
+        if (lane == 0) {
+            atomicAdd(out, 32ull * top);
+            atomicAdd(out + 1, (unsigned long long)sum);
+        }
+    }
+    uint32_t longest = 0, heaviest = 0;
+    for (uint64_t r = t; r < n; r += all) {
+        const uint32_t b = row[r];
+        longest = max(longest, row[r + 1] - b);
+        if (r % G == 0) heaviest = max(heaviest, row[min(r + G, (uint64_t)n)] - b);
+    }
+    longest = __reduce_max_sync(kFull, longest);
+    heaviest = __reduce_max_sync(kFull, heaviest);
+    if (lane == 0) {
+        atomicMax(out + 2, (unsigned long long)longest);
+        atomicMax(out + 3, (unsigned long long)heaviest);
+    }
+}
+
+// Whether a matrix's products run on k_csr rather than on the row-stream kernel: local columns;
+// rows of even length (over a sample of groups of 32 rows, 32 times the longest at most 2.5 times
+// the elements); FP64 rows of 2.5 elements or more on average (3M rows of 1 / 2 / 3: 18.7 / 25.7 /
+// 45.4 us on the row-stream kernel, 22.8 / 31.0 / 35.1 here); enough of them; and no group of a
+// warp's rows that the warp would still be walking when the others are done.  A single long row is
+// none (one warp walks it in either kernel: 300,000 rows of 5 and one of 30,000 296 us there, 144
+// here), nor a group of 1 1/4 windows (of 480 at least), nor one within 1/8000 of the elements
+// (some 10 % of the product's time); several long rows side by side are (1M rows of 27, 16 of 2,000
+// among them 81 us there and 166 here, 64 of 10,000 123 and 946; 300,000 of 5 with 128 of 300 11
+// and 49).
+static bool csr_suits(uint32_t n, uint32_t nnz, gs_dtype vtype, const unsigned long long steps[2],
+                      const unsigned long long shape[4])
+{
+    const bool f64 = vtype == GS_F64, random = steps[1] * 4 < steps[0];
+    if (random || shape[0] * 2 > shape[1] * 5) return false;
+    if (f64 && (double)nnz < 2.5 * n) return false;
+    if (!csr_enough_rows(n, nnz, vtype)) return false;
+    const CsrShape c = csr_shape(n, nnz, f64);
+    const double own = 1.25 * c.rows * (double)nnz / n;
+    return shape[3] <= (c.cap > 480 ? 1280u : 600u) || shape[3] <= nnz / 8000u ||
+           (double)shape[3] <= (double)shape[2] + own;
+}
+
+gs_status csr_choice(const uint32_t *d_row, const uint32_t *d_col, uint32_t n, uint32_t nnz,
+                     gs_dtype vtype, CsrChoice *out, cudaStream_t s)
+{
+    *out = CsrChoice();
+    if (n == 0) return GS_OK;
+    StreamBuf cnt(s);
+    GS_TRY(cnt.alloc_zero(48));
+    unsigned long long *c = cnt.as<unsigned long long>();
+    GS_TRY(sample_col_steps(d_row, d_col, n, c, s));
+    const uint32_t groups = n / 32, take = groups < 4096u ? groups : 4096u;
+    const uint32_t blocks = (n - 1) / 256 + 1;
+    k_row_shape<<<blocks < 148u * 8u ? blocks : 148u * 8u, 256, 0, s>>>(
+        d_row, n, take ? groups / take : 0u, take,
+        (uint32_t)csr_shape(n, nnz, vtype == GS_F64).rows, c + 2);
+    GS_CHECK_LAUNCH();
+    unsigned long long h[6] = {0, 0, 0, 0, 0, 0};
+    GS_CUDA(cudaMemcpyAsync(h, c, 48, cudaMemcpyDeviceToHost, s));
+    GS_CUDA(cudaStreamSynchronize(s));
+    out->random = h[1] * 4 < h[0];
+    out->local = csr_suits(n, nnz, vtype, h, h + 2);
+    return GS_OK;
 }
 
 gs_status launch_csr(const CsrArgs &a0, gs_dtype vtype, gs_itype itype, gs_dtype ytype,

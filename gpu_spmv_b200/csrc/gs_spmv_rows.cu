@@ -1705,48 +1705,29 @@ gs_status launch_tiles_t(const RowsArgs &a, cudaStream_t s)
     return GS_OK;
 }
 
-// Over `take` groups of 32 rows, `stride` groups apart: out[0] += 32 times the longest row,
-// out[1] += elements
-__global__ void k_row_spread(const uint32_t *__restrict__ row, uint32_t stride, uint32_t take,
-                             unsigned long long *out)
-{
-    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (w >= take) return;
-    const uint32_t r = w * stride * 32u + (threadIdx.x & 31u);
-    const uint32_t len = row[r + 1] - row[r];
-    const uint32_t top = __reduce_max_sync(kFull, len), sum = __reduce_add_sync(kFull, len);
-    if ((threadIdx.x & 31u) == 0) {
-        atomicAdd(out, 32ull * top);
-        atomicAdd(out + 1, (unsigned long long)sum);
-    }
-}
-
 }  // namespace
 
+gs_status sample_col_steps(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
+                           unsigned long long *cnt, cudaStream_t s)
+{
+    const uint32_t samples = n < 65536u ? n : 65536u;
+    k_col_steps<<<(samples + 255) / 256, 256, 0, s>>>(d_row, d_col, n / samples, samples, cnt);
+    GS_CHECK_LAUNCH();
+    return GS_OK;
+}
+
 gs_status random_columns(const uint32_t *d_row, const uint32_t *d_col, uint32_t n,
-                         bool *random, cudaStream_t s, bool *even)
+                         bool *random, cudaStream_t s)
 {
     *random = false;
-    if (even) *even = true;
     if (n == 0) return GS_OK;
-    const uint32_t samples = n < 65536u ? n : 65536u;
-    const uint32_t stride = n / samples;
     StreamBuf cnt(s);
-    GS_TRY(cnt.alloc_zero(32));
-    k_col_steps<<<(samples + 255) / 256, 256, 0, s>>>(d_row, d_col, stride, samples,
-                                                      cnt.as<unsigned long long>());
-    GS_CHECK_LAUNCH();
-    if (even && n >= 32) {
-        const uint32_t groups = n / 32, take = groups < 4096u ? groups : 4096u;
-        k_row_spread<<<(take + 7) / 8, 256, 0, s>>>(d_row, groups / take, take,
-                                                    cnt.as<unsigned long long>() + 2);
-        GS_CHECK_LAUNCH();
-    }
-    unsigned long long h[4] = {0, 0, 0, 0};
-    GS_CUDA(cudaMemcpyAsync(h, cnt.p, 32, cudaMemcpyDeviceToHost, s));
+    GS_TRY(cnt.alloc_zero(16));
+    GS_TRY(sample_col_steps(d_row, d_col, n, cnt.as<unsigned long long>(), s));
+    unsigned long long h[2] = {0, 0};
+    GS_CUDA(cudaMemcpyAsync(h, cnt.p, 16, cudaMemcpyDeviceToHost, s));
     GS_CUDA(cudaStreamSynchronize(s));
     *random = h[1] * 4 < h[0];
-    if (even) *even = h[2] * 2 <= h[3] * 5;
     return GS_OK;
 }
 

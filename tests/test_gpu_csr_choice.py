@@ -109,3 +109,41 @@ def test_few_long_rows(n, length, want):
                                              (6000, 400, CSR), (30, 10000, ROWS)])
 def test_few_long_rows_reduced(vtype, itype, n, length, want):
     assert reduced([length] * n, vtype, itype) == want
+
+
+def _with(n, length, at):
+    """n rows of `length`, but for at = {row: (rows, length)}."""
+    lens = [length] * n
+    for r, (rows, l) in at.items():
+        lens[r:r + rows] = [l] * rows
+    return lens
+
+
+# long rows side by side, which one warp of the CSR kernel would walk one after the other; long rows
+# alone or apart, which either kernel gives to one warp
+SIDE = {
+    "16 of 500": (_with(20000, 28, {9000: (16, 500)}), ROWS),
+    "last 8 of 2000": (_with(20000, 28, {19992: (8, 2000)}), ROWS),
+    "two apart": (_with(20000, 28, {40: (1, 1000), 17000: (1, 1000)}), CSR),
+    "one": (_with(20000, 28, {19999: (1, 12000)}), CSR),
+    "one among short ones": (_with(300000, 4, {299999: (1, 30000)}), CSR),
+    "128 of 300": (_with(300000, 4, {150016: (128, 300)}), ROWS),
+    "64 of 40": (_with(1000, 8, {480: (64, 40)}), ROWS),
+    "64 of 40 in many": (_with(3000000, 4, {480: (64, 40)}), CSR),
+    "none": ([28] * 20000, CSR),
+}
+
+
+@pytest.mark.parametrize("name", SIDE)
+def test_long_rows_side_by_side(name):
+    lens, want = SIDE[name]
+    assert product(lens) == want
+    assert product(lens, dict(fmt="AXT", mode="COM", tileH=1)) == want
+    assert dropin(lens) == want
+
+
+@pytest.mark.parametrize("vtype, itype", [("f32", "u32"), ("bf16", "u16")])
+@pytest.mark.parametrize("name, want", [("16 of 500", ROWS), ("one", CSR), ("none", CSR),
+                                        ("64 of 40", ROWS)])
+def test_long_rows_side_by_side_reduced(vtype, itype, name, want):
+    assert reduced(SIDE[name][0], vtype, itype) == want
