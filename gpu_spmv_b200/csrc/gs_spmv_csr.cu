@@ -320,8 +320,13 @@ __global__ void __launch_bounds__(256) k_row_shape(const uint32_t *__restrict__ 
 
 // Whether a matrix's products run on k_csr rather than on the row-stream kernel: local columns;
 // rows of even length (over a sample of groups of 32 rows, 32 times the longest at most 2.5 times
-// the elements); FP64 rows of 2.5 elements or more on average (3M rows of 1 / 2 / 3: 18.7 / 25.7 /
-// 45.4 us on the row-stream kernel, 22.8 / 31.0 / 35.1 here); enough of them; and no group of a
+// the elements); rows of 2.5 elements or more on average (FP64, 3M rows of 1 / 2 / 3: 18.7 / 25.7 /
+// 45.4 us on the row-stream kernel, 22.8 / 31.0 / 35.1 here; FP32, 12M: 66 / 66 / 92 and 77 / 77 /
+// 85), for the reduced types of 4.5 unless they are nearly all the same (32 times the longest at
+// most 1.25 times the elements; 12M rows of 4 in the four reduced types 108 / 94 / 96 / 93 us and
+// 104 / 99 / 104 / 93, of 1 to 5 92 / 87 / 88 / 84 and 99 / 96 / 104 / 103, of 1 to 8 122 / 118 / 121
+// / 119 and 125 / 124 / 137 / 130, of 5 137 / 132 / 134 / 131 and 116 / 110 / 118 / 107, of 1 to 9
+// level); enough of them; and no group of a
 // warp's rows that the warp would still be walking when the others are done.  A single long row is
 // none (one warp walks it in either kernel: 300,000 rows of 5 and one of 30,000 296 us there, 144
 // here), nor a group of 1 1/4 windows (of 480 at least), nor one within 1/8000 of the elements
@@ -333,7 +338,8 @@ static bool csr_suits(uint32_t n, uint32_t nnz, gs_dtype vtype, const unsigned l
 {
     const bool f64 = vtype == GS_F64, random = steps[1] * 4 < steps[0];
     if (random || shape[0] * 2 > shape[1] * 5) return false;
-    if (f64 && (double)nnz < 2.5 * n) return false;
+    if ((double)nnz < 2.5 * n) return false;
+    if (!f64 && (double)nnz < 4.5 * n && shape[0] * 4 > shape[1] * 5) return false;
     if (!csr_enough_rows(n, nnz, vtype)) return false;
     const CsrShape c = csr_shape(n, nnz, f64);
     const double own = 1.25 * c.rows * (double)nnz / n;

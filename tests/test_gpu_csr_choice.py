@@ -147,3 +147,22 @@ def test_long_rows_side_by_side(name):
                                         ("64 of 40", ROWS)])
 def test_long_rows_side_by_side_reduced(vtype, itype, name, want):
     assert reduced(SIDE[name][0], vtype, itype) == want
+
+
+# rows of 4.5 elements at least, or of 2.5 and nearly all the same; of the FP64 ones 2.5
+SHORT = {
+    "1 on average": ([4, 0, 0, 0] * 20000, ROWS, ROWS),
+    "4": ([4] * 50000, CSR, CSR),
+    "4 and none": ([4, 4, 0, 4] * 20000, CSR, ROWS),
+    "8 and none": ([8, 0, 8, 0] * 20000, CSR, ROWS),
+    "4 and 8": ([4, 8] * 20000, CSR, CSR),
+}
+
+
+@pytest.mark.parametrize("name", SHORT)
+def test_short_rows(name):
+    lens, f64, other = SHORT[name]
+    if max(lens) > 4:  # a pair or two leave no rounding error in either kernel
+        assert product(lens) == f64
+    for vtype, itype in [("f32", "u32"), ("f32", "u16"), ("bf16", "u32"), ("bf16", "u16")]:
+        assert reduced(lens, vtype, itype) == other
