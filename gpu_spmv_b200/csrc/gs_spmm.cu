@@ -41,11 +41,20 @@ using namespace mm;
 constexpr int kMMThreads = 64;
 // One right-hand side streams: 32 warps (FP64 on a 27-point stencil 80^3 33.6 -> 31.1 us; with 16
 // 40.3).
-template <class T, int K>
-constexpr int kMMBlocks = (K == 1 ? 32 : (K * (int)sizeof(T) >= 64 ? 24 : 16)) / 2;
+// The adjoint with its value gradient holds a row of X besides and takes the warps that leave it its
+// registers: with the product's 24 warps it spilled 0.1 to 2.3 KB a thread from rows of 128 bytes on
+// (slot order on a 524,288-row power-law, FP64 k = 16 / 32: 323 / 1043 us, 204 / 397 here; FP32 k =
+// 32: 338, 201; FP64 k = 1 with 32 warps 69, with 24 55).
+template <class T, int K, bool ADJ> constexpr int mm_warps()
+{
+    constexpr int row = K * (int)sizeof(T);
+    if (K == 1) return ADJ && sizeof(T) == 8 ? 24 : 32;
+    if (ADJ && row >= 128) return row >= 256 ? 8 : 16;
+    return row >= 64 ? 24 : 16;
+}
 
 template <class T, int K, bool ADJ>
-__global__ void __launch_bounds__(kMMThreads, kMMBlocks<T, K>) k_k1_mm(const MMArgs a)
+__global__ void __launch_bounds__(kMMThreads, mm_warps<T, K, ADJ>() * 32 / kMMThreads) k_k1_mm(const MMArgs a)
 {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < a.units;
