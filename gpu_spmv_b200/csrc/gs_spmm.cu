@@ -482,6 +482,15 @@ gs_status gather_vals(size_t n, const DevBuf &src, const T *v, T *out, cudaStrea
     return GS_OK;
 }
 
+// adjoint-layout slots -> CSR order
+template <class T>
+gs_status scatter_vals(const gs_matrix *A, const T *v, T *out, cudaStream_t s)
+{
+    k_scatter_vals<T><<<148u * 16u, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(), v, out);
+    GS_CHECK_LAUNCH();
+    return GS_OK;
+}
+
 template <class T, bool ADJ>
 gs_status launch_mm(const MMArgs &a, uint32_t k, cudaStream_t s)
 {
@@ -823,27 +832,20 @@ gs_status gs_matrix_convert_values(const gs_matrix *A, const void *d_in, gs_valu
     if (!A->adj_ready) return fail(GS_ERR_INVALID, "gs_matrix_prepare_adjoint must run first");
     if (dtype != A->p.vtype) return fail(GS_ERR_UNSUPPORTED, "values take the matrix value type");
     cudaStream_t s = cs(stream);
-    const unsigned gb = 148u * 16u;
     const bool f64 = dtype == GS_F64;
     if (in_order == GS_VALUES_CSR) {  // slots[t] = csr[tsrc[t]], padding 0
         return f64 ? gather_vals<double>(A->tlenVC, A->tsrc, static_cast<const double *>(d_in),
                                          static_cast<double *>(d_out), s)
                    : gather_vals<float>(A->tlenVC, A->tsrc, static_cast<const float *>(d_in),
                                         static_cast<float *>(d_out), s);
-    } else if (in_order == GS_VALUES_SLOTS) {  // csr[tsrc[t]] = slots[t]
-        if (f64)
-            k_scatter_vals<double><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                      static_cast<const double *>(d_in),
-                                                      static_cast<double *>(d_out));
-        else
-            k_scatter_vals<float><<<gb, 256, 0, s>>>(A->tlenVC, A->tsrc.as<uint32_t>(),
-                                                     static_cast<const float *>(d_in),
-                                                     static_cast<float *>(d_out));
-    } else {
-        return fail(GS_ERR_INVALID, "unknown value order %d", (int)in_order);
     }
-    GS_CHECK_LAUNCH();
-    return GS_OK;
+    if (in_order == GS_VALUES_SLOTS) {  // csr[tsrc[t]] = slots[t]
+        return f64 ? scatter_vals(A, static_cast<const double *>(d_in),
+                                  static_cast<double *>(d_out), s)
+                   : scatter_vals(A, static_cast<const float *>(d_in),
+                                  static_cast<float *>(d_out), s);
+    }
+    return fail(GS_ERR_INVALID, "unknown value order %d", (int)in_order);
 }
 
 gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, void *d_Xbar,
@@ -864,8 +866,14 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     const bool f64 = A->p.vtype == GS_F64;
     if (mode != GS_ADJ_ATOMIC && mode != GS_ADJ_DETERMINISTIC)
         return fail(GS_ERR_INVALID, "unknown adjoint mode %d", (int)mode);
-    // a value gradient in CSR order has its own kernel; one in slot order comes with Xbar
-    const bool csr_vbar = d_vbar && vbar_order == GS_VALUES_CSR;
+    // a value gradient in CSR order has its own kernel; one in slot order comes with Xbar.  With 32
+    // right-hand sides the own kernel gathers two more rows of 128 or 256 bytes an element than the
+    // pass that forms both, which then leads also in CSR order, its gradient scattered (FP64 on a
+    // 524,288-row power-law / a band / a 27-point stencil 80^3 667 / 452 / 882 us with the own
+    // kernel, 519 / 399 / 761 so; FP32 300 / 215 / 422 and 279 / 218 / 364)
+    const bool scatter = d_vbar && vbar_order == GS_VALUES_CSR && k == 32 &&
+                         mode == GS_ADJ_DETERMINISTIC;
+    const bool csr_vbar = d_vbar && vbar_order == GS_VALUES_CSR && !scatter;
     if (csr_vbar) {
         VbarArgs v{};
         v.nnz = A->nnz;
@@ -906,9 +914,14 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
     }
     MMArgs a = adjoint_args(A, d_Ybar, d_Xbar);
     a.xrow = d_X;
-    a.vbar = csr_vbar ? nullptr : d_vbar;
+    a.vbar = csr_vbar ? nullptr : scatter ? A->vslots.p : d_vbar;
     a.ld = a.k = a.ldx = a.ldy = k;
-    if (a.vbar) return f64 ? launch_mm<double, true>(a, k, s) : launch_mm<float, true>(a, k, s);
+    if (a.vbar) {
+        GS_TRY((f64 ? launch_mm<double, true>(a, k, s) : launch_mm<float, true>(a, k, s)));
+        if (!scatter) return GS_OK;
+        return f64 ? scatter_vals(A, A->vslots.as<double>(), static_cast<double *>(d_vbar), s)
+                   : scatter_vals(A, A->vslots.as<float>(), static_cast<float *>(d_vbar), s);
+    }
     if (several_lanes(k, dtype))
         return f64 ? launch_mm_wide<double>(a, k, s) : launch_mm_wide<float>(a, k, s);
     return f64 ? launch_mm<double, false>(a, k, s) : launch_mm<float, false>(a, k, s);

@@ -112,3 +112,22 @@ def test_adjoint_operand_forms(k):
     with pytest.raises(TypeError):
         A.spmm(X[:-1])
     A.close()
+
+
+@pytest.mark.parametrize("vtype", ["f64", "f32"])
+def test_value_gradient_orders_32(vtype):
+    """32 right-hand sides: the CSR-order value gradient is the slot-order one, moved (every entry
+    written), also beside an Xbar of its own."""
+    from gpu_spmv_b200 import engine as E
+
+    rng = np.random.default_rng(32)
+    row, col, val = _matrix(6)
+    dt = torch.float64 if vtype == "f64" else torch.float32
+    A = E.Matrix(row, col, val, ncols=900, fmt="K1", vtype=vtype, adjoint=True)
+    X, Yb = _operand(rng, 900, 32, dt, "tight"), _operand(rng, 1000, 32, dt, "tight")
+    for _ in range(2):
+        Xc, vc = A.adjoint(Yb, X)
+        Xs, vs = A.adjoint(Yb, X, order="slots")
+        assert torch.equal(vc, A.convert_values(vs, to="csr")) and torch.equal(Xc, Xs)
+        assert torch.equal(vs, A.convert_values(vc, to="slots"))
+    A.close()
