@@ -361,14 +361,17 @@ void get_errors(const UIN len, const FPT *ar, const FPT *ac, str_err *e)
     e->pos = pos;
 }
 
+// On the row-stream kernel, whatever the matrix: it rounds every product and adds a lane's share of
+// a row in order, as the CPU loop does (the CSR kernel fuses and interleaves).
 void ncsr(const UIN ompNT, const str_matCSR m, const FPT *vec, FPT *res)
 {
     (void)ompNT;
+    if (m.nrows == 0) return;
     DevBuf row, col, val, x, y;
     if (h2d(row, m.row, (size_t)m.nrows + 1) || h2d(col, m.col, m.nnz) ||
         h2d(val, m.val, m.nnz) || h2d(x, vec, m.nrows) || y.alloc((size_t)m.nrows * 8) ||
-        gs_csr_spmv_f64(m.nrows, m.nrows, m.nnz, row.as<UIN>(), col.as<UIN>(), val.as<double>(),
-                        x.as<double>(), y.as<double>(), nullptr) ||
+        gs::csr_rows_product(m.nrows, m.nnz, row.as<UIN>(), col.as<UIN>(), val.as<double>(),
+                             x.as<double>(), y.as<double>(), nullptr) ||
         cudaMemcpy(res, y.p, (size_t)m.nrows * 8, cudaMemcpyDeviceToHost) != cudaSuccess) {
         fflush(stdout);
         printf("ncsr: %s\n", gs_last_error());
