@@ -23,7 +23,9 @@
 //
 // No counterpart in the reference, which runs one matrix and one right-hand side per call.
 #include <algorithm>
+#include <map>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <vector>
 
@@ -793,26 +795,25 @@ gs_status launch(gs_batch *B, cudaStream_t s)
 
 namespace {
 // A stream to capture on, held for one capture and kept for the next (making one takes 100 to
-// 400 us; there are as many as captures have ever run at once on the device).
+// 400 us; there are as many as captures have ever run at once in the context).
 struct CaptureStream {
-    CaptureStream()
+    CaptureStream() : ctx(gs::context_id())
     {
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) dev = -1;
         std::lock_guard<std::mutex> lock(mutex);
-        if (dev >= 0 && !idle[dev].empty()) {
-            s = idle[dev].back();
-            idle[dev].pop_back();
-        }
+        const auto kept = idle.find(ctx);
+        if (kept == idle.end() || kept->second.empty()) return;
+        s = kept->second.back();
+        kept->second.pop_back();
     }
     ~CaptureStream()
     {
         if (!s) return;
-        if (dev < 0) {
+        try {
+            std::lock_guard<std::mutex> lock(mutex);
+            idle[ctx].push_back(s);
+        } catch (const std::bad_alloc &) {
             cudaStreamDestroy(s);
-            return;
         }
-        std::lock_guard<std::mutex> lock(mutex);
-        idle[dev].push_back(s);
     }
     gs_status ready()
     {
@@ -822,13 +823,13 @@ struct CaptureStream {
     cudaStream_t s = nullptr;
 
 private:
-    static constexpr int kDevices = 64;
     static std::mutex mutex;
-    static std::vector<cudaStream_t> idle[kDevices];
-    int dev = -1;
+    static std::map<uint64_t, std::vector<cudaStream_t>> &idle;  // never destroyed
+    uint64_t ctx;
 };
 std::mutex CaptureStream::mutex;
-std::vector<cudaStream_t> CaptureStream::idle[CaptureStream::kDevices];
+std::map<uint64_t, std::vector<cudaStream_t>> &CaptureStream::idle =
+    *new std::map<uint64_t, std::vector<cudaStream_t>>;
 }  // namespace
 
 using namespace gs;

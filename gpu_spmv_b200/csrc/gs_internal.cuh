@@ -51,6 +51,13 @@ inline size_t dtype_size(gs_dtype t) { return t == GS_F64 ? 8 : (t == GS_F32 ? 4
 // above the free memory granted).
 constexpr size_t kPoolIdle = size_t(4) << 30;
 
+// Streams and pools belong to a context, which cudaDeviceReset ends (the program's own, or another
+// library's in the process): they are kept per context, and what is left of an ended one is dropped.
+struct DevPool;
+// Number of the calling thread's current context, never used twice in a process (0: none can be
+// made).
+uint64_t context_id();
+
 // Owning allocation that may be used on any stream.  alloc(n) is usable everywhere at once;
 // alloc(n, s) is ordered on s like the work that fills it, which the caller orders (or
 // synchronises) before any other stream's use.  reset() waits for the device, as cudaFree does.
@@ -58,7 +65,7 @@ struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     size_t reserved = 0;  // bytes taken from the pool
-    int dev = -1;
+    DevPool *pool = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
@@ -67,7 +74,7 @@ struct DevBuf {
     {
         if (this != &o) {
             reset();
-            p = o.p, bytes = o.bytes, reserved = o.reserved, dev = o.dev;
+            p = o.p, bytes = o.bytes, reserved = o.reserved, pool = o.pool;
             o.p = nullptr, o.bytes = 0;
         }
         return *this;
@@ -103,7 +110,7 @@ struct StreamBuf {
 private:
     cudaStream_t s;
     size_t reserved = 0;
-    int dev = -1;
+    DevPool *pool = nullptr;
 };
 // Gives the pool's unused memory back, on the current device.
 gs_status release_cached();

@@ -7,9 +7,14 @@
 // has no carry between blocks.  Here those become one device-wide exclusive scan
 // (reduce / scan-of-block-sums / down-sweep, 64-bit offsets so 32-bit overflow is
 // detected, no inter-block waiting) and a stable LSD radix sort built on it.
+#include <cuda.h>
+
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <new>
+#include <utility>
 
 #include "gs_internal.cuh"
 
@@ -30,26 +35,51 @@ void clear_error() { g_err[0] = 0; }
 const char *last_error_text() { return g_err; }
 
 // ------------------------------------------------------------------ device memory
-namespace {
-
-constexpr int kMaxDevices = 64;
-
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;  // orders allocations and frees that belong to no stream
+    int dev = -1;
+    uint64_t ctx = 0;
     size_t live = 0, kept_for = 0;  // bytes in buffers; the value of `live` the pool was told
 };
+
+uint64_t context_id()
+{
+    using Get = CUresult (*)(CUcontext, unsigned long long *);
+    static const Get get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r) !=
+                cudaSuccess || r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Get>(f);
+    }();
+    if (!get) return 1;
+    unsigned long long id = 0;
+    if (get(nullptr, &id) == CUDA_SUCCESS && id) return id;
+    if (cudaFree(nullptr) != cudaSuccess) return 0;  // makes the context the thread's current one
+    return get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+namespace {
+
 std::mutex g_pool_mutex;
-DevPool g_pools[kMaxDevices];  // live as long as the process, like the device's own pool
+// by device and context; never destroyed, since buffers may be reset while the process ends
+auto &g_pools = *new std::map<std::pair<int, uint64_t>, DevPool>;
 
 thread_local int t_idle_device = -1;  // DeviceIdle
 
-gs_status pool_of(int dev, DevPool **out)
+gs_status pool_of(DevPool **out) try
 {
-    if (dev < 0 || dev >= kMaxDevices) return fail(GS_ERR_UNSUPPORTED, "device %d", dev);
+    int dev = -1;
+    GS_CUDA(cudaGetDevice(&dev));
+    const uint64_t ctx = context_id();
+    if (!ctx) return fail(GS_ERR_CUDA, "no context on device %d", dev);
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    DevPool &P = g_pools[dev];
+    DevPool &P = g_pools[{dev, ctx}];
     if (!P.pool) {
+        P.dev = dev;
+        P.ctx = ctx;
         if (!P.stream) GS_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
@@ -63,6 +93,8 @@ gs_status pool_of(int dev, DevPool **out)
     }
     *out = &P;
     return GS_OK;
+} catch (const std::bad_alloc &) {
+    return fail(GS_ERR_ALLOC, "host allocation failed");
 }
 
 // The pool holds on to what its buffers use and kPoolIdle more; it is told again when the use
@@ -85,25 +117,23 @@ size_t rounded(size_t nbytes)  // slack: vector loads may touch the tail
 }
 
 // n bytes ordered on s, or on the pool's own stream (own)
-gs_status pool_alloc(size_t n, cudaStream_t s, bool own, void **p, int *dev)
+gs_status pool_alloc(size_t n, cudaStream_t s, bool own, void **p, DevPool **pool)
 {
-    GS_CUDA(cudaGetDevice(dev));
-    DevPool *P = nullptr;
-    GS_TRY(pool_of(*dev, &P));
-    if (own) s = P->stream;
+    GS_TRY(pool_of(pool));
+    if (own) s = (*pool)->stream;
     // a captured allocation would belong to the graph, not to the buffer
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     GS_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone)
         return fail(GS_ERR_CUDA, "device memory is needed on a stream under capture");
-    cudaError_t e = cudaMallocFromPoolAsync(p, n, P->pool, s);
+    cudaError_t e = cudaMallocFromPoolAsync(p, n, (*pool)->pool, s);
     if (e == cudaSuccess && own) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
         return fail(GS_ERR_ALLOC, "allocation of %zu bytes failed: %s", n, cudaGetErrorString(e));
     }
-    pool_use(*P, n, 0);
+    pool_use(**pool, n, 0);
     return GS_OK;
 }
 
@@ -112,7 +142,7 @@ gs_status pool_alloc(size_t n, cudaStream_t s, bool own, void **p, int *dev)
 gs_status DevBuf::alloc(size_t nbytes)
 {
     reset();
-    GS_TRY(pool_alloc(rounded(nbytes), nullptr, true, &p, &dev));
+    GS_TRY(pool_alloc(rounded(nbytes), nullptr, true, &p, &pool));
     reserved = rounded(nbytes);
     bytes = nbytes;
     return GS_OK;
@@ -121,7 +151,7 @@ gs_status DevBuf::alloc(size_t nbytes)
 gs_status DevBuf::alloc(size_t nbytes, cudaStream_t s)
 {
     reset();
-    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &dev));
+    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &pool));
     reserved = rounded(nbytes);
     bytes = nbytes;
     return GS_OK;
@@ -139,15 +169,15 @@ void DevBuf::reset()
     if (!p) return;
     int cur = -1;
     cudaGetDevice(&cur);
-    if (cur != dev) cudaSetDevice(dev);
+    if (cur != pool->dev) cudaSetDevice(pool->dev);
     // kernels of any stream may still read it; memory of a device that cannot be waited for
-    // stays allocated
-    if (t_idle_device == dev || cudaDeviceSynchronize() == cudaSuccess) {
-        DevPool &P = g_pools[dev];
-        cudaFreeAsync(p, P.stream);
-        pool_use(P, 0, reserved);
+    // stays allocated, and that of an ended context has gone with it
+    if (context_id() == pool->ctx &&
+        (t_idle_device == pool->dev || cudaDeviceSynchronize() == cudaSuccess)) {
+        cudaFreeAsync(p, pool->stream);
+        pool_use(*pool, 0, reserved);
     }
-    if (cur != dev) cudaSetDevice(cur);
+    if (cur != pool->dev) cudaSetDevice(cur);
     p = nullptr;
     bytes = 0;
 }
@@ -162,7 +192,7 @@ DeviceIdle::~DeviceIdle() { t_idle_device = outer; }
 
 gs_status StreamBuf::alloc(size_t nbytes)
 {
-    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &dev));
+    GS_TRY(pool_alloc(rounded(nbytes), s, false, &p, &pool));
     reserved = rounded(nbytes);
     return GS_OK;
 }
@@ -178,15 +208,13 @@ StreamBuf::~StreamBuf()
 {
     if (!p) return;
     cudaFreeAsync(p, s);
-    pool_use(g_pools[dev], 0, reserved);
+    pool_use(*pool, 0, reserved);
 }
 
 gs_status release_cached()
 {
-    int dev = -1;
-    GS_CUDA(cudaGetDevice(&dev));
     DevPool *P = nullptr;
-    GS_TRY(pool_of(dev, &P));
+    GS_TRY(pool_of(&P));
     GS_CUDA(cudaDeviceSynchronize());
     GS_CUDA(cudaMemPoolTrimTo(P->pool, 0));
     return GS_OK;
