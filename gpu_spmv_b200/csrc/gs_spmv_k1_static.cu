@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(256) k_k1s(const K1StaticArgs a)
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 unsigned char *g_scratch[kMaxDevices];
+uint64_t g_scratch_ctx[kMaxDevices];  // the context it was looked up in: a new one loads it anew
 
 // Address of this device's copy of gs_k1_static_scratch.  The first call per device looks
 // the symbol up and zeroes the arrival counters; it synchronises the device, so it belongs
@@ -218,8 +219,9 @@ gs_status device_scratch(unsigned char **out)
     GS_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices)
         return fail(GS_ERR_UNSUPPORTED, "device ordinal %d is above %d", dev, kMaxDevices - 1);
+    const uint64_t ctx = context_id();
     std::lock_guard<std::mutex> lock(g_setup_mutex);
-    if (!g_scratch[dev]) {
+    if (!g_scratch[dev] || g_scratch_ctx[dev] != ctx) {
         void *p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, gs_k1_static_scratch);
         if (e != cudaSuccess || !p)
@@ -229,6 +231,7 @@ gs_status device_scratch(unsigned char **out)
         GS_CUDA(cudaMemset(base + kCountOff, 0, kCountBytes));
         GS_CUDA(cudaDeviceSynchronize());
         g_scratch[dev] = base;
+        g_scratch_ctx[dev] = ctx;
     }
     *out = g_scratch[dev];
     return GS_OK;

@@ -84,9 +84,26 @@ def batch():
     for m in mats:
         lib.gs_matrix_destroy(m)
 
+def static():  # the K1 product whose scratch is a device array of the library
+    k = L.StrMatK1()
+    assert lib.getFormatDataK1(32, h.s, R.f64p(x), C.byref(k)).name == b"fk1", lib.gs_last_error()
+    a = R.k1_arrays(k)
+    dev = []
+    for v in (a["val"], a["col"], a["nmc"], a["chp"], a["permi"], x, np.zeros(n)):
+        p = C.c_void_p()
+        assert rt.cudaMalloc(C.byref(p), v.nbytes) == 0
+        assert rt.cudaMemcpy(p, v.ctypes.data_as(C.c_void_p), v.nbytes, 1) == 0
+        dev.append(p.value)
+    L.check(lib.gs_k1_spmv_f64_static(n, k.chunkNum, k.lenVC, *dev, None), "static")
+    assert rt.cudaDeviceSynchronize() == 0
+    y = np.full(n, np.nan)
+    L.check(lib.gs_copy_to_host(y.ctypes.data, dev[-1], n * 8), "copy")
+    assert np.abs(y - want).max() <= 1e-13
+
 kept = []
 for step in range(3):
-    kept.append(dict(dropin=dropin, matrices=matrices, held=held, batch=batch)[what]())
+    kept.append(dict(dropin=dropin, matrices=matrices, held=held, batch=batch,
+                     static=static)[what]())
     assert rt.cudaDeviceSynchronize() == 0
     assert rt.cudaDeviceReset() == 0
     if what == "held":
@@ -95,7 +112,7 @@ print("done")
 '''
 
 
-@pytest.mark.parametrize("what", ["dropin", "matrices", "held", "batch"])
+@pytest.mark.parametrize("what", ["dropin", "matrices", "held", "batch", "static"])
 def test_after_reset(what):
     r = subprocess.run([sys.executable, "-c", PROGRAM, ROOT, what], capture_output=True, text=True,
                        timeout=300)
