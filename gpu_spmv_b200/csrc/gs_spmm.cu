@@ -549,6 +549,7 @@ gs_status ensure_mm_scratch(gs_matrix *A, cudaStream_t s)
     std::lock_guard<std::mutex> lock(g_mm_mutex);
     if (A->mm_ready) return GS_OK;
     GS_TRY(A->mmpartial.alloc((size_t)A->k1split_units * 32 * 32 * 8 + 8, s));
+    GS_CUDA(cudaStreamSynchronize(s));  // from here on any stream may use it
     A->mm_ready = true;
     return GS_OK;
 }

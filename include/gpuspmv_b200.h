@@ -385,7 +385,10 @@ typedef enum {
  * in which the deterministic adjoint writes vbar without scattering. */
 typedef enum { GS_VALUES_CSR = 0, GS_VALUES_SLOTS = 1 } gs_value_order;
 
-/* Y = A X.  The first call sizes the matrix's multi-RHS scratch (allocates, synchronises). */
+/* Y = A X.  The first multi-RHS call on a matrix sizes its scratch (allocates, synchronises the
+ * stream).  Every multi-RHS product and adjoint on one matrix uses that scratch and the matrix's
+ * arrival counters, so calls that could overlap in time (other streams, other threads) must be
+ * ordered by the caller, as for gs_spmv. */
 gs_status gs_spmm(gs_matrix *A, const void *d_X, void *d_Y, gs_dtype dtype, UIN k,
                   gs_stream stream);
 /* Y = A X for any k from 1 to 32 and rows of X and Y that are ldx and ldy entries apart, aligned
@@ -412,8 +415,7 @@ gs_status gs_matrix_convert_values(const gs_matrix *A, const void *d_in,
 /* Xbar = A^T Ybar (Xbar [ncols][k], overwritten) and, when d_vbar is given,
  * vbar[e] = sum_r Ybar[row_e][r] * X[col_e][r] for every stored element e, in vbar_order
  * (the gradient with respect to the values; d_X is then required).  X, Ybar and Xbar are
- * 32-byte aligned.  The atomic mode forms a slot-order vbar in a buffer of the matrix first, so
- * calls on one matrix must not overlap.
+ * 32-byte aligned.  Calls on one matrix must not overlap (gs_spmm).
  * The atomic mode without d_vbar reads neither X nor a second copy of the values. */
 gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, void *d_Xbar,
                           void *d_vbar, gs_dtype dtype, UIN k, gs_adjoint_mode mode,
