@@ -598,6 +598,7 @@ str_res test_gk1(const UIN cudaBlockSize, const str_matK1 k, const FPT *vec, con
         h2d(x, vec, k.nrows) || y.alloc((size_t)k.nrows * 8) ||
         own_chp.alloc((size_t)k.chunkNum * 4) || ub.alloc(((size_t)k.chunkNum + 1) * 4) ||
         gs::k1_layout_scan(nmc.as<UIN>(), k.chunkNum, own_chp.as<UIN>(), ub.as<UIN>(), total, 0) ||
+        (total[1] >= 0xffffffffull && gs::fail(GS_ERR_OVERFLOW, "K1 plan too large")) ||
         gs::build_k1_units(ub.as<UIN>(), k.chunkNum, (uint32_t)total[1], uc, &part, cnt, 0))
         return error_res("gk1", gs_last_error());
     const uint32_t units = (uint32_t)total[1];
