@@ -127,7 +127,8 @@ gs_status pool_alloc(size_t n, cudaStream_t s, bool own, void **p, DevPool **poo
     if (cap != cudaStreamCaptureStatusNone)
         return fail(GS_ERR_CUDA, "device memory is needed on a stream under capture");
     cudaError_t e = cudaMallocFromPoolAsync(p, n, (*pool)->pool, s);
-    if (e == cudaSuccess && own) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && own && (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        cudaFreeAsync(*p, s);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
