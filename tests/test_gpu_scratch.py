@@ -17,9 +17,10 @@ def test_first_call_waits(how):
     lens = rng.integers(0, 20, 500)
     lens[3] = 400  # a cut chunk: the scratch is used
     row, col, val = csr_from_lengths(lens, 500, rng)
-    A = E.Matrix(row, col, val, ncols=500, fmt="K1")
+    A, other = (E.Matrix(row, col, val, ncols=500, fmt="K1") for _ in range(2))
     X = torch.from_numpy(rng.standard_normal((500, 8))).cuda()
     X = X if how == "gs_spmm" else X[:, :3]
+    want = other.spmm(X)  # loads the kernels, which waits by itself
     torch.cuda.synchronize()
     s, t = torch.cuda.Stream(), torch.cuda.Stream()
     queued = torch.cuda.Event()
@@ -35,5 +36,6 @@ def test_first_call_waits(how):
         second = A.spmm(X)
         assert not queued.query()  # only the first call waits
     torch.cuda.synchronize()
-    assert torch.equal(first, second)
+    assert torch.equal(first, want) and torch.equal(second, want)
     A.close()
+    other.close()

@@ -99,7 +99,7 @@ def test_new_values_every_step(order):
         return (zero.index_add(0, i, v[:, None] * D[j]),
                 zero.index_add(0, i, v.abs()[:, None] * D[j].abs()))
 
-    for i in range(4):
+    def check(i):  # nothing outlives it: the next step's tensors take this one's places
         v = theta * (i + 1.0)
         g = (B[r] * X[c]) * (i + 1.0)
         # sums of at most 30 products
@@ -107,4 +107,7 @@ def test_new_values_every_step(order):
                                               (g.sum(1), g.abs().sum(1)),
                                               product(200, c, r, v, B))):
             assert torch.all((got - want).abs() <= 64 * 2.0 ** -53 * mag)
+
+    for i in range(4):
+        check(i)
     op.close()
