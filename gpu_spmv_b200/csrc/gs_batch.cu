@@ -23,9 +23,6 @@
 //
 // No counterpart in the reference, which runs one matrix and one right-hand side per call.
 #include <algorithm>
-#include <map>
-#include <mutex>
-#include <new>
 #include <numeric>
 #include <vector>
 
@@ -797,23 +794,10 @@ namespace {
 // A stream to capture on, held for one capture and kept for the next (making one takes 100 to
 // 400 us; there are as many as captures have ever run at once in the context).
 struct CaptureStream {
-    CaptureStream() : ctx(gs::context_id())
-    {
-        std::lock_guard<std::mutex> lock(mutex);
-        const auto kept = idle.find(ctx);
-        if (kept == idle.end() || kept->second.empty()) return;
-        s = kept->second.back();
-        kept->second.pop_back();
-    }
+    CaptureStream() : ctx(gs::context_id()) { kept.take(ctx, &s); }
     ~CaptureStream()
     {
-        if (!s) return;
-        try {
-            std::lock_guard<std::mutex> lock(mutex);
-            idle[ctx].push_back(s);
-        } catch (const std::bad_alloc &) {
-            cudaStreamDestroy(s);
-        }
+        if (s && !kept.give(ctx, s)) cudaStreamDestroy(s);
     }
     gs_status ready()
     {
@@ -823,13 +807,10 @@ struct CaptureStream {
     cudaStream_t s = nullptr;
 
 private:
-    static std::mutex mutex;
-    static std::map<uint64_t, std::vector<cudaStream_t>> &idle;  // never destroyed
+    static gs::Kept<cudaStream_t> &kept;  // never destroyed
     uint64_t ctx;
 };
-std::mutex CaptureStream::mutex;
-std::map<uint64_t, std::vector<cudaStream_t>> &CaptureStream::idle =
-    *new std::map<uint64_t, std::vector<cudaStream_t>>;
+gs::Kept<cudaStream_t> &CaptureStream::kept = *new gs::Kept<cudaStream_t>;
 }  // namespace
 
 using namespace gs;

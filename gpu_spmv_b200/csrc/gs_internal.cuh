@@ -7,7 +7,11 @@
 
 #include <cstdarg>
 #include <cstddef>
+#include <map>
+#include <mutex>
+#include <new>
 #include <type_traits>
+#include <vector>
 
 #include "gpuspmv_b200.h"
 
@@ -57,6 +61,32 @@ struct DevPool;
 // Number of the calling thread's current context, never used twice in a process (0: none can be
 // made).
 uint64_t context_id();
+
+// What calls hold one at a time and leave for the next, per context: as many as were ever held at
+// once.
+template <class T> class Kept {
+public:
+    bool take(uint64_t ctx, T *t)
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        const auto i = idle.find(ctx);
+        if (i == idle.end() || i->second.empty()) return false;
+        *t = i->second.back();
+        i->second.pop_back();
+        return true;
+    }
+    bool give(uint64_t ctx, T t) try {
+        std::lock_guard<std::mutex> lock(mutex);
+        idle[ctx].push_back(t);
+        return true;
+    } catch (const std::bad_alloc &) {
+        return false;
+    }
+
+private:
+    std::mutex mutex;
+    std::map<uint64_t, std::vector<T>> idle;
+};
 
 // Owning allocation that may be used on any stream.  alloc(n) is usable everywhere at once;
 // alloc(n, s) is ordered on s like the work that fills it, which the caller orders (or
@@ -312,6 +342,7 @@ struct CsrArgs {
     const uint32_t *colbase;   // 16-bit columns: base of each 256 positions
     const void *val, *col, *x;
     void *y;
+    uint32_t *overlong;        // nullptr, or a word (0) that gets 1 if warps left long rows undone
     bool y64;                  // set by launch_csr
 };
 gs_status launch_csr(const CsrArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype ytype,

@@ -25,9 +25,10 @@
 // products staged in position order), and so do rows of very uneven length, which leave lanes
 // idle here (lognormal lengths of sigma 1.2, local columns, 24.5M elements: FP64 107 against 120
 // us, BF16 60 against 133), few long rows (csr_enough_rows) and long rows side by side:
-// gs_matrix_create looks at the matrix (csr_suits).  A product straight from CSR arrays runs here without the sample,
-// whose read-back costs more than it could save: 27-point 101^3 180 us with the row-stream kernel
-// and its plan's kernels, 79 us here.
+// gs_matrix_create looks at the matrix (csr_suits).  A product straight from CSR arrays runs here
+// without that look, whose read-back would cost more than it saves (27-point 101^3 180 us with the
+// row-stream kernel and its plan's kernels, 79 us here), until a warp meets long rows side by side
+// (kCsrOverlong).
 #include <cmath>
 
 #include "gs_internal.cuh"
@@ -38,6 +39,11 @@ namespace {
 
 constexpr int kCsrWarps = 2;  // warps per block: its place is free when two warps end
 constexpr unsigned kFull = 0xffffffffu;
+// With CsrArgs::overlong: elements beside its longest row from which on a warp leaves its rows
+// undone and says so.  One warp walks 150 (rows one by one) to 300 a microsecond, so this is about
+// the time that the row-stream kernel's plan takes (30 rows of 12,000, 36,000 beside the longest:
+// 325 us here, 367 with the plan; 1M rows of 27 and 128 of 30,000 side by side: 1457, 533).
+constexpr uint32_t kCsrOverlong = 49152;
 
 // Shared-memory index of position p for elements of B bytes: as it is, or (PAD) with a gap of 16
 // bytes after every 128, for rows of about 8 m elements, whose lanes would otherwise meet in the
@@ -173,6 +179,16 @@ __global__ void __launch_bounds__(kCsrWarps * 32) k_csr(const CsrArgs a)
         return;
     }
     // too long for one window: as many rows at a time as fit, a longer row alone in windows
+    if (a.overlong && end > c0) {
+        uint32_t longest = 0;
+#pragma unroll
+        for (int k = 0; k < R; k++) longest = max(longest, re[k] > rp[k] ? re[k] - rp[k] : 0u);
+        longest = __reduce_max_sync(kFull, longest);
+        if (end - c0 > longest && end - c0 - longest > kCsrOverlong) {
+            if (lane == 0) *static_cast<volatile uint32_t *>(a.overlong) = 1u;
+            return;
+        }
+    }
 #pragma unroll 1
     for (int k = 0; k < R; k++) {
         const uint32_t b0 = r0 + (uint32_t)(W * k);

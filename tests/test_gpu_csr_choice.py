@@ -98,7 +98,6 @@ def test_few_long_rows(n, length, want):
     lens = [length] * n
     assert product(lens) == want
     assert product(lens, dict(fmt="AXT", mode="COM", tileH=1)) == want
-    assert arrays(lens) == want
     if length <= n:
         assert dropin(lens) == want
 
@@ -166,3 +165,25 @@ def test_short_rows(name):
         assert product(lens) == f64
     for vtype, itype in [("f32", "u32"), ("f32", "u16"), ("bf16", "u32"), ("bf16", "u16")]:
         assert reduced(lens, vtype, itype) == other
+
+
+# straight from CSR arrays nothing is known of the rows beforehand: a warp that meets more than 49152
+# elements beside its longest row leaves them, and the call goes to the row-stream kernel
+@pytest.mark.parametrize("name, lens, want", [
+    ("16 of 2000", _with(20000, 28, {19984: (16, 2000)}), CSR),
+    ("16 of 4000", _with(20000, 28, {19984: (16, 4000)}), CSR),  # 31.2 on average: 8 rows a warp
+    ("16 of 8000", _with(20000, 28, {19984: (16, 8000)}), ROWS),
+    ("300 of 300", [300] * 300, CSR),
+    ("30 of 10000", [10000] * 30, CSR),
+    ("30 of 12000", [12000] * 30, CSR),
+    ("30 of 20000", [20000] * 30, ROWS),
+    ("first 2 of 40000", _with(60000, 28, {0: (2, 40000)}), CSR),
+    ("first 2 of 60000", _with(60000, 28, {0: (2, 59998)}), ROWS),
+    ("one", _with(100000, 28, {99999: (1, 90000)}), CSR),
+    ("two apart", _with(100000, 28, {5: (1, 60000), 99999: (1, 90000)}), CSR),
+    ("one among short ones", _with(700000, 4, {699999: (1, 60000)}), CSR),
+    ("2 among short ones", _with(700000, 4, {699998: (2, 60000)}), ROWS),
+])
+def test_arrays_long_rows(name, lens, want):
+    for _ in range(2):
+        assert arrays(lens) == want
