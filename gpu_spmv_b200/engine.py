@@ -336,6 +336,13 @@ def csr_spmv_f64(row: torch.Tensor, col: torch.Tensor, val: torch.Tensor, x: tor
     return y
 
 
+def release_cached(device="cuda"):
+    """Give the device memory of destroyed matrices and of conversions' scratch, which the engine
+    keeps for the next ones (up to 4 GiB per device), back to the device (waits for it)."""
+    with torch.cuda.device(torch.device(device)):
+        L.check(L.lib().gs_release_cached(), "gs_release_cached")
+
+
 def algorithmic_bytes(nrows, ncols, nnz, k=1, s_v=8, s_i=4, s_x=8, s_y=8) -> float:
     return L.lib().gs_algorithmic_bytes(nrows, ncols, nnz, k, s_v, s_i, s_x, s_y)
 

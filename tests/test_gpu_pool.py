@@ -67,3 +67,18 @@ def test_release_cached():
     before = torch.cuda.mem_get_info()[0]
     L.check(L.lib().gs_release_cached(), "gs_release_cached")
     assert torch.cuda.mem_get_info()[0] - before >= held
+
+
+def test_release_cached_python():
+    """A Python program gives the memory of closed matrices back without the C library."""
+    from gpu_spmv_b200 import engine as E
+
+    rng = np.random.default_rng(6)
+    row, col, val = csr_from_lengths(np.full(100000, 50), 200000, rng)
+    A = E.Matrix(row, col, val, ncols=200000, fmt="K1")
+    held = A.info.nslots * 12
+    A.close()
+    before = torch.cuda.mem_get_info()[0]
+    E.release_cached()
+    assert torch.cuda.mem_get_info()[0] - before >= held
+    E.release_cached("cuda:0")
