@@ -150,7 +150,6 @@ gs_status release_cached();
 // offsets out[0..n] (out[n] = total).  Implemented in gs_scan.cu for the functors listed
 // there; `total` receives out[n] on the host (synchronises the stream).
 enum class CountKind {
-    RowLen,         // row[i+1]-row[i]
     RowTiles,       // ceil((row[i+1]-row[i]) / a)
     Array,          // arr[i]
     WindowPopc,     // popcount of the a words arr[i*a .. i*a+a)
@@ -158,7 +157,7 @@ enum class CountKind {
 };
 struct CountSpec {
     CountKind kind;
-    const uint32_t *row = nullptr;  // RowLen / RowTiles
+    const uint32_t *row = nullptr;  // RowTiles / NonEmpty
     const uint32_t *arr = nullptr;  // Array
     uint32_t a = 1;
 };

@@ -6,7 +6,7 @@
 // qsort for the K1 permutation (716-737); its block-local scan micro-benchmark (scan.cu)
 // has no carry between blocks.  Here those become one device-wide exclusive scan
 // (reduce / scan-of-block-sums / down-sweep, 64-bit offsets so 32-bit overflow is
-// detected, no inter-block waiting) and a stable LSD radix sort built on it.
+// detected, no inter-block waiting) and a stable LSD radix sort of up to 8 bits a pass.
 #include <cuda.h>
 
 #include <cstdio>
@@ -231,13 +231,12 @@ struct CountDev {
     __device__ __forceinline__ uint64_t operator()(size_t i) const
     {
         switch (kind) {
-        case 0: return (uint64_t)(row[i + 1] - row[i]);
-        case 1: {
+        case 0: {
             uint32_t l = row[i + 1] - row[i];
             return (uint64_t)((l + a - 1) / a);
         }
-        case 2: return (uint64_t)arr[i];
-        case 3: {
+        case 1: return (uint64_t)arr[i];
+        case 2: {
             uint64_t c = 0;
             for (uint32_t j = 0; j < a; j++) c += __popc(arr[i * a + j]);
             return c;

@@ -35,12 +35,13 @@ using namespace mm;
 // Blocks of 2 warps (a place on the SM is free when two units end: FP32 k = 8 on a 524,288-row
 // power-law 53.9 us in blocks of 8, 52.0 in blocks of 2), and registers for the rows in flight
 // before warps: the gathers are bound by the L1's line requests, which 16 warps of 4 to 8 rows in
-// flight per lane keep busy (32 warps capped at 64 registers 52.0 us, 24 49.6, 16 48.0, the start
-// 58.4; k = 4 101 -> 46, FP64 k = 2 118 -> 44).  Rows of 64 bytes and more hold to 24 warps (FP64
-// k = 8 on a band 62.5 -> 60.4 us; with 16 64.6).
+// flight per lane keep busy (32 warps capped at 64 registers 52.0 us, 24 49.6, 16 48.0, before the
+// streams loaded ahead 58.4; k = 4 101 -> 46, FP64 k = 2 118 -> 44).  On 1,048,576 rows the same
+// product gains 2 % in all: 88 -> 86 us.
 constexpr int kMMThreads = 64;
 // One right-hand side streams: 32 warps (FP64 on a 27-point stencil 80^3 33.6 -> 31.1 us; with 16
-// 40.3).
+// 40.3).  Rows of 64 bytes (FP32 k = 16; the adjoint's FP64 k = 8) hold to 24, as FP64 k = 8 did
+// before it went by several lanes (a band 62.5 -> 60.4 us; with 16 64.6).
 // The adjoint with its value gradient holds a row of X besides and takes the warps that leave it its
 // registers: with the product's 24 warps it spilled 0.1 to 2.3 KB a thread from rows of 128 bytes on
 // (slot order on a 524,288-row power-law, FP64 k = 16 / 32: 323 / 1043 us, 204 / 397 here; FP32 k =
@@ -491,22 +492,41 @@ gs_status scatter_vals(const gs_matrix *A, const T *v, T *out, cudaStream_t s)
     return GS_OK;
 }
 
+// Rows of 64 bytes and more go by several lanes per row (FP64 k = 8 / 16 / 32, a band 60 / 138 / 293
+// -> 46 / 87 / 141 us, a 524,288-row power-law 96 / 246 / 400 -> 75 / 194 / 300; FP32 k = 32 140 ->
+// 83 and 264 -> 200), but for FP32 k = 16, whose two lanes a row lose on a 27-point stencil 80^3 (81
+// -> 99; a band 60 -> 53, the power-law 96 -> 96).
+template <class T> constexpr bool several_lanes(uint32_t k)
+{
+    return sizeof(T) == 8 ? k >= 8 : k > 16;
+}
+
+// The products of one lane a row, and the adjoint with its value gradient at every width
+template <class T, int K, bool ADJ> gs_status launch_mm_k(const MMArgs &a, cudaStream_t s)
+{
+    if constexpr (ADJ || !several_lanes<T>(K)) {
+        const uint32_t blocks = (a.units + kMMThreads / 32 - 1) / (kMMThreads / 32);
+        k_k1_mm<T, K, ADJ><<<blocks, kMMThreads, 0, s>>>(a);
+        GS_CHECK_LAUNCH();
+        return GS_OK;
+    } else {
+        return launch_mm_wide<T>(a, K, s);
+    }
+}
+
 template <class T, bool ADJ>
 gs_status launch_mm(const MMArgs &a, uint32_t k, cudaStream_t s)
 {
     if (!a.units) return GS_OK;
-    const uint32_t blocks = (a.units + kMMThreads / 32 - 1) / (kMMThreads / 32);
     switch (k) {
-    case 1: k_k1_mm<T, 1, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
-    case 2: k_k1_mm<T, 2, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
-    case 4: k_k1_mm<T, 4, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
-    case 8: k_k1_mm<T, 8, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
-    case 16: k_k1_mm<T, 16, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
-    case 32: k_k1_mm<T, 32, ADJ><<<blocks, kMMThreads, 0, s>>>(a); break;
+    case 1: return launch_mm_k<T, 1, ADJ>(a, s);
+    case 2: return launch_mm_k<T, 2, ADJ>(a, s);
+    case 4: return launch_mm_k<T, 4, ADJ>(a, s);
+    case 8: return launch_mm_k<T, 8, ADJ>(a, s);
+    case 16: return launch_mm_k<T, 16, ADJ>(a, s);
+    case 32: return launch_mm_k<T, 32, ADJ>(a, s);
     default: return fail(GS_ERR_UNSUPPORTED, "k = %u right-hand sides (1, 2, 4, 8, 16, 32)", k);
     }
-    GS_CHECK_LAUNCH();
-    return GS_OK;
 }
 
 template <class T>
@@ -635,15 +655,6 @@ MMArgs adjoint_args(const gs_matrix *A, const void *ybar, void *xbar)
     return a;
 }
 
-// Rows of 64 bytes and more go by several lanes per row (FP64 k = 8 / 16 / 32, a band 60 / 138 / 293
-// -> 46 / 87 / 141 us, a 524,288-row power-law 96 / 246 / 400 -> 75 / 194 / 300; FP32 k = 32 140 ->
-// 83 and 264 -> 200), but for FP32 k = 16, whose two lanes a row lose on a 27-point stencil 80^3 (81
-// -> 99; a band 60 -> 53, the power-law 96 -> 96).
-bool several_lanes(uint32_t k, gs_dtype dtype)
-{
-    return dtype == GS_F64 ? k >= 8 : k > 16;
-}
-
 gs_status check_strided(const gs_matrix *A, gs_dtype dtype, uint32_t k, uint32_t cols)
 {
     GS_TRY(check_mm_matrix(A));
@@ -683,8 +694,6 @@ gs_status gs_spmm(gs_matrix *A, const void *d_X, void *d_Y, gs_dtype dtype, UIN 
     GS_TRY(ensure_mm_scratch(A, s));
     MMArgs a = forward_args(A, d_X, d_Y);
     a.ld = a.k = a.ldx = a.ldy = k;
-    if (several_lanes(k, dtype))
-        return dtype == GS_F64 ? launch_mm_wide<double>(a, k, s) : launch_mm_wide<float>(a, k, s);
     if (A->p.vtype == GS_F64) return launch_mm<double, false>(a, k, s);
     return launch_mm<float, false>(a, k, s);
 }
@@ -923,8 +932,6 @@ gs_status gs_spmm_adjoint(gs_matrix *A, const void *d_Ybar, const void *d_X, voi
         return f64 ? scatter_vals(A, A->vslots.as<double>(), static_cast<double *>(d_vbar), s)
                    : scatter_vals(A, A->vslots.as<float>(), static_cast<float *>(d_vbar), s);
     }
-    if (several_lanes(k, dtype))
-        return f64 ? launch_mm_wide<double>(a, k, s) : launch_mm_wide<float>(a, k, s);
     return f64 ? launch_mm<double, false>(a, k, s) : launch_mm<float, false>(a, k, s);
 }
 
