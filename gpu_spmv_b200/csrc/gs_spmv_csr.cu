@@ -266,8 +266,10 @@ gs_status launch_csr_t(const CsrArgs &a, cudaStream_t s)
     constexpr int BIG = sizeof(VT) == 8 ? 480 : 1024;
     const CsrShape c = csr_shape(a.n, a.nnz, sizeof(VT) == 8);
     if (c.cap == 288) return launch_csr_g<VT, IT, 288, 32, PAD>(a, s);
-    if (c.rows == 128) return launch_csr_g<VT, IT, 480, 128, PAD>(a, s);
-    if (c.rows == 64) return launch_csr_g<VT, IT, 480, 64, PAD>(a, s);
+    if constexpr (!PAD) {  // 64 rows a warp average 7 elements at most
+        if (c.rows == 128) return launch_csr_g<VT, IT, 480, 128, PAD>(a, s);
+        if (c.rows == 64) return launch_csr_g<VT, IT, 480, 64, PAD>(a, s);
+    }
     if (c.rows == 32 && c.cap == 480) return launch_csr_g<VT, IT, 480, 32, PAD>(a, s);
     if (c.rows == 32) return launch_csr_g<VT, IT, BIG, 32, PAD>(a, s);
     if (c.rows == 16) return launch_csr_g<VT, IT, BIG, 16, PAD>(a, s);
