@@ -187,3 +187,25 @@ def test_short_rows(name):
 def test_arrays_long_rows(name, lens, want):
     for _ in range(2):
         assert arrays(lens) == want
+
+
+def test_uneven_rows_of_local_columns():
+    """FP64 rows of very uneven length, 8 or more elements on average: the row-stream kernel with 8
+    positions per lane; y against the exact sums, 1e-13 (|A||x|)_i."""
+    from gpu_spmv_b200 import engine as E
+
+    rng = np.random.default_rng(9)
+    lens = np.minimum(np.exp(2.0 + 1.5 * rng.standard_normal(300000)), 2000).astype(int) // 4 * 4
+    assert lens.mean() >= 8 and product(lens.tolist()) == ROWS
+    row, col, e, m = _structure(lens)
+    val = torch.randn(col.numel(), dtype=torch.float64, device="cuda")
+    x = torch.rand(m, dtype=torch.float64, device="cuda") - 0.5
+    A = E.Matrix(row, col.int(), val, ncols=m, fmt="CSR")
+    assert A.info.lane_positions == 8
+    y = A.spmv(x).cpu().numpy()
+    A.close()
+    p = (val.cpu().numpy().astype(np.longdouble) * x[col].cpu().numpy().astype(np.longdouble))
+    some, at = lens > 0, row.cpu().numpy()[:-1][lens > 0]
+    want, mag = np.zeros(len(lens), np.longdouble), np.zeros(len(lens), np.longdouble)
+    want[some], mag[some] = np.add.reduceat(p, at), np.add.reduceat(np.abs(p), at)
+    assert np.all(np.abs(y - want) <= 1e-13 * mag)

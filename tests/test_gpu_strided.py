@@ -131,3 +131,38 @@ def test_value_gradient_orders_32(vtype):
         assert torch.equal(vc, A.convert_values(vs, to="csr")) and torch.equal(Xc, Xs)
         assert torch.equal(vs, A.convert_values(vc, to="slots"))
     A.close()
+
+
+def test_adjoint_refusals():
+    from gpu_spmv_b200 import _lib as L
+    from gpu_spmv_b200 import engine as E
+
+    row, col, val = _matrix(4)
+    A = E.Matrix(row, col, val, ncols=900, fmt="K1", adjoint=True)
+    B = E.Matrix(row, col, val, ncols=900, fmt="K1")
+    C = E.Matrix(row, col, val, ncols=900, fmt="CSR")
+    X, Xb = (torch.zeros(900, 40, device="cuda").double() for _ in range(2))
+    Yb, v = torch.zeros(1000, 40, device="cuda").double(), torch.zeros(len(col)).double().cuda()
+    x, xb, yb, vb = X.data_ptr(), Xb.data_ptr(), Yb.data_ptr(), v.data_ptr()
+    bad, no = L.GS_ERR_INVALID, L.GS_ERR_UNSUPPORTED
+    for want, m, args in [
+            (no, A, (yb, 40, x, 40, xb, 40, vb, L.GS_F64, 33, 40)),
+            (no, A, (yb, 40, x, 40, xb, 40, vb, L.GS_F64, 0, 40)),
+            (no, A, (yb, 40, x, 40, xb, 40, vb, L.GS_F32, 5, 5)),
+            (no, C, (yb, 40, x, 40, xb, 40, vb, L.GS_F64, 5, 5)),
+            (bad, B, (yb, 40, x, 40, xb, 40, vb, L.GS_F64, 5, 5)),     # no adjoint prepared
+            (bad, A, (yb, 40, x, 40, xb, 40, vb, L.GS_F64, 5, 4)),     # fewer columns than k
+            (bad, A, (yb, 6, x, 40, xb, 40, vb, L.GS_F64, 5, 8)),      # readable past a row
+            (bad, A, (yb, 40, x, 6, xb, 40, vb, L.GS_F64, 5, 8)),
+            (bad, A, (yb, 40, x, 40, xb, 4, vb, L.GS_F64, 5, 5)),      # rows overlap
+            (bad, A, (yb + 4, 40, x, 40, xb, 40, vb, L.GS_F64, 5, 5)),
+            (bad, A, (yb, 40, x + 4, 40, xb, 40, vb, L.GS_F64, 5, 5)),
+            (bad, A, (yb, 40, x, 40, xb + 4, 40, vb, L.GS_F64, 5, 5)),
+            (bad, A, (None, 40, x, 40, xb, 40, vb, L.GS_F64, 5, 5)),
+            (bad, A, (yb, 40, None, 40, xb, 40, vb, L.GS_F64, 5, 5)),  # a value gradient needs X
+            (bad, A, (yb, 40, x, 40, None, 40, vb, L.GS_F64, 5, 5)),
+            (L.GS_OK, A, (yb, 40, None, 0, xb, 40, None, L.GS_F64, 5, 5))]:
+        assert L.lib().gs_spmm_adjoint_strided(m._h, *args, None) == want, args
+    torch.cuda.synchronize()
+    for m in (A, B, C):
+        m.close()
