@@ -102,12 +102,23 @@ namespace {
 
 constexpr uint32_t kGrab = 4;  // items a warp takes per atomic
 
+// Launch shape.  The multi-RHS unit (mm_unit) loads its streams a batch ahead, which costs registers
+// (FP32 up to 16 columns 80 -> 97: 2 blocks of 256 per SM, not 3) and still is the faster for most
+// widths; the two that lost by it run in blocks of 2 warps, 20 and 16 warps per SM.  24 power-law
+// matrices of 4,000 to 200,000 rows, before / with the loads ahead / so: FP64 k 1-4 199 / 222 / 208 us
+// (1-8 386 / 285 / 306; bands and Laplacians gain), FP32 k 17-32 783 / 788 / 646.
+template <class T, int MAXK>
+constexpr bool kBatchSmall = sizeof(T) == 8 ? MAXK == 8 : MAXK == 32;
+template <class T, int MAXK> constexpr int kBatchThreads = kBatchSmall<T, MAXK> ? 64 : 256;
+template <class T, int MAXK>
+constexpr int kBatchBlocks = !kBatchSmall<T, MAXK> ? 0 : MAXK == 8 ? 10 : 8;  // 0: the compiler's
+
 // MAXK: the widest block in the batch (8, 16 or 32); narrower instantiations need fewer
 // registers and keep more warps resident
 template <class T, int MAXK>
-__global__ void __launch_bounds__(256) k_batch(const mm::MMArgs *__restrict__ desc,
-                                               const uint2 *__restrict__ items, uint32_t nitems,
-                                               uint32_t *next)
+__global__ void __launch_bounds__(kBatchThreads<T, MAXK>, kBatchBlocks<T, MAXK>) k_batch(
+    const mm::MMArgs *__restrict__ desc, const uint2 *__restrict__ items, uint32_t nitems,
+    uint32_t *next)
 {
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -735,15 +746,16 @@ template <class T, int MAXK>
 gs_status launch_batch(gs_batch *B, cudaStream_t s)
 {
     int per_sm = 0, dev = 0, sms = 148;
-    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<T, MAXK>, 256, 0));
+    constexpr int threads = kBatchThreads<T, MAXK>;
+    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<T, MAXK>, threads, 0));
     GS_CUDA(cudaGetDevice(&dev));
     GS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     B->blocks = std::max(1, per_sm) * sms;  // persistent: every resident block, once
     GS_CUDA(cudaMemsetAsync(B->d_next.p, 0, 4, s));
     if (B->nitems)
-        k_batch<T, MAXK><<<B->blocks, 256, 0, s>>>(B->d_desc.as<mm::MMArgs>(),
-                                                   B->d_items.as<uint2>(), B->nitems,
-                                                   B->d_next.as<uint32_t>());
+        k_batch<T, MAXK><<<B->blocks, threads, 0, s>>>(B->d_desc.as<mm::MMArgs>(),
+                                                       B->d_items.as<uint2>(), B->nitems,
+                                                       B->d_next.as<uint32_t>());
     GS_CHECK_LAUNCH();
     return GS_OK;
 }
