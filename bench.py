@@ -440,7 +440,8 @@ def time_adjoint(steps: int):
             "fwd_plus_adj_over_fwd_csr_order": round((f + adc) / f, 3),
             "fwd_plus_adj_over_fwd_atomic": round((f + aa) / f, 3),
             "fwd_plus_xbar_over_fwd_atomic": round((f + ax_a) / f, 3),
-            "note": "adjoint = Xbar = A^T Ybar and vbar (value gradient) in one launch; "
+            "note": "adjoint = Xbar = A^T Ybar and vbar (value gradient), in one launch where "
+                    "vbar is in slot order; "
                     "slots = values kept in the adjoint layout's order"}
 
 

@@ -332,7 +332,9 @@ gs_status gs_matrix_device_status(const gs_matrix *A, UIN *word, int reset);
 
 /* y = A x on the device.  x has ncols entries of xtype, y nrows entries of ytype.
  * F64 matrices take F64 x/y; F32/BF16 matrices take F32 x and F32 or F64 y.
- * Deterministic: every y entry is written once, with a fixed summation order.
+ * Deterministic: every y entry is written once, with a fixed summation order.  CSR and COM
+ * tileH = 1 matrices of local columns fuse multiply and add (FP64) and add interleaved sums
+ * in FP64, so their rows do not have the bits of a sequential loop.
  * Products on one matrix (gs_spmv, gs_spmm, gs_spmm_adjoint, batches holding it) share its
  * K1 split-chunk counters and status word: calls that could overlap in time (other
  * streams, other threads) must be ordered by the caller. */
@@ -365,7 +367,9 @@ gs_status gs_release_cached(void);
 gs_status gs_copy_to_host(void *h_dst, const void *d_src, size_t bytes);
 
 /* CSR SpMV straight from device CSR arrays: y = A x, FP64, in one kernel on the row pointers;
- * returns when y is complete.  For repeated products convert once with
+ * returns when y is complete.  Where a warp of it meets long rows side by side (more than 49,152
+ * elements beside its longest row), the row-stream kernel does the product on a plan made for the
+ * call (allocates).  For repeated products convert once with
  * gs_matrix_create(GS_FMT_CSR) and call gs_spmv.  val and col must be 16-byte aligned. */
 gs_status gs_csr_spmv_f64(UIN nrows, UIN ncols, UIN nnz, const UIN *d_row, const UIN *d_col,
                           const double *d_val, const double *d_x, double *d_y,
