@@ -506,7 +506,7 @@ gs_status convert(gs_matrix *A, const gs_convert_params &p, uint32_t n, uint32_t
         bool aligned = false;
         if (!A->tiled && !need_rlen) {  // CSR and COM tileH = 1
             CsrChoice c;
-            GS_TRY(csr_choice(d_row, d_col, n, nnz, p.vtype, &c, s));
+            GS_TRY(csr_choice(d_row, d_col, n, nnz, p.vtype, maxlen, &c, s));
             A->csr_local = c.local;
             if (!reduced) V = direct_lane_positions(n, nnz, c.random);
         }

@@ -349,12 +349,13 @@ gs_status launch_csr(const CsrArgs &a, gs_dtype vtype, gs_itype itype, gs_dtype 
 // Whether n rows (> 0) of nnz elements are enough to keep that kernel's warps busy.
 bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype);
 // What a look at a CSR matrix says: whether its x gathers are close to random, and whether its
-// products suit that kernel (see csr_suits in gs_spmv_csr.cu).  Synchronises.
+// products suit that kernel (see csr_suits in gs_spmv_csr.cu).  longest: the longest row, or 0 to
+// have it looked up.  Synchronises.
 struct CsrChoice {
     bool random = false, local = false;
 };
 gs_status csr_choice(const uint32_t *d_row, const uint32_t *d_col, uint32_t n, uint32_t nnz,
-                     gs_dtype vtype, CsrChoice *out, cudaStream_t s);
+                     gs_dtype vtype, uint32_t longest, CsrChoice *out, cudaStream_t s);
 // y = A x from CSR arrays, FP64, by the row-stream kernel on a plan made for the call
 // (synchronises).
 gs_status csr_rows_product(uint32_t n, uint32_t nnz, const uint32_t *d_row, const uint32_t *d_col,

@@ -517,7 +517,7 @@ str_res test_gcsr(const UIN cudaBlockSize, const str_matCSR m, const FPT *vec, c
     DevBuf row, col, val, x, y;
     gs::CsrChoice choice;
     if (upload_csr(m, row, col, val) || h2d(x, vec, m.nrows) || y.alloc((size_t)m.nrows * 8) ||
-        gs::csr_choice(row.as<UIN>(), col.as<UIN>(), m.nrows, m.nnz, GS_F64, &choice, 0))
+        gs::csr_choice(row.as<UIN>(), col.as<UIN>(), m.nrows, m.nnz, GS_F64, 0, &choice, 0))
         return error_res("gcsr", gs_last_error());
     if (choice.local) {
         gs::CsrArgs c{};

@@ -305,12 +305,15 @@ bool csr_enough_rows(uint32_t n, uint32_t nnz, gs_dtype vtype)
 }
 
 // Row lengths, for csr_suits: over `take` groups of 32 rows, `stride` groups apart, out[0] += 32
-// times the longest row, out[1] += elements; over all n rows out[2] = the longest, and over all
-// groups of G rows out[3] = the most elements (out cleared before).
+// times the longest row, out[1] += elements; out[2] = the longest row (where `rows` is n; 0 rows: it
+// is known), and over all groups of G rows out[3] = the most elements (out cleared before).
 __global__ void __launch_bounds__(256) k_row_shape(const uint32_t *__restrict__ row, uint32_t n,
                                                    uint32_t stride, uint32_t take, uint32_t G,
-                                                   unsigned long long *out)
+                                                   uint32_t rows, unsigned long long *out)
 {
+    __shared__ unsigned long long part[4];  // one atomic a block and number (a warp each: 10 us)
+    if (threadIdx.x < 4) part[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t t = blockIdx.x * 256ull + threadIdx.x, all = gridDim.x * 256ull;
     for (uint64_t w = t >> 5; w < take; w += all >> 5) {
@@ -318,22 +321,24 @@ __global__ void __launch_bounds__(256) k_row_shape(const uint32_t *__restrict__ 
         const uint32_t len = row[r + 1] - row[r];
         const uint32_t top = __reduce_max_sync(kFull, len), sum = __reduce_add_sync(kFull, len);
         if (lane == 0) {
-            atomicAdd(out, 32ull * top);
-            atomicAdd(out + 1, (unsigned long long)sum);
+            atomicAdd(part, 32ull * top);
+            atomicAdd(part + 1, (unsigned long long)sum);
         }
     }
     uint32_t longest = 0, heaviest = 0;
-    for (uint64_t r = t; r < n; r += all) {
-        const uint32_t b = row[r];
-        longest = max(longest, row[r + 1] - b);
-        if (r % G == 0) heaviest = max(heaviest, row[min(r + G, (uint64_t)n)] - b);
-    }
+    for (uint64_t r = t; r < rows; r += all) longest = max(longest, row[r + 1] - row[r]);
+    for (uint64_t r = t * G; r < n; r += all * G)
+        heaviest = max(heaviest, row[min(r + G, (uint64_t)n)] - row[r]);
     longest = __reduce_max_sync(kFull, longest);
     heaviest = __reduce_max_sync(kFull, heaviest);
     if (lane == 0) {
-        atomicMax(out + 2, (unsigned long long)longest);
-        atomicMax(out + 3, (unsigned long long)heaviest);
+        atomicMax(part + 2, (unsigned long long)longest);
+        atomicMax(part + 3, (unsigned long long)heaviest);
     }
+    __syncthreads();
+    if (threadIdx.x < 2 && part[threadIdx.x]) atomicAdd(out + threadIdx.x, part[threadIdx.x]);
+    if ((threadIdx.x == 2 || threadIdx.x == 3) && part[threadIdx.x])
+        atomicMax(out + threadIdx.x, part[threadIdx.x]);
 }
 
 // Whether a matrix's products run on k_csr rather than on the row-stream kernel: local columns;
@@ -366,7 +371,7 @@ static bool csr_suits(uint32_t n, uint32_t nnz, gs_dtype vtype, const unsigned l
 }
 
 gs_status csr_choice(const uint32_t *d_row, const uint32_t *d_col, uint32_t n, uint32_t nnz,
-                     gs_dtype vtype, CsrChoice *out, cudaStream_t s)
+                     gs_dtype vtype, uint32_t longest, CsrChoice *out, cudaStream_t s)
 {
     *out = CsrChoice();
     if (n == 0) return GS_OK;
@@ -376,13 +381,14 @@ gs_status csr_choice(const uint32_t *d_row, const uint32_t *d_col, uint32_t n, u
     GS_TRY(sample_col_steps(d_row, d_col, n, c, s));
     const uint32_t groups = n / 32, take = groups < 4096u ? groups : 4096u;
     const uint32_t blocks = (n - 1) / 256 + 1;
-    k_row_shape<<<blocks < 148u * 8u ? blocks : 148u * 8u, 256, 0, s>>>(
+    k_row_shape<<<blocks < 592u ? blocks : 592u, 256, 0, s>>>(
         d_row, n, take ? groups / take : 0u, take,
-        (uint32_t)csr_shape(n, nnz, vtype == GS_F64).rows, c + 2);
+        (uint32_t)csr_shape(n, nnz, vtype == GS_F64).rows, longest ? 0u : n, c + 2);
     GS_CHECK_LAUNCH();
     unsigned long long h[6] = {0, 0, 0, 0, 0, 0};
     GS_CUDA(cudaMemcpyAsync(h, c, 48, cudaMemcpyDeviceToHost, s));
     GS_CUDA(cudaStreamSynchronize(s));
+    if (longest) h[4] = longest;
     out->random = h[1] * 4 < h[0];
     out->local = csr_suits(n, nnz, vtype, h, h + 2);
     return GS_OK;
