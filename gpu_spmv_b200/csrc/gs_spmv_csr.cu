@@ -349,13 +349,12 @@ __global__ void __launch_bounds__(256) k_row_shape(const uint32_t *__restrict__ 
 // most 1.25 times the elements; 12M rows of 4 in the four reduced types 108 / 94 / 96 / 93 us and
 // 104 / 99 / 104 / 93, of 1 to 5 92 / 87 / 88 / 84 and 99 / 96 / 104 / 103, of 1 to 8 122 / 118 / 121
 // / 119 and 125 / 124 / 137 / 130, of 5 137 / 132 / 134 / 131 and 116 / 110 / 118 / 107, of 1 to 9
-// level); enough of them; and no group of a
-// warp's rows that the warp would still be walking when the others are done.  A single long row is
-// none (one warp walks it in either kernel: 300,000 rows of 5 and one of 30,000 296 us there, 144
-// here), nor a group of 1 1/4 windows (of 480 at least), nor one within 1/8000 of the elements
-// (some 10 % of the product's time); several long rows side by side are (1M rows of 27, 16 of 2,000
-// among them 81 us there and 166 here, 64 of 10,000 123 and 946; 300,000 of 5 with 128 of 300 11
-// and 49).
+// level); enough of them; and no group of a warp's rows that the warp would still be walking when
+// the others are done.  A single long row is none (one warp walks it in either kernel: 300,000 rows
+// of 5 and one of 30,000 288 us there, 141 here), nor a group of 1 1/4 windows (of 480 at least),
+// nor one within 1/8000 of the elements (some 10 % of the product's time); several long rows side
+// by side are (1M rows of 27, 16 of 2,000 among them 81 us there and 166 here, 64 of 10,000 123 and
+// 946; 300,000 of 5 with 128 of 300 11 and 49).
 static bool csr_suits(uint32_t n, uint32_t nnz, gs_dtype vtype, const unsigned long long steps[2],
                       const unsigned long long shape[4])
 {
